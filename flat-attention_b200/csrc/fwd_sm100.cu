@@ -471,7 +471,8 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                     tc_commit(s_full(w));
                     if (it.n_tiles[w] == 1) tc_commit(q_empty(w));  // the slot's last S of this item
                 }
-                if (ok) {
+                // (an item past its sequence's live rows has no KV tile and takes no ring entry: nothing is released)
+                if (ok && n_max > 0) {
                     tc_commit(kv_empty(stage_of(0)));
                     TRACEB(k, 2, 3);
                 }

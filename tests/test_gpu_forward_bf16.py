@@ -207,6 +207,28 @@ def test_variable_length_projection_bf16(B, Hq, Hkv, Nq, Nkv, D, causal, kvoff, 
     assert ctx().device_status() == 0
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,N,D,lens", [
+    (4, 32, 8, 1100, 64, [1100, 3, 256, 700]),
+    (6, 16, 4, 777, 128, [257, 777, 1, 512, 130, 31]),
+])
+def test_variable_length_blocks_without_a_live_row(B, Hq, Hkv, N, D, lens):
+    """Sequences much shorter than the padded length leave query blocks with no live row, and a CTA of the persistent
+    grid meets such blocks between live ones: they must take no K/V ring entry and release none.  Against the generic
+    f32 kernel on the same bf16-rounded inputs."""
+    q, k, v = randn(B * N * Hq * D, 51), randn(B * N * Hkv * D, 52), randn(B * N * Hkv * D, 53)
+    seqs = [fa.VarlenSequence(n, n, 0, 0) for n in lens]
+    shp = fa.shape(B, Hq, Hkv, N, N, D)
+    rot = fa.rotary(5e5, 0)
+    o, l = run_forward("projection_rope_varlen", fa.BF16, shp, fa.config(True), q, k, v, rot=rot, sequences=seqs)
+    assert ctx().device_status() == 0
+    eo, el = run_forward("projection_rope_varlen", fa.F32, shp, fa.config(True), q, k, v, rot=rot, sequences=seqs)
+    o, l, eo, el = o.reshape(B, N, Hq * D), l.reshape(B, Hq, N), eo.reshape(B, N, Hq * D), el.reshape(B, Hq, N)
+    for b, n in enumerate(lens):
+        check(o[b, :n].reshape(-1), l[b, :, :n].reshape(-1), eo[b, :n].reshape(-1), el[b, :, :n].reshape(-1), f"sequence {b}")
+        assert np.all(o[b, n:] == 0.0)
+        assert np.all(l[b, :, n:].reshape(-1).view(np.uint32) == 0xFF800000)
+
+
 def test_random_shapes_tensor_core_path_against_f32_path():
     """Differential sweep: the tcgen05 kernel (bf16) against the generic f32 kernel (itself pinned to the oracle at
     1e-4) on the same bf16-rounded inputs, over seeded random shapes: ragged and rectangular lengths, causal offsets,
