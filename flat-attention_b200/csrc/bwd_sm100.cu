@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
     const uint32_t ds_staged = bar0 + 8u * (6 + 2 * C::kStages);  // SPILL: the dS^T tile is complete in shared memory
     const uint32_t ds_free = bar0 + 8u * (7 + 2 * C::kStages);    // SPILL: ... and its bulk store has read it
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index_uniform(), lane = threadIdx.x & 31;
 
     // block -> (key tile, kv head, batch); early key tiles see the most queries and go first
     const int heads = p.kv_heads;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
     if (warp >= 8) {
         // 72 x 128 + 216 x 256 registers: exactly the CTA's launch allocation of 168 x 384
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        if (warp == kProducerWarp && lane == 0) {
+        if (warp == kProducerWarp && elect_one()) {
             // ================= TMA producer =================
             mbar_expect_tx(st_full, 2 * C::kTileBytes);
             for (int kb = 0; kb < C::kBoxes; ++kb) {
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
                 bulk_copy_g2s(smem_u32(stage + 2 * C::kTileBytes), p.neg_lse2 + row0, 512, rg_full(s));
                 bulk_copy_g2s(smem_u32(stage + 2 * C::kTileBytes + 512), p.delta + row0, 512, rg_full(s));
             }
-        } else if (warp == kMmaWarp && lane == 0) {
+        } else if (warp == kMmaWarp && elect_one()) {
             // ================= MMA issuer =================
             bool ok = true;
             auto wait = [&](uint32_t bar, uint32_t parity, int where) {
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
                 if (it < 16) TRS(it, 4);
             }
             if (ok) tc_commit(acc_final);
-        } else if (SPILL && warp == kMmaWarp + 1 && lane == 0) {
+        } else if (SPILL && warp == kMmaWarp + 1 && elect_one()) {
             // ================= dS^T spill =================
             // One bulk store of the staged 32 KiB tile per streamed tile; the elementwise warps may refill the staging
             // space once the store has read it.  The latency of the stores is spent here, not in the warps that compute.
@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
     const uint32_t acc_final = bar0 + 8u * (5 + 2 * C::kStages);
     const uint32_t a_ready = bar0 + 8u * (6 + 2 * C::kStages);   // Q is in TMEM
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index_uniform(), lane = threadIdx.x & 31;
 
     // block -> (query tile, head, batch); late query tiles see the most keys and go first
     const int lin = blockIdx.x;
@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
     if (warp >= 8) {
         // 72 x 128 + 216 x 256 registers: exactly the CTA's launch allocation of 168 x 384
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        if (warp == kProducerWarp && lane == 0) {
+        if (warp == kProducerWarp && elect_one()) {
             // ================= TMA producer =================
             mbar_expect_tx(st_full, 2 * C::kTileBytes);
             for (int kb = 0; kb < C::kBoxes; ++kb) {
@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
                                 rg_full(s));
                 }
             }
-        } else if (warp == kMmaWarp && lane == 0) {
+        } else if (warp == kMmaWarp && elect_one()) {
             // ================= MMA issuer =================
             bool ok = true;
             auto wait = [&](uint32_t bar, uint32_t parity, int where) {
@@ -837,7 +837,7 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
     auto rg_full = [&](int s) { return bar0 + 8u * s; };
     auto rg_empty = [&](int s) { return bar0 + 8u * (C::kStages + s); };
     const uint32_t acc_final = bar0 + 8u * (2 * C::kStages);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index_uniform(), lane = threadIdx.x & 31;
 
     // block -> (query tile, head, batch); late query tiles see the most keys and go first
     const int lin = blockIdx.x;
@@ -868,7 +868,7 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 4 && lane == 0 && !*abort_flag) {
+    if (warp == 4 && !*abort_flag && elect_one()) {
         // ================= producer =================
         const int kvh = h / p.group;
         for (int it = 0; it < n_iter; ++it) {
@@ -883,7 +883,7 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
             for (int kb = 0; kb < C::kBoxes; ++kb)
                 tma_load_4d(smem_u32(stage + C::kDsBytes + kb * C::kBoxBytes), &p.map_k, kb * 64, it * kTile, kvh, b, rg_full(s));
         }
-    } else if (warp == 5 && lane == 0 && !*abort_flag) {
+    } else if (warp == 5 && !*abort_flag && elect_one()) {
         // ================= MMA issuer =================
         bool ok = true;
         for (int it = 0; ok && it < n_iter; ++it) {

@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
     auto q_empty = [&](int w) { return bar0 + 8u * (10 + 2 * C::kStages + w); };
     auto k_ready = [&](int s) { return bar0 + 8u * (12 + 2 * C::kStages + s); };  // K tile converted (CONVK)
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = warp_index_uniform();
     const int lane = threadIdx.x & 31;
 
     if (warp == kProducerWarp && lane == 0) {
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
         }
     } else if (warp == kMmaWarp) {
         // ================= MMA issuer =================
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             auto wait = [&](uint32_t bar, uint32_t parity, int where) {
                 if (!ok) return;
