@@ -110,11 +110,9 @@ __device__ __forceinline__ int fast_div(int n, const FastDiv &f) {
 struct KernelParams {
     CUtensorMap map_q, map_k, map_v;
     CUtensorMap map_o;  // O as (d, row, head, batch) with boxes of 64 columns x 32 rows: the epilogue's bulk stores, one per warp
-    int o_tma;          // the epilogue stores O tiles through shared memory with bulk copies (not for padded batches)
     void *o;
     float *lse;
     int64_t o_bs, o_hs, o_rs, lse_hs;
-    int o_align32;  // every O row starts on a 32-byte boundary: 256-bit stores may be used
     int batch, q_heads, kv_heads, q_len, kv_len, group;
     FastDiv div_bh, div_heads, div_group;  // by batch * q_heads, by q_heads, by group
     int causal;
@@ -184,6 +182,7 @@ struct SplitRecord {
     int part_slot;  // index of its partial record
 };
 
+template <bool VARLEN>
 __device__ __forceinline__ WorkItem make_item_whole(const KernelParams &p, int lin) {
     // item index -> (query block, batch, head); late (long) query blocks first
     WorkItem it;
@@ -201,7 +200,7 @@ __device__ __forceinline__ WorkItem make_item_whole(const KernelParams &p, int l
     it.table_row0 = 0;
     it.j0 = 0;
     it.part_slot = -1;
-    if (p.varlen) {  // padded batch: src/wgpu_external_variable.rs:21-33
+    if constexpr (VARLEN) {  // padded batch: src/wgpu_external_variable.rs:21-33
         const flat_varlen_sequence m = p.varlen[it.b];
         it.q_len = (int)m.active_query_len;
         it.kv_len = (int)m.active_kv_len;
@@ -228,7 +227,7 @@ __device__ __forceinline__ SplitRecord decode_part(const KernelParams &p, int id
     const int v = idx - p.split_first;
     const int part = v / p.rem_items;
     r.lin = p.split_first + v % p.rem_items;
-    const WorkItem it = make_item_whole(p, r.lin);
+    const WorkItem it = make_item_whole<false>(p, r.lin);
     const int n = max(it.n_tiles[0], it.n_tiles[1]);
     const int lo = part * n / p.split, hi = (part + 1) * n / p.split;
     r.j0 = lo;
@@ -240,17 +239,17 @@ __device__ __forceinline__ SplitRecord decode_part(const KernelParams &p, int id
 
 // SPLIT: the launch cuts the items of its last round into KV parts (a template flag, so that launches without a split
 // carry none of its bookkeeping); `rec` is the CTA's decoded part in shared memory.
-template <bool SPLIT>
+template <bool SPLIT, bool VARLEN>
 __device__ __forceinline__ WorkItem make_item(const KernelParams &p, int lin, const volatile SplitRecord *rec) {
     if (SPLIT && lin >= p.split_first) {
-        WorkItem it = make_item_whole(p, rec->lin);
+        WorkItem it = make_item_whole<false>(p, rec->lin);
         it.j0 = rec->j0;
         it.n_tiles[0] = rec->n_tiles[0];
         it.n_tiles[1] = rec->n_tiles[1];
         it.part_slot = rec->part_slot;
         return it;
     }
-    return make_item_whole(p, lin);
+    return make_item_whole<VARLEN>(p, lin);
 }
 
 // The k-th item of this CTA, or -1.  Items are sorted longest first; CTAs take them in rounds of gridDim.x,
@@ -265,7 +264,10 @@ __device__ __forceinline__ int item_index(const KernelParams &p, int k) {
 // (src/attention_bias.rs:82-95) before the running maximum is taken.
 // F16IO: Q, K, V and O are IEEE binary16 instead of bf16 (P is then written as binary16 too, since one MMA takes A and B
 // of one format); accumulation, softmax and LSE stay f32.
-template <int D, bool CONVK, bool ALIBI, bool F16IO, bool SPLIT>
+// VARLEN: a padded variable-length batch (never split).  The rows past a sequence's live ones get O = 0, LSE = -inf
+// (src/asymmetric_grouped.rs:103-104) from the epilogue: filling O and LSE before the launch took 28 us of the 251 us of
+// a padded batch of 16 x 1024 rows, 32 heads, D = 128.
+template <int D, bool CONVK, bool ALIBI, bool F16IO, bool SPLIT, bool VARLEN>
 __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_constant__ KernelParams p) {
     using C = Cfg<D, CONVK>;
     extern __shared__ uint8_t smem_raw[];
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             for (int k = 0; ok; ++k) {
                 const int lin = item_index(p, k);
                 if (lin < 0) break;
-                const WorkItem it = make_item<SPLIT>(p, lin, split_rec);
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
                 const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
                 for (int w = 0; w < 2 && ok; ++w) {
                     if (it.n_tiles[w] == 0) continue;
@@ -448,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             for (int k = 0; ok; ++k) {
                 const int lin = item_index(p, k);
                 if (lin < 0) break;
-                const WorkItem it = make_item<SPLIT>(p, lin, split_rec);
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
                 const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
                 const bool trace_item = k == FLAT_TRACE_ITEM;
                 (void)trace_item;
@@ -521,7 +523,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
         for (int k = 0; ok; ++k) {
             const int lin = item_index(p, k);
             if (lin < 0) break;
-            const WorkItem it = make_item<SPLIT>(p, lin, split_rec);
+            const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
             const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
             for (int j = 0; ok && j < n_max; ++j, ring += 2) {
                 const int s = ring % C::kStages;
@@ -576,7 +578,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             float m = -INFINITY, l = 0.f;
             bool run = false;
             if (k >= 0) {
-                const WorkItem it = make_item<SPLIT>(p, item_index(p, k), split_rec);
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
                 run = it.n_tiles[w] > 0;
                 const int n = it.n_tiles[w];
                 int lim = it.kv_len - 1;  // last visible key of this row
@@ -738,7 +740,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 0);
             const int next_lin = item_index(p, k + 1);
             if (p.rope_q_table && next_lin >= 0 && ok) {
-                const WorkItem nx = make_item<SPLIT>(p, next_lin, split_rec);
+                const WorkItem nx = make_item<SPLIT, VARLEN>(p, next_lin, split_rec);
                 if (nx.n_tiles[w] > 0) {
                     // Rotate the Q tile in place (bf16 in, fp16 out).  A warp rotates its 32 rows; lane l
                     // takes the 16-byte chunk (l mod CH) of row (step * RPS + l / CH), so that the (cos, sin) table is
@@ -831,7 +833,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 3);
             if (run && ok) {
                 tc_fence_after();
-                const WorkItem it = make_item<SPLIT>(p, item_index(p, k), split_rec);
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
                 const int row = it.r0 + w * kTileRows + row_in_tile, b = it.b, h = it.h;
                 if (SPLIT && it.part_slot >= 0) {
                     // a part of a split item: unnormalised O, running max and sum go to the partial record
@@ -849,7 +851,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                     }
                     p.part_ml[prow] = make_float2(m, l);
                     tc_fence_before();
-                } else if (p.o_tma) {
+                } else {
                     // O leaves through shared memory: every thread writes its row's 128 bytes of a 64-column box in the
                     // swizzled box layout and each warp sends its 32 rows with one bulk store (whole lines), instead of
                     // 32-byte stores 256 bytes apart per thread
@@ -874,6 +876,10 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                                 pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
                             }
                         }
+                        if (VARLEN && row >= it.q_len) {  // a padded row of a variable-length batch: O = 0
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) pk[i] = 0;
+                        }
                         // A warp stages and sends its own 32 rows, so the four warps of the slot never wait for one
                         // another here.  The staging rows are reused by the next box: the lane that sent the previous one
                         // waits for that bulk store's read only now, after the next box has been fetched and converted
@@ -890,63 +896,45 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                         fence_proxy_async();  // generic-proxy writes -> visible to the bulk copy's async proxy
                         __syncwarp();
                         // (rows past q_len are clipped by the tensor map; a box that starts past it is not sent at all)
-                        if (lane == 0 && it.r0 + w * kTileRows + lane_base < it.q_len) {
+                        if (lane == 0 && it.r0 + w * kTileRows + lane_base < p.q_len) {
                             tma_store_4d(&p.map_o, hf * 64, it.r0 + w * kTileRows + lane_base, h, b, smem_u32(stg + lane_base * 128));
                             bulk_commit_group();
                             store_pending = true;
                         }
                     }
-                    if (row < it.q_len) p.lse[((long long)b * p.q_heads + h) * p.lse_hs + row] = (m + log2f(l)) * kLn2;
+                    if (row < p.q_len)
+                        p.lse[((long long)b * p.q_heads + h) * p.lse_hs + row] = VARLEN && row >= it.q_len ? -INFINITY : (m + log2f(l)) * kLn2;
+                    // the O columns are overwritten by the next item's first PV MMA, which is issued only after this
+                    // thread's next hand-over of P: program order keeps the reads above ahead of it
                     tc_fence_before();
-                } else {
-                const float inv = 1.0f / l;
-                const bool store = row < it.q_len;
-                __nv_bfloat16 *op = reinterpret_cast<__nv_bfloat16 *>(p.o) + (long long)b * p.o_bs + (long long)h * p.o_hs +
-                                    (long long)row * p.o_rs;
-                uint32_t r[32];
-#pragma unroll
-                for (int c = 0; c < D / 32; ++c) {
-                    tmem_ld32(t_o + c * 32, r);
-                    tc_wait_ld();
-                    if (store) {
-                        uint32_t pk[16];
-#pragma unroll
-                        for (int i = 0; i < 32; i += 2) {
-                            if constexpr (F16IO) {
-                                __half2 h2 = __floats2half2_rn(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
-                                pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                            } else {
-                                __nv_bfloat162 h2 =
-                                    __floats2bfloat162_rn(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
-                                pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                            }
-                        }
-                        if (p.o_align32) {
-                            // 32-byte stores: a lane fills whole 32-byte sectors of its row
-#pragma unroll
-                            for (int q8 = 0; q8 < 2; ++q8)
-                                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(op + c * 32 + q8 * 16),
-                                             "r"(pk[q8 * 8]), "r"(pk[q8 * 8 + 1]), "r"(pk[q8 * 8 + 2]), "r"(pk[q8 * 8 + 3]),
-                                             "r"(pk[q8 * 8 + 4]), "r"(pk[q8 * 8 + 5]), "r"(pk[q8 * 8 + 6]), "r"(pk[q8 * 8 + 7])
-                                             : "memory");
-                        } else {
-                            uint4 *dst = reinterpret_cast<uint4 *>(op + c * 32);
-#pragma unroll
-                            for (int q4 = 0; q4 < 4; ++q4)
-                                dst[q4] = make_uint4(pk[q4 * 4], pk[q4 * 4 + 1], pk[q4 * 4 + 2], pk[q4 * 4 + 3]);
-                        }
-                    }
-                }
-                if (store) p.lse[((long long)b * p.q_heads + h) * p.lse_hs + row] = (m + log2f(l)) * kLn2;
-                // the O columns are overwritten by the next item's first PV MMA, which is issued only after this
-                // thread's next hand-over of P: program order keeps the reads above ahead of it
-                tc_fence_before();
                 }
             } else if (SPLIT && k >= 0 && ok) {
                 // a part in which this Q tile has no KV tile at all still owns a partial record: an empty one
-                const WorkItem it = make_item<SPLIT>(p, item_index(p, k), split_rec);
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
                 if (it.part_slot >= 0)
                     p.part_ml[(long long)it.part_slot * (2 * kTileRows) + w * kTileRows + row_in_tile] = make_float2(-INFINITY, 0.f);
+            }
+            if (VARLEN && k >= 0 && !run && ok) {
+                // a tile past its sequence's live rows: O = 0, LSE = -inf (src/asymmetric_grouped.rs:103-104)
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
+                const int row = it.r0 + w * kTileRows + row_in_tile;
+                uint8_t *stg = o_stage + w * C::kOutStageBytes;
+                if (lane == 0 && store_pending) {
+                    bulk_wait_group_read0();
+                    store_pending = false;
+                }
+                __syncwarp();
+#pragma unroll
+                for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<uint4 *>(stg + row_in_tile * 128 + (ch << 4)) = make_uint4(0, 0, 0, 0);
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0 && it.r0 + w * kTileRows + lane_base < p.q_len) {
+                    for (int hf = 0; hf < D / 64; ++hf)
+                        tma_store_4d(&p.map_o, hf * 64, it.r0 + w * kTileRows + lane_base, it.h, it.b, smem_u32(stg + lane_base * 128));
+                    bulk_commit_group();
+                    store_pending = true;
+                }
+                if (row < p.q_len) p.lse[((long long)it.b * p.q_heads + it.h) * p.lse_hs + row] = -INFINITY;
             }
             if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 4);
             if (next_lin < 0) break;
@@ -982,10 +970,6 @@ __global__ void __launch_bounds__(256) rope_table_kernel(float2 *__restrict__ ta
         sincosf(angle, &s, &c);
         table[i] = make_float2(c, s);
     }
-}
-
-__global__ void __launch_bounds__(256) fill_u32_kernel(uint32_t *__restrict__ dst, uint32_t value, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) dst[i] = value;
 }
 
 // Finishes the rows of the split items of the last round: for each row the parts' unnormalised O_i, running maxima
@@ -1217,9 +1201,8 @@ void forward_sm100_geometry(const flat_ctx *ctx, const FwdParams &p, uint32_t *q
     const SplitPlan pl = plan_split(ctx->sm_count, p);
     grid[0] = pl.grid;  // persistent: one CTA per SM
     grid[1] = grid[2] = 1;
-    // the attention kernel, the K rotation pass when K arrives raw, the LSE fill of a padded variable-length batch and
-    // the merge of the last round's split items
-    *dispatches = 1 + (p.rope_k ? 1 : 0) + (p.varlen ? 1 : 0) + (pl.split > 1 ? 1 : 0);
+    // the attention kernel, the K rotation pass when K arrives raw and the merge of the last round's split items
+    *dispatches = 1 + (p.rope_k ? 1 : 0) + (pl.split > 1 ? 1 : 0);
 }
 
 int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
@@ -1278,15 +1261,11 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
         if ((st = make_map(ctx, &kp.map_k, k_f16 || io16, k_ptr, D, p.kv_len, p.kv_heads, p.batch, k_rs, k_hs, k_bs, kTileRows))) return st;
         if ((st = make_map(ctx, &kp.map_v, io16, p.v, D, p.kv_len, p.kv_heads, p.batch, p.kv_rs, p.kv_hs, p.kv_bs, kTileRows))) return st;
     }
-    // the epilogue's bulk stores clip at the call's q_len, not at a sequence's active length: padded batches keep the
-    // per-thread stores
-    kp.o_tma = p.varlen ? 0 : 1;
-    if (kp.o_tma && (st = make_map(ctx, &kp.map_o, io16, p.o, D, p.q_len, p.q_heads, p.batch, p.o_rs, p.o_hs, p.o_bs, 32)))
+    if ((st = make_map(ctx, &kp.map_o, io16, p.o, D, p.q_len, p.q_heads, p.batch, p.o_rs, p.o_hs, p.o_bs, 32)))
         return st;
     kp.o = p.o;
     kp.lse = p.lse;
     kp.o_bs = p.o_bs; kp.o_hs = p.o_hs; kp.o_rs = p.o_rs; kp.lse_hs = p.lse_hs;
-    kp.o_align32 = (reinterpret_cast<uintptr_t>(p.o) % 32 == 0 && p.o_bs % 16 == 0 && p.o_hs % 16 == 0 && p.o_rs % 16 == 0) ? 1 : 0;
     kp.batch = p.batch; kp.q_heads = p.q_heads; kp.kv_heads = p.kv_heads; kp.q_len = p.q_len; kp.kv_len = p.kv_len;
     kp.group = p.group;
     kp.div_bh = make_fastdiv(p.batch * p.q_heads);
@@ -1306,15 +1285,6 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     kp.rope_q_table = q_table;
     kp.varlen = p.varlen;
     kp.rope_table_base = p.varlen ? p.varlen_rope_min : 0;
-    if (p.varlen) {
-        // padded query rows: O = 0, LSE = -inf (src/asymmetric_grouped.rs:103-104); the kernel writes only live rows.
-        // The projection layout of this entry point makes O one contiguous block.
-        const int64_t o_elems = (int64_t)p.batch * p.q_len * p.q_heads * D, lse_elems = (int64_t)p.batch * p.q_heads * p.q_len;
-        FLAT_CUDA_OK(ctx, cudaMemsetAsync(p.o, 0, o_elems * 2, ctx->stream));
-        fill_u32_kernel<<<(unsigned)std::min<int64_t>((lse_elems + 255) / 256, 4096), 256, 0, ctx->stream>>>(
-            reinterpret_cast<uint32_t *>(p.lse), 0xff800000u, lse_elems);
-        ctx->launches += 1;
-    }
     if (q_table) {
         const double rows_per_step = 32.0 / (D / 8);
         for (int j = 0; j < D / 2; ++j) {
@@ -1364,12 +1334,15 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     kp.alibi_slopes = p.alibi_slopes;
     kp.alibi_delta = (int)(p.alibi_kv_off - p.alibi_q_off);
     kp.alibi_inv_scale = 1.0f / p.scale;
-    // <head_dim, CONVK, ALIBI, F16IO, SPLIT>
+    // <head_dim, CONVK, ALIBI, F16IO, SPLIT, VARLEN>
     auto pick = [&](auto d_tag, auto convk_tag, auto alibi_tag, auto f16_tag) -> int {
         constexpr int kD = decltype(d_tag)::value;
         constexpr bool kConv = decltype(convk_tag)::value, kAlibi = decltype(alibi_tag)::value, kF16 = decltype(f16_tag)::value;
-        if (plan.split > 1) return run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, true>, Cfg<kD, kConv>::kSmemBytes);
-        return run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, false>, Cfg<kD, kConv>::kSmemBytes);
+        constexpr int kSmem = Cfg<kD, kConv>::kSmemBytes;
+        if constexpr (!kAlibi)
+            if (p.varlen) return run(fwd_sm100_kernel<kD, kConv, false, kF16, false, true>, kSmem);
+        if (plan.split > 1) return run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, true, false>, kSmem);
+        return run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, false, false>, kSmem);
     };
     using T = std::true_type;
     using F = std::false_type;
