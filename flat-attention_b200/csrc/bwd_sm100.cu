@@ -34,6 +34,8 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "common.h"
 #include "sm100_host.cuh"
 #include "sm100_ptx.cuh"
@@ -69,6 +71,7 @@ struct BwdKernelParams {
     int batch, q_heads, kv_heads, seq_len, group, n_tiles;
     int seq_pad;            // seq_len rounded up to whole tiles: row stride of neg_lse2 / delta
     int causal;
+    int parts;              // KV-stationary kernel: CTAs (one cluster) that share the query tiles of a key tile
     float scale, scale_log2;
     uint32_t idesc_k, idesc_mn, idesc_dq;
     DeviceStatus *status;
@@ -155,14 +158,17 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
 
     // block -> (key tile, kv head, batch); early key tiles see the most queries and go first
     const int heads = p.kv_heads;
-    const int lin = blockIdx.x;
+    const int part = blockIdx.x % p.parts, lin = blockIdx.x / p.parts;
     const int tile_rank = lin / (heads * p.batch);
     const int bh = lin % (heads * p.batch);
     const int b = bh / heads, h = bh % heads;
     const int t_own = tile_rank;
     const int first = p.causal ? t_own : 0;
     const int per_head = p.n_tiles - first;
-    const int n_iter = per_head * p.group;
+    // streamed (query head, query tile) pairs of the key tile: this CTA takes [it0, it0 + n_iter)
+    const int n_total = per_head * p.group;
+    const int it0 = part * n_total / p.parts;
+    const int n_iter = (part + 1) * n_total / p.parts - it0;
 
     if (threadIdx.x == 0) {
         *abort_flag = (smem_u32(smem) & 1023u) ? 1 : 0;  // a misplaced shared window would break the swizzle: refuse to run
@@ -195,7 +201,9 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
     if (warp >= 8) {
         // 72 x 128 + 216 x 256 registers: exactly the CTA's launch allocation of 168 x 384
         asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-        if (warp == kProducerWarp && elect_one()) {
+        if (n_iter == 0) {
+            // nothing is streamed to this CTA
+        } else if (warp == kProducerWarp && elect_one()) {
             // ================= TMA producer =================
             mbar_expect_tx(st_full, 2 * C::kTileBytes);
             for (int kb = 0; kb < C::kBoxes; ++kb) {
@@ -209,8 +217,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
                     timeout(p, 100 + s);
                     break;
                 }
-                const int t = first + it % per_head;
-                const int hs = h * p.group + it / per_head;  // query head of the streamed tensors
+                const int t = first + (it0 + it) % per_head;
+                const int hs = h * p.group + (it0 + it) / per_head;  // query head of the streamed tensors
                 uint8_t *stage = ring + s * C::kStageBytes;
                 mbar_expect_tx(rg_full(s), C::kStageBytes);
                 for (int kb = 0; kb < C::kBoxes; ++kb) {
@@ -301,8 +309,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
                     timeout(p, 400);
                     break;
                 }
-                const int t = first + it % per_head;
-                const int hs = h * p.group + it / per_head;
+                const int t = first + (it0 + it) % per_head;
+                const int hs = h * p.group + (it0 + it) / per_head;
                 bulk_copy_s2g(p.ds_spill + ds_tile_index(p, b, hs, t_own, t) * C::kDsBytes, smem_u32(ds_s), C::kDsBytes);
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -329,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
             }
             const float *lse_s = reinterpret_cast<const float *>(stage + 2 * C::kTileBytes) + half * 64;
             const float *delta_s = lse_s + 128;
-            const int t = first + it % per_head;
+            const int t = first + (it0 + it) % per_head;
             const bool diag = p.causal && t == t_own;
             // ---- phase 1: P^T ----
             if (!mbar_wait(x_full, it & 1, abort_flag)) {
@@ -441,11 +449,31 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
             if (SPILL && lane == 0) mbar_arrive(ds_staged);
             if (warp == 0 && lane == 0 && it < 16) TRS(it, 7);
         }
-        if (ok && !mbar_wait(acc_final, 0, abort_flag)) {
+        if (ok && n_iter > 0 && !mbar_wait(acc_final, 0, abort_flag)) {
             timeout(p, 320);
             ok = false;
         }
-        if (ok) {
+        if (p.parts > 1) {
+            // the accumulators wait for the other CTAs of the cluster in shared memory (over the K, V and streamed tiles,
+            // which every MMA has read), 16-byte chunks swizzled by the row
+            if (ok && n_iter > 0) {
+                tc_fence_after();
+                float *acc_s = reinterpret_cast<float *>(smem);
+#pragma unroll
+                for (int a = 0; a < 2; ++a)
+#pragma unroll
+                    for (int c = 0; c < D / 64; ++c) {
+                        uint32_t r[32];
+                        const int col = half * (D / 2) + c * 32;
+                        tmem_ld32(t_lane + (a == 0 ? kColA0 : kColA1) + col, r);
+                        tc_wait_ld();
+#pragma unroll
+                        for (int q4 = 0; q4 < 8; ++q4)
+                            *reinterpret_cast<uint4 *>(acc_s + (a * kTile + row_local) * D + col + ((q4 ^ (row_local & 7)) << 2)) =
+                                make_uint4(r[q4 * 4], r[q4 * 4 + 1], r[q4 * 4 + 2], r[q4 * 4 + 3]);
+                    }
+            }
+        } else if (ok) {
             tc_fence_after();
             // each warp group writes half of the head dimension of the accumulator rows
             const long long out_row = ((long long)b * heads + h) * p.seq_len + (long long)t_own * kTile + row_local;
@@ -477,6 +505,30 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
     }
     tc_fence_before();
     __syncthreads();
+    if (p.parts > 1) {
+        // dV and dK: every CTA finishes its share of the 16-byte chunks, adding the parts in rank order
+        namespace cg = cooperative_groups;
+        cg::cluster_group cluster = cg::this_cluster();
+        cluster.sync();
+        constexpr int kRowVecs = D / 4, kVecs = 2 * kTile * kRowVecs;
+        const int v_end = (part + 1) * kVecs / p.parts;
+        for (int v = part * kVecs / p.parts + threadIdx.x; v < v_end; v += kThreads) {
+            const int a = v / (kTile * kRowVecs), row = v / kRowVecs % kTile, ch = v % kRowVecs;
+            if (t_own * kTile + row >= p.seq_len) continue;  // keys past seq_len were zero-filled, not real
+            float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int x = 0; x < p.parts; ++x) {
+                if ((x + 1) * n_total / p.parts == x * n_total / p.parts) continue;  // a CTA without a streamed tile
+                const float *from = cluster.map_shared_rank(reinterpret_cast<float *>(smem), x);
+                const float4 y = *reinterpret_cast<const float4 *>(from + (a * kTile + row) * D + ((ch ^ (row & 7)) << 2));
+                sum = make_float4(sum.x + y.x, sum.y + y.y, sum.z + y.z, sum.w + y.w);
+            }
+            const float mul = a == 0 ? 1.0f : p.scale;  // dV unscaled; dK carries the softmax scale
+            float *to = reinterpret_cast<float *>(a == 0 ? p.out0 : p.out1) +
+                        (((long long)b * heads + h) * p.seq_len + (long long)t_own * kTile + row) * D + ch * 4;
+            *reinterpret_cast<float4 *>(to) = make_float4(sum.x * mul, sum.y * mul, sum.z * mul, sum.w * mul);
+        }
+        cluster.sync();  // a CTA's shared memory outlives its readers
+    }
 #ifdef FLAT_TRACE
     if (p.trace && blockIdx.x == 0)
         for (int i = threadIdx.x; i < 32 * 8; i += kThreads) p.trace[1 * 64 * 8 + i] = tr_s[i];
@@ -944,14 +996,18 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
 // neighbouring lanes share a row, so a warp covers 256 / head_dim rows with full-width loads.
 __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *__restrict__ d_out,
                                                        const __nv_bfloat16 *__restrict__ out, const float *__restrict__ lse,
-                                                       float *__restrict__ delta, float *__restrict__ neg_lse2, int64_t rows,
+                                                       float *__restrict__ delta, float *__restrict__ neg_lse2, int64_t rows_pad,
                                                        int head_dim, int seq_len, int seq_pad) {
     const int lanes_per_row = head_dim / 8;  // 8 or 16
     const int rows_per_block = 256 / lanes_per_row;
     const int sub = threadIdx.x % lanes_per_row;
-    const int64_t row = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / lanes_per_row;
+    // rows of a (batch, head) are padded to whole tiles; the slots of rows past seq_len must hold finite values, and with
+    // zeros the zero-filled Q / dO rows contribute nothing
+    const int64_t dst = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / lanes_per_row;
+    const bool live = dst < rows_pad && dst % seq_pad < seq_len;
+    const int64_t row = dst / seq_pad * seq_len + dst % seq_pad;
     float acc = 0.f;
-    if (row < rows) {
+    if (live) {
         const uint4 a = __ldg(reinterpret_cast<const uint4 *>(d_out + row * head_dim) + sub);
         const uint4 o = __ldg(reinterpret_cast<const uint4 *>(out + row * head_dim) + sub);
         const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, ow[4] = {o.x, o.y, o.z, o.w};
@@ -962,10 +1018,9 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *__re
         }
     }
     for (int w = lanes_per_row / 2; w >= 1; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
-    if (sub == 0 && row < rows) {
-        const int64_t dst = row / seq_len * seq_pad + row % seq_len;  // rows of a (batch, head) padded to whole tiles
+    if (sub == 0 && dst < rows_pad) {
         delta[dst] = acc;
-        neg_lse2[dst] = -lse[row] * kLog2e;
+        neg_lse2[dst] = live ? -lse[row] * kLog2e : 0.f;
     }
 }
 
@@ -992,6 +1047,18 @@ uint64_t small_scratch_bytes(const BwdParams &p) {
     const uint64_t seq_pad = ((uint64_t)p.seq_len + kTile - 1) / kTile * kTile;
     return (2 * (uint64_t)p.batch * p.q_heads * seq_pad * sizeof(float) + 1023) & ~uint64_t(1023);
 }
+// CTAs per key tile in the dK/dV kernel.  A key tile streams n * group (query tile, head) pairs, under a causal mask the
+// first tile n times as many as the last, so a small call has fewer key tiles than SMs, or one long CTA that the others
+// wait for.  The smallest cluster is taken whose longest CTA stays within a quarter of an even share of all pairs, but no
+// CTA should get fewer than kMinPairs of them: its start and its share of the sum cost as much as three or four.
+constexpr int kMinPairs = 4;
+int key_tile_parts(const flat_ctx *ctx, const BwdParams &p) {
+    const long long n = ((long long)p.seq_len + kTile - 1) / kTile;
+    const long long pairs = (p.causal ? n * (n + 1) / 2 : n * n) * p.q_heads * p.batch, longest = n * p.group;
+    int parts = 1;
+    while (parts < 8 && (parts + 1) * kMinPairs <= longest && 4 * ((longest + parts - 1) / parts) * ctx->sm_count > 5 * pairs) ++parts;
+    return parts;
+}
 bool use_spill(const flat_ctx *ctx, const BwdParams &p) { return spill_bytes(p) <= ctx->backward_scratch_budget; }
 }  // namespace
 
@@ -1004,17 +1071,14 @@ int launch_backward_sm100(flat_ctx *ctx, const BwdParams &p) {
     if (st) return st;
     const int D = p.head_dim, N = p.seq_len;
     const bool spill = use_spill(ctx, p);
-    const int64_t rows = (int64_t)p.batch * p.q_heads * N;
     const int seq_pad = (N + kTile - 1) / kTile * kTile;
     const int64_t rows_pad = (int64_t)p.batch * p.q_heads * seq_pad;
     float *delta = reinterpret_cast<float *>(scratch_ptr(ctx));
     float *neg_lse2 = delta + rows_pad;
-    // the slots of rows past seq_len must hold finite values: with zeros the zero-filled Q / dO rows contribute nothing
-    if (seq_pad != N) FLAT_CUDA_OK(ctx, cudaMemsetAsync(delta, 0, 2 * rows_pad * sizeof(float), ctx->stream));
     const int prep_rows_per_block = 256 / (D / 8);
-    bwd_prep_kernel<<<(unsigned)((rows + prep_rows_per_block - 1) / prep_rows_per_block), 256, 0, ctx->stream>>>(
-        static_cast<const __nv_bfloat16 *>(p.d_out), static_cast<const __nv_bfloat16 *>(p.out), p.lse, delta, neg_lse2, rows, D,
-        N, seq_pad);
+    bwd_prep_kernel<<<(unsigned)((rows_pad + prep_rows_per_block - 1) / prep_rows_per_block), 256, 0, ctx->stream>>>(
+        static_cast<const __nv_bfloat16 *>(p.d_out), static_cast<const __nv_bfloat16 *>(p.out), p.lse, delta, neg_lse2, rows_pad,
+        D, N, seq_pad);
     ctx->launches += 1;
 
     BwdKernelParams kp{};
@@ -1041,21 +1105,33 @@ int launch_backward_sm100(flat_ctx *ctx, const BwdParams &p) {
     if (const char *tp = getenv("FLAT_TRACE_PTR")) kp.trace = reinterpret_cast<long long *>(strtoull(tp, nullptr, 0));
 #endif
 
-    auto run = [&](auto kernel, int smem_bytes, long long grid, int threads = kThreads) -> int {
+    auto run = [&](auto kernel, int smem_bytes, long long grid, int threads = kThreads, int cluster = 1) -> int {
         FLAT_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3((unsigned)threads);
+        cfg.dynamicSmemBytes = (size_t)smem_bytes;
+        cfg.stream = ctx->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = cluster > 1 ? 1 : 0;
         KernelTimer timer(ctx);
-        kernel<<<(unsigned)grid, threads, smem_bytes, ctx->stream>>>(kp);
+        FLAT_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kernel, kp));
         return FLAT_OK;
     };
-    const long long grid_kv = (long long)kp.n_tiles * p.kv_heads * p.batch;
+    kp.parts = key_tile_parts(ctx, p);
+    const long long grid_kv = (long long)kp.n_tiles * p.kv_heads * p.batch * kp.parts;
     const long long grid_q = (long long)kp.n_tiles * p.q_heads * p.batch;
     kp.out0 = p.dv;
     kp.out1 = p.dk;
     if (spill) {
-        if (D == 128) st = run(bwd_sm100_kernel<128, true>, BCfg<128>::kSmemBytes, grid_kv);
-        else st = run(bwd_sm100_kernel<64, true>, BCfg<64>::kSmemBytes, grid_kv);
-    } else if (D == 128) st = run(bwd_sm100_kernel<128, false>, BCfg<128>::kSmemBytes, grid_kv);
-    else st = run(bwd_sm100_kernel<64, false>, BCfg<64>::kSmemBytes, grid_kv);
+        if (D == 128) st = run(bwd_sm100_kernel<128, true>, BCfg<128>::kSmemBytes, grid_kv, kThreads, kp.parts);
+        else st = run(bwd_sm100_kernel<64, true>, BCfg<64>::kSmemBytes, grid_kv, kThreads, kp.parts);
+    } else if (D == 128) st = run(bwd_sm100_kernel<128, false>, BCfg<128>::kSmemBytes, grid_kv, kThreads, kp.parts);
+    else st = run(bwd_sm100_kernel<64, false>, BCfg<64>::kSmemBytes, grid_kv, kThreads, kp.parts);
     if (st) return st;
     kp.out0 = p.dq;
     kp.out1 = nullptr;
