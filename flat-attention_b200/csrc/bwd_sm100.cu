@@ -170,6 +170,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
     const int it0 = part * n_total / p.parts;
     const int n_iter = (part + 1) * n_total / p.parts - it0;
 
+    grid_dependency_launch();  // the dQ kernel
     if (threadIdx.x == 0) {
         *abort_flag = (smem_u32(smem) & 1023u) ? 1 : 0;  // a misplaced shared window would break the swizzle: refuse to run
         if (*abort_flag) timeout(p, 90);
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
                 tma_load_4d(smem_u32(st0 + kb * C::kBoxBytes), &p.map_k, kb * 64, t_own * kTile, h, b, st_full);
                 tma_load_4d(smem_u32(st1 + kb * C::kBoxBytes), &p.map_v, kb * 64, t_own * kTile, h, b, st_full);
             }
+            grid_dependency_wait();  // LSE and delta come from the kernel before this one
             for (int it = 0; it < n_iter; ++it) {
                 const int s = it % C::kStages;
                 const uint32_t phase = (it / C::kStages) & 1;
@@ -627,6 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
     constexpr uint32_t kColQ = 0, kColX = 64, kColY = 192, kColDS = 320, kColAcc = 384;
 
     if (warp >= 8) {
@@ -919,6 +922,7 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_wait();
 
     if (warp == 4 && !*abort_flag && elect_one()) {
         // ================= producer =================
@@ -998,6 +1002,7 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *__re
                                                        const __nv_bfloat16 *__restrict__ out, const float *__restrict__ lse,
                                                        float *__restrict__ delta, float *__restrict__ neg_lse2, int64_t rows_pad,
                                                        int head_dim, int seq_len, int seq_pad) {
+    grid_dependency_launch();
     const int lanes_per_row = head_dim / 8;  // 8 or 16
     const int rows_per_block = 256 / lanes_per_row;
     const int sub = threadIdx.x % lanes_per_row;
@@ -1112,12 +1117,14 @@ int launch_backward_sm100(flat_ctx *ctx, const BwdParams &p) {
         cfg.blockDim = dim3((unsigned)threads);
         cfg.dynamicSmemBytes = (size_t)smem_bytes;
         cfg.stream = ctx->stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)cluster;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_dependent()
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)cluster;
+        attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
         cfg.attrs = attr;
-        cfg.numAttrs = cluster > 1 ? 1 : 0;
+        cfg.numAttrs = cluster > 1 ? 2 : 1;
         KernelTimer timer(ctx);
         FLAT_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kernel, kp));
         return FLAT_OK;

@@ -116,6 +116,30 @@ inline char *scratch_ptr(flat_ctx *ctx) { return static_cast<char *>(ctx->worksp
             return ::flat::fail((ctx), FLAT_ERR_EXECUTION, "%s: %s", #expr, cudaGetErrorString(e__)); \
     } while (0)
 
+// A kernel launched so that it may start while the kernel before it in the stream (one of this library's, launched by the
+// same call) is still running: it must execute grid_dependency_wait() before it reads what that kernel writes, and the
+// other one tells when its dependent may start with grid_dependency_launch().  Between two short kernels this hides
+// the launch and the second one's set-up.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
+                                    A &&...args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+#endif
+
 // ---- forward ---------------------------------------------------------------------------------
 // One parameter block serves every forward flavour: layouts are element strides, RoPE is two
 // switches plus three position domains, variable-length batches and paged K/V are optional

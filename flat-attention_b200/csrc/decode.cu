@@ -279,6 +279,7 @@ __global__ void __launch_bounds__(kMergeDims * GROUPS) merge_kernel(int parts, i
     const int dim = tid % kMergeDims, group = tid / kMergeDims;
     const int64_t row = blockIdx.x;
     int live = parts;
+    grid_dependency_wait();
     if (seq_offsets) {
         const int seq = (int)(row / rows_per_seq);
         live = (seq_offsets[seq + 1] - 1) / span_tokens - seq_offsets[seq] / span_tokens + 1;
@@ -342,15 +343,12 @@ template <typename T>
 int merge_chunks(flat_ctx *ctx, const DecodeParams &p) {
     if (p.kv_splits <= 1) return FLAT_OK;
     int64_t rows = (int64_t)p.num_seqs * p.q_heads;
-    int blocks = (int)rows;
-    if (p.kv_splits >= kMergeWideFrom)
-        merge_kernel<T, kMergeGroupsWide><<<blocks, kMergeDims * kMergeGroupsWide, 0, ctx->stream>>>(
-            p.kv_splits, rows, p.head_dim, p.partial_o, p.partial_lse, (T *)p.o, p.lse, p.context_lens, p.uniform_len,
-            p.chunk_tokens, p.q_heads, p.balanced ? p.seq_offsets : nullptr, p.span_tokens, rows * p.head_dim, rows);
-    else
-        merge_kernel<T, 1><<<blocks, kMergeDims, 0, ctx->stream>>>(
-            p.kv_splits, rows, p.head_dim, p.partial_o, p.partial_lse, (T *)p.o, p.lse, p.context_lens, p.uniform_len,
-            p.chunk_tokens, p.q_heads, p.balanced ? p.seq_offsets : nullptr, p.span_tokens, rows * p.head_dim, rows);
+    const bool wide = p.kv_splits >= kMergeWideFrom;
+    FLAT_CUDA_OK(ctx, launch_dependent(true, wide ? merge_kernel<T, kMergeGroupsWide> : merge_kernel<T, 1>, dim3((unsigned)rows),
+                                       wide ? kMergeDims * kMergeGroupsWide : kMergeDims, 0, ctx->stream, p.kv_splits, rows,
+                                       p.head_dim, p.partial_o, p.partial_lse, (T *)p.o, p.lse, p.context_lens, p.uniform_len,
+                                       p.chunk_tokens, p.q_heads, p.balanced ? p.seq_offsets : nullptr, p.span_tokens,
+                                       rows * p.head_dim, rows));
     ctx->launches += 1;
     FLAT_CUDA_OK(ctx, cudaGetLastError());
     return FLAT_OK;
