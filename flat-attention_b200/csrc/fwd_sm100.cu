@@ -50,6 +50,43 @@ constexpr int kMmaWarp = 9;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
+// At D = 64 the two products of a score cost the tensor pipe half of what they do at D = 128, and the special-function unit
+// (16 exponentials per clock and SM) becomes the bound: every kPolyEvery-th pair of scores takes 2^t from the FMA and
+// integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, D = 64: 137 us without, 133 / 127 / 138 us with every 8th /
+// 4th / 8 of 3 pairs.  At D = 128 the same costs time (the tensor pipe and the power limit bound there: a 32768-token
+// chunked prefill 18.5 -> 19.5 ms), so the flag follows D.
+constexpr int kPolyEvery = 4;
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+// 2^t of two scores, t <= 100: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds to an integer), 2^f as the minimax
+// polynomial of degree 5 (relative error 7.5e-8, 2.1e-7 as evaluated: that of ex2.approx), scaled by 2^n.  The
+// integer carries the exponent bias, so that its low byte shifted by 23 is 2^n; t below -127 gives exactly 0, NaN stays NaN.
+__device__ __forceinline__ void ex2_poly(float &t0, float &t1) {
+    constexpr float kRound = 12582912.f + 127.f;
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(t0) : "f"(-127.f));
+    asm("max.NaN.f32 %0, %0, %1;" : "+f"(t1) : "f"(-127.f));
+    const uint64_t t = pack2(t0, t1);
+    uint64_t n, f, r, scale;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(n) : "l"(t), "l"(pack2(kRound, kRound)));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(f) : "l"(n), "l"(pack2(-kRound, -kRound)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(f) : "l"(pack2(-1.f, -1.f)), "l"(t));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;"
+        : "=l"(r)
+        : "l"(f), "l"(pack2(0x1.5c08e6p-10f, 0x1.5c08e6p-10f)), "l"(pack2(0x1.3d0c52p-7f, 0x1.3d0c52p-7f)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(r) : "l"(f), "l"(pack2(0x1.c6b6e4p-5f, 0x1.c6b6e4p-5f)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(r) : "l"(f), "l"(pack2(0x1.ebf918p-3f, 0x1.ebf918p-3f)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(r) : "l"(f), "l"(pack2(0x1.62e428p-1f, 0x1.62e428p-1f)));
+    asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(r) : "l"(f), "l"(pack2(1.f, 1.f)));
+    uint32_t n0, n1;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(n0), "=r"(n1) : "l"(n));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(scale) : "r"(n0 << 23), "r"(n1 << 23));
+    asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(r) : "l"(scale));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(r));
+}
 
 // Debug timeline (compiled in with -DFLAT_TRACE): clock64 stamps of CTA FLAT_TRACE_BLOCK (default 0), written to the buffer whose
 // address is given in the environment variable FLAT_TRACE_PTR.  Layout [role 0..2][iteration 0..63][slot 0..7].
@@ -709,7 +746,13 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                             if constexpr (ALIBI) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(nm2) : "l"(step2));
                             float t0, t1;
                             asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t2));
-                            const float p0 = ex2(t0), p1 = ex2(t1);
+                            float p0 = t0, p1 = t1;
+                            if (D == 64 && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
+                                ex2_poly(p0, p1);
+                            } else {
+                                p0 = ex2(t0);
+                                p1 = ex2(t1);
+                            }
                             asm("mov.b64 %0, {%1, %2};" : "=l"(p2) : "f"(p0), "f"(p1));
                             if (i & 2) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum3) : "l"(p2));
                             else asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum2) : "l"(p2));
