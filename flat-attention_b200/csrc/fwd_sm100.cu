@@ -52,7 +52,7 @@ constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
 // At D = 64 the two products of a score cost the tensor pipe half of what they do at D = 128, and the special-function unit
 // (16 exponentials per clock and SM) becomes the bound: every kPolyEvery-th pair of scores takes 2^t from the FMA and
-// integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, D = 64: 137 us without, 133 / 127 / 138 us with every 8th /
+// integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, D = 64: 135 us without, 133 / 129 / 138 us with every 8th /
 // 4th / 8 of 3 pairs.  At D = 128 the same costs time (the tensor pipe and the power limit bound there: a 32768-token
 // chunked prefill 18.5 -> 19.5 ms), so the flag follows D.
 constexpr int kPolyEvery = 4;
@@ -186,7 +186,7 @@ template <int D, bool CONVK> struct Cfg {
     static constexpr int kTileBytes = kBoxes * kBoxBytes;  // one Q / K / V tile
     static constexpr int kStages = D == 128 ? 4 : 8;  // K/V ring entries
     static constexpr int kOutStageBytes = kTileRows * 128;  // one box of the O tile: 128 rows x 64 columns of 16 bits
-    static constexpr int kBars = 2 + 3 * kStages + 10;
+    static constexpr int kBars = 2 + 3 * kStages + 12;
     static constexpr int kSmemBytes = (2 + kStages) * kTileBytes + 2 * kOutStageBytes + kBars * 8 + 16 + 32 + 1024;
     static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
 };
@@ -327,6 +327,12 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
     auto q_ready = [&](int w) { return bar0 + 8u * (8 + 2 * C::kStages + w); };
     auto q_empty = [&](int w) { return bar0 + 8u * (10 + 2 * C::kStages + w); };
     auto k_ready = [&](int s) { return bar0 + 8u * (12 + 2 * C::kStages + s); };  // K tile converted (CONVK)
+    auto p_part = [&](int w) { return bar0 + 8u * (12 + 3 * C::kStages + w); };   // the first kEarlyKeys columns of P are written
+    // ALiBi's exponent pass is longer (the addend advances with the columns), and the value product of the first 96 keys is
+    // issued while the last 32 are still being exponentiated: B = 2, 1000 new rows against 3000 keys, 32 / 8 heads, D = 128,
+    // 118.5 -> 111.0 us.  Without the bias the second wait costs the issuing thread more than the overlap gives (587 -> 606 us
+    // for B = 4, N = 4096).
+    constexpr int kEarlyKeys = ALIBI ? 96 : 0;
 
     const int warp = warp_index_uniform();
     const int lane = threadIdx.x & 31;
@@ -338,6 +344,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             mbar_init(q_full(w), 1);
             mbar_init(s_full(w), 1);
             mbar_init(p_full(w), 4);
+            mbar_init(p_part(w), 4);
             mbar_init(o_final(w), 1);
             mbar_init(q_ready(w), 4);
             mbar_init(q_empty(w), 1);
@@ -473,10 +480,10 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                     mma_ss_off(tmem_base + col_s[w], a_desc, b_desc, off16, p.idesc_qk, kk > 0);
                 }
             };
-            auto issue_pv = [&](int w, int stage, int j) {
+            auto issue_pv = [&](int w, int stage, int j, int first, int last) {  // 16-key steps [first, last)
                 const uint64_t b_desc = make_smem_desc(smem_u32(kv_s + stage * C::kTileBytes), C::kBoxBytes, 1024);
 #pragma unroll
-                for (int kk = 0; kk < kTileRows / 16; ++kk)
+                for (int kk = first; kk < last; ++kk)
                     mma_ts_off(tmem_base + col_o[w], tmem_base + col_s[w] + kk * 8, b_desc, kk * (16 * 128 >> 4), p.idesc_pv,
                                (j > 0 || kk > 0));
             };
@@ -523,12 +530,18 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                     bool k_next = false;
                     for (int w = 0; w < 2 && ok; ++w) {
                         if (j >= it.n_tiles[w]) continue;
+                        if constexpr (kEarlyKeys > 0) {
+                            wait(p_part(w), p_waits[w] & 1, 235 + w);
+                            if (!ok) break;
+                            tc_fence_after();
+                            issue_pv(w, stage_of(iv), j, 0, kEarlyKeys / 16);
+                        }
                         wait(p_full(w), p_waits[w] & 1, 230 + w);
                         if (!ok) break;
                         ++p_waits[w];
                         TRACE(2, j, w * 4 + 0);
                         tc_fence_after();
-                        issue_pv(w, stage_of(iv), j);
+                        issue_pv(w, stage_of(iv), j, kEarlyKeys / 16, kTileRows / 16);
                         TRACE(2, j, w * 4 + 1);
                         if (w == 1 || j >= it.n_tiles[1]) tc_commit(kv_empty(stage_of(iv)));  // last reader of V_j
                         if (j + 1 < it.n_tiles[w]) {
@@ -765,6 +778,12 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                             }
                         }
                         tmem_st16(t_s + c * 16, pk);
+                        if (kEarlyKeys > 0 && (c + 1) * 32 == kEarlyKeys) {
+                            tc_wait_st();
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(p_part(w));
+                        }
                     }
                     {
                         float s0, s1, s2f, s3;
