@@ -152,6 +152,7 @@ struct ForwardCall {
 
 int launch_forward(flat_ctx *ctx, int dtype, const FwdParams &p) {
     if (storage16(dtype) && forward_sm100_supported(p)) return launch_forward_sm100(ctx, p);
+    if (dtype == FLAT_F32 && forward_f32_supported(p)) return launch_forward_f32(ctx, p);
     return launch_forward_simt(ctx, dtype, p);
 }
 
@@ -290,7 +291,7 @@ int forward_common(flat_ctx *ctx, const ForwardCall &call, const flat_attention_
         FLAT_CUDA_OK(ctx, cudaMemcpyAsync(ctx->workspace, call.alibi_slopes, call.alibi_count * sizeof(float),
                                           cudaMemcpyHostToDevice, ctx->stream));
         p.alibi_slopes = static_cast<const float *>(ctx->workspace);
-        return tensor_path ? launch_forward_sm100(ctx, p) : launch_forward_simt(ctx, call.dtype, p);
+        return launch_forward(ctx, call.dtype, p);
     }
     if (params_out) {
         *params_out = p;
@@ -893,7 +894,8 @@ int32_t flat_forward_runtime_telemetry(flat_ctx *ctx, int32_t dtype, int32_t lay
         return FLAT_OK;
     }
     out->kernel_id = FLAT_KERNEL_FORWARD_GENERIC;
-    forward_simt_geometry(p, &out->query_rows, &out->kv_rows, out->workgroups);
+    if (dtype == FLAT_F32 && forward_f32_supported(p)) forward_f32_geometry(ctx, p, &out->query_rows, &out->kv_rows, out->workgroups);
+    else forward_simt_geometry(p, &out->query_rows, &out->kv_rows, out->workgroups);
     out->dispatch_count = 1;
     out->has_fallback_reason = 1;
     if (!storage16(dtype))

@@ -175,7 +175,13 @@ struct FwdParams {
 
 // Generic SIMT forward (f32 arithmetic; T = float or __nv_bfloat16 storage).
 int launch_forward_simt(flat_ctx *ctx, int dtype, const FwdParams &p);
-// tile geometry and grid of the two forward kernels for a parameter block (telemetry; nothing is launched)
+// f32, head_dim 64 / 128, uniform lengths, contiguous K/V: register-tiled f32 FMAs.
+bool forward_f32_supported(const FwdParams &p);
+void forward_f32_geometry(const flat_ctx *ctx, const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3]);
+int launch_forward_f32(flat_ctx *ctx, const FwdParams &p);
+// (cos, sin) of `rows` positions from pos_off on, [rows][half_dim], from the context's tables or computed now on its stream.
+int rope_table(flat_ctx *ctx, const float *inv_freq, int half_dim, int rows, int64_t pos_off, const float2 **out);
+// tile geometry and grid of the forward kernels for a parameter block (telemetry; nothing is launched)
 void forward_simt_geometry(const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3]);
 void forward_sm100_geometry(const flat_ctx *ctx, const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3],
                             uint32_t *dispatches);

@@ -1,0 +1,423 @@
+// f32 forward for head_dim 64 and 128: register-tiled products on the FMA pipe.
+//
+// Bound by the f32 FMA pipe (128 lanes per clock and SM; the tensor cores have no f32 mode of this precision), so both
+// products are laid out to feed it: a CTA owns 64 query rows of one (batch, q_head) and streams K/V tiles of 64 keys
+// through shared memory; 128 threads hold 4 rows x 8 keys of the scores and 4 rows x D/8 columns of O in registers, so
+// a 16-byte shared-memory read serves 10 to 13 multiply-adds (the row-per-four-threads kernel in fwd_simt.cu reads one
+// K and one V vector for four).  Products run as packed f32x2 FMAs: a score is two running sums (even and odd
+// dimensions) over each half of the head dimension, an O pair is two adjacent columns.
+// Few query blocks leave most SMs idle and the causal diagonal makes them uneven, so the KV tiles of a query block are
+// dealt to a cluster of up to 8 CTAs, which combine their (max, sum, O) through distributed shared memory in rank
+// order: one launch, no scratch, bitwise repeatable.  8 / 2 heads, 512 rows, D = 128, causal, RoPE: 219 us with the kernel of
+// fwd_simt.cu, 45 us here; 2 x 2048 rows, 16 / 4 heads 3470 us and 1180 us (29 TFLOP/s).
+// RoPE: K and Q are rotated on the way into shared memory with the (cos, sin) table of the call's positions; without a
+// table (a call under stream capture, where none can be allocated) the same sincosf runs here.
+#include <cooperative_groups.h>
+
+#include <type_traits>
+
+#include "common.h"
+
+namespace flat {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kRows = 64;    // query rows per CTA
+constexpr int kKeys = 64;    // keys per tile
+constexpr int kThreads = 128;
+constexpr int kRowsPerThread = 4;   // ty + 16 r
+constexpr int kKeysPerThread = 8;   // tx + 8 i
+constexpr int kMaxCluster = 8;
+
+struct F32Params {
+    FwdParams f;
+    const float2 *q_table, *k_table;  // (cos, sin) of query row / key r, pair j at [r * D/2 + j]
+};
+
+template <int D> struct Tile {
+    static constexpr int kStride = D + 4;       // floats per Q / K row: 8 rows cover all banks
+    static constexpr int kPStride = kKeys + 4;  // P takes K's place
+    static constexpr int kQ = 0, kK = kRows * kStride, kV = kK + kKeys * kStride, kStat = kV + kKeys * D;
+    static constexpr int kFloats = kStat + 2 * kRows;
+    static_assert(kPStride <= kStride, "P fits K's rows");
+};
+
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(uint64_t v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(uint64_t &d, uint64_t a, uint64_t b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ void mul2(uint64_t &d, uint64_t a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(a)); }
+
+__device__ __forceinline__ void cp_async16(float *dst, const float *src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+                 "l"(src), "r"(live ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// 64 rows of `src` (row stride rs) into dst (row stride `stride`) with cp.async; rows from `live` on become zero.
+template <int D>
+__device__ __forceinline__ void load_rows(float *dst, int stride, const float *src, int64_t rs, int64_t first, int live) {
+    constexpr int kVec = D / 4;
+#pragma unroll
+    for (int u = 0; u < 64 * kVec / kThreads; ++u) {
+        const int i = u * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+        cp_async16(dst + r * stride + 4 * v, src + (first + (r < live ? r : 0)) * rs + 4 * v, r < live);
+    }
+}
+// The same with the interleaved pairs of row r rotated by the table's row first + r, or by the angle of position
+// pos0 + first + r.  A thread's loads are in flight eight at a time: the tile waits for the last of them.
+template <int D>
+__device__ __forceinline__ void load_rotated_rows(float *dst, int stride, const float *src, int64_t rs, int64_t first, int live,
+                                                  const float2 *table, int64_t pos0, const float *inv_freq) {
+    constexpr int kVec = D / 4, kBatch = 8;
+#pragma unroll
+    for (int u0 = 0; u0 < 64 * kVec / kThreads; u0 += kBatch) {
+        float4 x[kBatch], cs[kBatch];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+            x[u] = *reinterpret_cast<const float4 *>(src + (first + (r < live ? r : 0)) * rs + 4 * v);
+        }
+        if (table) {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+                cs[u] = *reinterpret_cast<const float4 *>(table + (first + (r < live ? r : 0)) * (D / 2) + 2 * v);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < kBatch; ++u) {
+                const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+                const float pos = (float)(pos0 + first + r);
+                sincosf(__fmul_rn(pos, inv_freq[2 * v]), &cs[u].y, &cs[u].x);
+                sincosf(__fmul_rn(pos, inv_freq[2 * v + 1]), &cs[u].w, &cs[u].z);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+            const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+            const float4 y = x[u], c = cs[u];
+            *reinterpret_cast<float4 *>(dst + r * stride + 4 * v) =
+                r < live ? make_float4(y.x * c.x - y.y * c.y, y.x * c.y + y.y * c.x, y.z * c.z - y.w * c.w, y.z * c.w + y.w * c.z)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+}
+
+template <int D, bool ALIBI>
+__global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_constant__ F32Params fp) {
+    using T = Tile<D>;
+    constexpr int kCols = D / 32;  // float4 columns of O per thread and row
+    const FwdParams &p = fp.f;
+    extern __shared__ __align__(16) float smem[];
+    float *qs = smem + T::kQ, *ks = smem + T::kK, *vs = smem + T::kV, *stat = smem + T::kStat;
+    float *ps = ks;
+
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
+    const int q_blocks = (int)gridDim.x / parts;
+    const int r0 = (q_blocks - 1 - (int)blockIdx.x / parts) * kRows;  // long query blocks first
+    const int h = blockIdx.y, b = blockIdx.z, kvh = h / p.group;
+
+    const int rows = min(kRows, p.q_len - r0);
+    int64_t visible = p.kv_len;  // keys the block's last row sees
+    if (p.causal) visible = min(visible, p.causal_off + r0 + rows);
+    const int n_tiles = (int)((visible + kKeys - 1) / kKeys);
+    const int t_begin = (int)((int64_t)part * n_tiles / parts), t_end = (int)((int64_t)(part + 1) * n_tiles / parts);
+
+    const float *kbase = (const float *)p.k + (int64_t)b * p.kv_bs + (int64_t)kvh * p.kv_hs;
+    const float *vbase = (const float *)p.v + (int64_t)b * p.kv_bs + (int64_t)kvh * p.kv_hs;
+
+    const float slope = ALIBI ? p.alibi_slopes[h] : 0.f;
+    uint64_t o[kRowsPerThread][2 * kCols];
+    float m[kRowsPerThread], l[kRowsPerThread];  // l: this thread's keys only
+#pragma unroll
+    for (int r = 0; r < kRowsPerThread; ++r) {
+        m[r] = -INFINITY;
+        l[r] = 0.f;
+#pragma unroll
+        for (int c = 0; c < 2 * kCols; ++c) o[r][c] = 0;
+    }
+
+    if (t_begin < t_end) {
+        const float *qbase = (const float *)p.q + (int64_t)b * p.q_bs + (int64_t)h * p.q_hs;
+        if (p.rope_q) load_rotated_rows<D>(qs, T::kStride, qbase, p.q_rs, r0, rows, fp.q_table, p.q_rope_off, p.inv_freq);
+        else load_rows<D>(qs, T::kStride, qbase, p.q_rs, r0, rows);
+    }
+    for (int t = t_begin; t < t_end; ++t) {
+        const int64_t k0 = (int64_t)t * kKeys;
+        const int live = (int)min((int64_t)kKeys, visible - k0);
+        // V is asked for first where K takes a detour through registers, and arrives during the score product
+        if (!p.rope_k) load_rows<D>(ks, T::kStride, kbase, p.kv_rs, k0, live);
+        cp_async_commit();
+        load_rows<D>(vs, D, vbase, p.kv_rs, k0, live);
+        cp_async_commit();
+        if (p.rope_k) load_rotated_rows<D>(ks, T::kStride, kbase, p.kv_rs, k0, live, fp.k_table, p.k_rope_off, p.inv_freq);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");  // Q and K
+        __syncthreads();
+
+        // S = Q K^T: two half products of D/2 dimensions, each as sums over even and over odd dimensions
+        float s[kRowsPerThread][kKeysPerThread];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            uint64_t acc[kRowsPerThread][kKeysPerThread];
+#pragma unroll
+            for (int r = 0; r < kRowsPerThread; ++r)
+#pragma unroll
+                for (int i = 0; i < kKeysPerThread; ++i) acc[r][i] = 0;
+            const float *qp = qs + ty * T::kStride + half * (D / 2), *kp = ks + tx * T::kStride + half * (D / 2);
+#pragma unroll 2
+            for (int d = 0; d < D / 2; d += 4) {
+                ulonglong2 qv[kRowsPerThread];
+#pragma unroll
+                for (int r = 0; r < kRowsPerThread; ++r) qv[r] = *reinterpret_cast<const ulonglong2 *>(qp + 16 * r * T::kStride + d);
+#pragma unroll
+                for (int i = 0; i < kKeysPerThread; ++i) {
+                    const ulonglong2 kv = *reinterpret_cast<const ulonglong2 *>(kp + 8 * i * T::kStride + d);
+#pragma unroll
+                    for (int r = 0; r < kRowsPerThread; ++r) {
+                        fma2(acc[r][i], qv[r].x, kv.x);
+                        fma2(acc[r][i], qv[r].y, kv.y);
+                    }
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < kRowsPerThread; ++r)
+#pragma unroll
+                for (int i = 0; i < kKeysPerThread; ++i) {
+                    const float2 e = unpack2(acc[r][i]);
+                    s[r][i] = half ? s[r][i] + (e.x + e.y) : e.x + e.y;
+                }
+        }
+        __syncthreads();  // K has been read: P takes its place
+
+#pragma unroll
+        for (int r = 0; r < kRowsPerThread; ++r) {
+            const int row = ty + 16 * r;
+            int64_t limit = p.kv_len;  // visible keys of this row
+            if (p.causal) limit = min(limit, p.causal_off + r0 + row + 1);
+            const int lim = (int)min((int64_t)kKeys, limit - k0);
+            float mx = -INFINITY;
+            // ALiBi: the position difference is formed in integers and rounded to f32 once, like the f64 difference of
+            // src/attention_bias.rs:93-94
+            const int64_t bias0 = ALIBI ? p.alibi_kv_off - p.alibi_q_off - (r0 + row) + k0 + tx : 0;
+#pragma unroll
+            for (int i = 0; i < kKeysPerThread; ++i) {
+                float sc = s[r][i] * p.scale;
+                if constexpr (ALIBI) sc = __fadd_rn(sc, __fmul_rn(slope, (float)(bias0 + 8 * i)));
+                s[r][i] = tx + 8 * i < lim ? sc : -INFINITY;
+                mx = fmaxf(mx, s[r][i]);
+            }
+#pragma unroll
+            for (int w = 1; w < 8; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            const bool any = mx != -INFINITY;  // a row none of whose keys counts in this tile keeps its state
+            const float m_new = fmaxf(m[r], mx);
+            const float alpha = !any ? 1.f : m[r] == -INFINITY ? 0.f : expf(m[r] - m_new);
+            m[r] = m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < kKeysPerThread; ++i) {
+                const float e = !any || s[r][i] == -INFINITY ? 0.f : expf(s[r][i] - m_new);
+                sum += e;
+                ps[row * T::kPStride + tx + 8 * i] = e;
+            }
+            l[r] = l[r] * alpha + sum;
+            const uint64_t a2 = pack2(alpha, alpha);
+#pragma unroll
+            for (int c = 0; c < 2 * kCols; ++c) mul2(o[r][c], a2);
+        }
+        cp_async_wait_all();
+        __syncthreads();  // V is there; a row of P is written and read by the same eight lanes
+
+        // O += P V
+#pragma unroll 2
+        for (int k = 0; k < kKeys; k += 4) {
+            float4 pv[kRowsPerThread];
+#pragma unroll
+            for (int r = 0; r < kRowsPerThread; ++r)
+                pv[r] = *reinterpret_cast<const float4 *>(ps + (ty + 16 * r) * T::kPStride + k);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                ulonglong2 vv[kCols];
+#pragma unroll
+                for (int c = 0; c < kCols; ++c) vv[c] = *reinterpret_cast<const ulonglong2 *>(vs + (k + e) * D + 4 * tx + 32 * c);
+#pragma unroll
+                for (int r = 0; r < kRowsPerThread; ++r) {
+                    const float x = e == 0 ? pv[r].x : e == 1 ? pv[r].y : e == 2 ? pv[r].z : pv[r].w;
+                    const uint64_t x2 = pack2(x, x);
+#pragma unroll
+                    for (int c = 0; c < kCols; ++c) {
+                        fma2(o[r][2 * c], x2, vv[c].x);
+                        fma2(o[r][2 * c + 1], x2, vv[c].y);
+                    }
+                }
+            }
+        }
+        __syncthreads();  // the next tile overwrites P and V
+    }
+
+#pragma unroll
+    for (int r = 0; r < kRowsPerThread; ++r)
+#pragma unroll
+        for (int w = 1; w < 8; w <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], w);
+
+    float *obase = (float *)p.o + (int64_t)b * p.o_bs + (int64_t)h * p.o_hs;
+    float *lse = p.lse + ((int64_t)b * p.q_heads + h) * p.lse_hs;
+    if (parts == 1) {
+#pragma unroll
+        for (int r = 0; r < kRowsPerThread; ++r) {
+            const int row = ty + 16 * r;
+            if (row >= rows) continue;
+            const float inv = 1.0f / l[r];
+#pragma unroll
+            for (int c = 0; c < kCols; ++c) {
+                const float2 a = unpack2(o[r][2 * c]), e = unpack2(o[r][2 * c + 1]);
+                *reinterpret_cast<float4 *>(obase + (int64_t)(r0 + row) * p.o_rs + 4 * tx + 32 * c) =
+                    make_float4(a.x * inv, a.y * inv, e.x * inv, e.y * inv);
+            }
+            if (tx == 0) lse[r0 + row] = m[r] + logf(l[r]);
+        }
+        return;
+    }
+
+    // ---- combine the cluster's parts: each CTA leaves (max, sum) and its O rows in its own shared memory (over Q and
+    // K/P, which are read no more), and finishes its share of the 16-byte vectors, adding the parts in rank order
+    float *os = smem;
+    if (tx == 0)
+#pragma unroll
+        for (int r = 0; r < kRowsPerThread; ++r) {
+            stat[2 * (ty + 16 * r)] = m[r];
+            stat[2 * (ty + 16 * r) + 1] = l[r];
+        }
+#pragma unroll
+    for (int r = 0; r < kRowsPerThread; ++r)
+#pragma unroll
+        for (int c = 0; c < kCols; ++c)
+            *reinterpret_cast<ulonglong2 *>(os + (ty + 16 * r) * D + 4 * tx + 32 * c) = make_ulonglong2(o[r][2 * c], o[r][2 * c + 1]);
+    cluster.sync();
+    constexpr int kVecs = kRows * (D / 4);
+    for (int i = part * kVecs / parts + threadIdx.x; i < (part + 1) * kVecs / parts; i += kThreads) {
+        const int row = i / (D / 4), v = i % (D / 4);
+        if (row >= rows) continue;
+        float mx = -INFINITY;
+        for (int x = 0; x < parts; ++x) mx = fmaxf(mx, cluster.map_shared_rank(stat, x)[2 * row]);
+        float sum = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int x = 0; x < parts; ++x) {
+            const float2 ml = *reinterpret_cast<const float2 *>(cluster.map_shared_rank(stat, x) + 2 * row);
+            const float w = ml.x == -INFINITY ? 0.f : expf(ml.x - mx);
+            const float4 part_o = *reinterpret_cast<const float4 *>(cluster.map_shared_rank(os, x) + row * D + 4 * v);
+            sum = fmaf(w, ml.y, sum);
+            acc = make_float4(fmaf(w, part_o.x, acc.x), fmaf(w, part_o.y, acc.y), fmaf(w, part_o.z, acc.z), fmaf(w, part_o.w, acc.w));
+        }
+        const float inv = 1.0f / sum;
+        *reinterpret_cast<float4 *>(obase + (int64_t)(r0 + row) * p.o_rs + 4 * v) =
+            make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+        if (v == 0) lse[r0 + row] = mx + logf(sum);
+    }
+    cluster.sync();  // a CTA's shared memory outlives its readers
+}
+
+template <int D>
+int launch(flat_ctx *ctx, const F32Params &fp, int parts) {
+    const FwdParams &p = fp.f;
+    const int smem = Tile<D>::kFloats * (int)sizeof(float);
+    auto *kernel = p.alibi_slopes ? fwd_f32_kernel<D, true> : fwd_f32_kernel<D, false>;
+    FLAT_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)((p.q_len + kRows - 1) / kRows * parts), (unsigned)p.q_heads, (unsigned)p.batch);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)parts;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FLAT_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kernel, fp));
+    ctx->launches += 1;
+    return FLAT_OK;
+}
+
+// CTAs per query block.  A CTA costs its tiles and about kOverheadTiles more (its Q rows, its share of the combination); the
+// call lasts as long as its longest CTA, and as long as everything takes over the CTAs that run at once (two per SM).
+// The cluster size with the smaller of the two maxima is taken.  8 heads, D = 128, causal: 512 rows 45 us with 4 CTAs (49
+// with 8, 57 us before loads were batched), 1024 rows 118 us with 4 (131 with 2), 2048 rows 400 us with 2 (472 with 1).
+constexpr int kOverheadTiles = 2;
+int cluster_parts(const flat_ctx *ctx, const FwdParams &p) {
+    const int64_t blocks = (p.q_len + kRows - 1) / kRows;
+    int64_t tiles = 0, longest = 0;
+    for (int64_t i = 0; i < blocks; ++i) {
+        int64_t keys = p.kv_len;
+        if (p.causal) keys = std::min<int64_t>(keys, p.causal_off + std::min<int64_t>((i + 1) * kRows, p.q_len));
+        const int64_t n = (keys + kKeys - 1) / kKeys;
+        tiles += n;
+        longest = std::max(longest, n);
+    }
+    tiles *= (int64_t)p.q_heads * p.batch;
+    const int64_t slots = 2 * (int64_t)ctx->sm_count, all = blocks * p.q_heads * p.batch;
+    int parts = 1;
+    int64_t best = INT64_MAX;
+    for (int c = 1; c <= kMaxCluster && c <= longest; ++c) {
+        const int64_t cost = std::max(slots * (kOverheadTiles + (longest + c - 1) / c), tiles + kOverheadTiles * all * c);
+        if (cost < best) best = cost, parts = c;
+    }
+    return parts;
+}
+
+}  // namespace
+
+bool forward_f32_supported(const FwdParams &p) {
+    if (p.head_dim != 64 && p.head_dim != 128) return false;
+    if (p.varlen || p.page_table) return false;
+    if (p.q_len < 16) return false;  // a block has 64 rows: a few rows waste it
+    const void *ptrs[] = {p.q, p.k, p.v, p.o};
+    for (const void *x : ptrs)
+        if (reinterpret_cast<uintptr_t>(x) & 15) return false;
+    const int64_t strides[] = {p.q_bs, p.q_hs, p.q_rs, p.kv_bs, p.kv_hs, p.kv_rs, p.o_bs, p.o_hs, p.o_rs};
+    for (int64_t s : strides)
+        if (s % 4 != 0) return false;
+    return true;
+}
+
+void forward_f32_geometry(const flat_ctx *ctx, const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3]) {
+    *query_rows = kRows;
+    *kv_rows = kKeys;
+    grid[0] = (uint32_t)((p.q_len + kRows - 1) / kRows * cluster_parts(ctx, p));
+    grid[1] = (uint32_t)p.q_heads;
+    grid[2] = (uint32_t)p.batch;
+}
+
+int launch_forward_f32(flat_ctx *ctx, const FwdParams &p) {
+    if (p.q_heads > 65535 || p.batch > 65535)
+        return fail(ctx, FLAT_ERR_DISPATCH_LIMIT, "grid dimension %d exceeds 65535", p.q_heads > 65535 ? p.q_heads : p.batch);
+    F32Params fp{};
+    fp.f = p;
+    // where no table is to be had (a capturing stream allows no allocation, the device may be full) or it would be
+    // larger than 64 MiB, the kernel evaluates the angles itself, with the same result
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    FLAT_CUDA_OK(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
+    const int64_t row_bytes = p.head_dim / 2 * (int64_t)sizeof(float2);
+    if (capture == cudaStreamCaptureStatusNone && std::max(p.q_len, p.kv_len) * row_bytes <= (64ll << 20)) {
+        if (p.rope_q && rope_table(ctx, p.inv_freq, p.head_dim / 2, p.q_len, p.q_rope_off, &fp.q_table)) cudaGetLastError();
+        if (p.rope_k && rope_table(ctx, p.inv_freq, p.head_dim / 2, p.kv_len, p.k_rope_off, &fp.k_table)) cudaGetLastError();
+    }
+    const int parts = cluster_parts(ctx, p);
+    return p.head_dim == 128 ? launch<128>(ctx, fp, parts) : launch<64>(ctx, fp, parts);
+}
+
+}  // namespace flat

@@ -1,7 +1,7 @@
 // Generic SIMT forward: f32 arithmetic, f32 or bf16 storage, every layout and mode of the
 // forward contract (head-major / projection strides, rectangular shapes, three position domains,
 // optional RoPE on Q and/or K, padded variable-length batches, K/V read through a page table).
-// It is the f32 parity kernel and the catch-all for shapes the tcgen05 kernel does not take.
+// It is the catch-all for shapes that neither the tcgen05 kernel nor the register-tiled f32 kernel takes.
 //
 // Mapping: one CTA = 32 consecutive query rows of one (batch, q_head); 4 threads share a row, each
 // owning every 4th float4 chunk of the head dimension.  K/V tiles of 32 keys are staged (and, when

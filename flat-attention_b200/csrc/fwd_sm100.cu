@@ -1145,12 +1145,14 @@ __global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *__re
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+}  // namespace
+
 // (cos, sin) table of `rows` positions starting at pos_off, from the context's cache or computed now on its stream.
-int rope_table(flat_ctx *ctx, const InvFreq &f, int half_dim, int rows, int64_t pos_off, const float2 **out) {
+int rope_table(flat_ctx *ctx, const float *inv_freq, int half_dim, int rows, int64_t pos_off, const float2 **out) {
     flat_ctx::RopeTable *slot = nullptr;
     for (auto &t : ctx->rope_tables) {
         if (t.rows >= rows && t.half_dim == half_dim && t.pos_off == pos_off &&
-            std::memcmp(t.inv_freq, f.f, sizeof(float) * half_dim) == 0) {
+            std::memcmp(t.inv_freq, inv_freq, sizeof(float) * half_dim) == 0) {
             t.last_use = ++ctx->rope_clock;
             *out = static_cast<const float2 *>(t.dev);
             return FLAT_OK;
@@ -1167,10 +1169,12 @@ int rope_table(flat_ctx *ctx, const InvFreq &f, int half_dim, int rows, int64_t 
         slot->bytes = bytes;
     }
     const int64_t n = (int64_t)rows * half_dim;
+    InvFreq f{};
+    std::memcpy(f.f, inv_freq, sizeof(float) * half_dim);
     rope_table_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, ctx->stream>>>(
         static_cast<float2 *>(slot->dev), rows, half_dim, pos_off, f);
     ctx->launches += 1;
-    std::memcpy(slot->inv_freq, f.f, sizeof(float) * half_dim);
+    std::memcpy(slot->inv_freq, inv_freq, sizeof(float) * half_dim);
     slot->half_dim = half_dim;
     slot->rows = rows;
     slot->pos_off = pos_off;
@@ -1178,8 +1182,6 @@ int rope_table(flat_ctx *ctx, const InvFreq &f, int half_dim, int rows, int64_t 
     *out = static_cast<const float2 *>(slot->dev);
     return FLAT_OK;
 }
-
-}  // namespace
 
 bool forward_sm100_supported(const FwdParams &p) {
     if (p.head_dim != 64 && p.head_dim != 128) return false;
@@ -1296,18 +1298,16 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     char *scratch = scratch_ptr(ctx);
     const float2 *q_table = nullptr;
     if (p.rope_q) {
-        InvFreq f;
-        std::memcpy(f.f, p.inv_freq, sizeof f.f);
         __half *rk = reinterpret_cast<__half *>(scratch);
         if (p.varlen) {
             const int rows = (int)(p.varlen_rope_max - p.varlen_rope_min) + p.q_len;
-            if ((st = rope_table(ctx, f, D / 2, rows, p.varlen_rope_min, &q_table))) return st;
-        } else if ((st = rope_table(ctx, f, D / 2, p.q_len, p.q_rope_off, &q_table))) {
+            if ((st = rope_table(ctx, p.inv_freq, D / 2, rows, p.varlen_rope_min, &q_table))) return st;
+        } else if ((st = rope_table(ctx, p.inv_freq, D / 2, p.q_len, p.q_rope_off, &q_table))) {
             return st;
         }
         if (p.rope_k) {
             const float2 *kt = nullptr;
-            if ((st = rope_table(ctx, f, D / 2, p.kv_len, p.k_rope_off, &kt))) return st;
+            if ((st = rope_table(ctx, p.inv_freq, D / 2, p.kv_len, p.k_rope_off, &kt))) return st;
             const int batch_heads = p.batch * p.kv_heads;
             const dim3 blocks((unsigned)(((int64_t)p.kv_len * (D / 8) + 255) / 256),
                               (unsigned)std::min((batch_heads + kRotateHeads - 1) / kRotateHeads, 65535));
