@@ -996,36 +996,46 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
     }
 }
 
-// delta = dO . O and -LSE*log2(e).  A thread takes 8 elements (16 bytes) of a row of each tensor, head_dim / 8
-// neighbouring lanes share a row, so a warp covers 256 / head_dim rows with full-width loads.
+// delta = dO . O and -LSE*log2(e), one block per kPrepRows rows of a (batch, head), whose rows are padded to whole tiles.
+// Bound by the read of the two tensors: D / 8 neighbouring lanes share a row with 16-byte loads, and a thread has the loads
+// of kPrepFlight rows in flight.  The slots of rows past seq_len must hold finite values: with zeros the zero-filled
+// Q / dO rows contribute nothing.
+constexpr int kPrepFlight = 4;
+template <int D> constexpr int kPrepRows = kPrepFlight * 256 / (D / 8);
+template <int D>
 __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *__restrict__ d_out,
                                                        const __nv_bfloat16 *__restrict__ out, const float *__restrict__ lse,
-                                                       float *__restrict__ delta, float *__restrict__ neg_lse2, int64_t rows_pad,
-                                                       int head_dim, int seq_len, int seq_pad) {
+                                                       float *__restrict__ delta, float *__restrict__ neg_lse2, int seq_len,
+                                                       int seq_pad) {
     grid_dependency_launch();
-    const int lanes_per_row = head_dim / 8;  // 8 or 16
-    const int rows_per_block = 256 / lanes_per_row;
-    const int sub = threadIdx.x % lanes_per_row;
-    // rows of a (batch, head) are padded to whole tiles; the slots of rows past seq_len must hold finite values, and with
-    // zeros the zero-filled Q / dO rows contribute nothing
-    const int64_t dst = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / lanes_per_row;
-    const bool live = dst < rows_pad && dst % seq_pad < seq_len;
-    const int64_t row = dst / seq_pad * seq_len + dst % seq_pad;
-    float acc = 0.f;
-    if (live) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4 *>(d_out + row * head_dim) + sub);
-        const uint4 o = __ldg(reinterpret_cast<const uint4 *>(out + row * head_dim) + sub);
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, ow[4] = {o.x, o.y, o.z, o.w};
+    constexpr int kLanes = D / 8, kStep = 256 / kLanes;
+    static_assert(kTile % kPrepRows<D> == 0, "a block's rows lie in one (batch, head)");
+    const int64_t dst0 = (int64_t)blockIdx.x * kPrepRows<D>;
+    const int64_t bh = dst0 / seq_pad;
+    const int n0 = (int)(dst0 - bh * seq_pad) + threadIdx.x / kLanes, sub = threadIdx.x % kLanes;
+    uint4 a[kPrepFlight], o[kPrepFlight];
+#pragma unroll
+    for (int u = 0; u < kPrepFlight; ++u) {
+        const int64_t row = bh * seq_len + min(n0 + u * kStep, seq_len - 1);
+        a[u] = __ldg(reinterpret_cast<const uint4 *>(d_out + row * D) + sub);
+        o[u] = __ldg(reinterpret_cast<const uint4 *>(out + row * D) + sub);
+    }
+#pragma unroll
+    for (int u = 0; u < kPrepFlight; ++u) {
+        const int n = n0 + u * kStep;
+        const uint32_t aw[4] = {a[u].x, a[u].y, a[u].z, a[u].w}, ow[4] = {o[u].x, o[u].y, o[u].z, o[u].w};
+        float acc = 0.f;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             acc = fmaf(__uint_as_float(aw[e] << 16), __uint_as_float(ow[e] << 16), acc);
             acc = fmaf(__uint_as_float(aw[e] & 0xffff0000u), __uint_as_float(ow[e] & 0xffff0000u), acc);
         }
-    }
-    for (int w = lanes_per_row / 2; w >= 1; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
-    if (sub == 0 && dst < rows_pad) {
-        delta[dst] = acc;
-        neg_lse2[dst] = live ? -lse[row] * kLog2e : 0.f;
+#pragma unroll
+        for (int w = kLanes / 2; w >= 1; w >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, w);
+        if (sub == 0) {
+            delta[bh * seq_pad + n] = n < seq_len ? acc : 0.f;
+            neg_lse2[bh * seq_pad + n] = n < seq_len ? -lse[bh * seq_len + n] * kLog2e : 0.f;
+        }
     }
 }
 
@@ -1080,10 +1090,9 @@ int launch_backward_sm100(flat_ctx *ctx, const BwdParams &p) {
     const int64_t rows_pad = (int64_t)p.batch * p.q_heads * seq_pad;
     float *delta = reinterpret_cast<float *>(scratch_ptr(ctx));
     float *neg_lse2 = delta + rows_pad;
-    const int prep_rows_per_block = 256 / (D / 8);
-    bwd_prep_kernel<<<(unsigned)((rows_pad + prep_rows_per_block - 1) / prep_rows_per_block), 256, 0, ctx->stream>>>(
-        static_cast<const __nv_bfloat16 *>(p.d_out), static_cast<const __nv_bfloat16 *>(p.out), p.lse, delta, neg_lse2, rows_pad,
-        D, N, seq_pad);
+    auto *prep = D == 128 ? bwd_prep_kernel<128> : bwd_prep_kernel<64>;
+    prep<<<(unsigned)(rows_pad / (D == 128 ? kPrepRows<128> : kPrepRows<64>)), 256, 0, ctx->stream>>>(
+        static_cast<const __nv_bfloat16 *>(p.d_out), static_cast<const __nv_bfloat16 *>(p.out), p.lse, delta, neg_lse2, N, seq_pad);
     ctx->launches += 1;
 
     BwdKernelParams kp{};
