@@ -865,25 +865,26 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
 }
 #undef TRS
 
-// dQ from spilled dS^T tiles: one CTA owns 128 queries of one (batch, q_head) and streams, per visible key tile j, the
-// 32 KiB dS^T tile (one contiguous bulk copy: the tile sits in scratch in the swizzled layout it was staged in) and
-// the K_j tile; dQ += dS_ij K_j is eight SS MMAs (A = the dS^T tile read M-major, B = K_j read N-major).  No
-// elementwise work; the kernel is bound by the stream of dS^T tiles from HBM.  Warps 0-3 epilogue, 4 producer, 5 MMA.
-template <int D> struct DqSpillCfg {
+// dQ from spilled dS^T tiles: one CTA owns 128 queries of HEADS query heads of one KV head and streams, per visible key
+// tile j, the heads' 32 KiB dS^T tiles (one contiguous bulk copy each: a tile sits in scratch in the swizzled layout it
+// was staged in) and the K_j tile; dQ += dS_ij K_j is eight SS MMAs (A = the dS^T tile read M-major, B = K_j read
+// N-major).  No elementwise work; the kernel is bound by the stream of dS^T tiles from HBM, and K_j from L2 on top of it:
+// two heads that share K_j bring 48 instead of 64 KiB per dS^T tile into the SM.  Warps 0-3 epilogue, 4 producer, 5 MMA.
+template <int D, int HEADS> struct DqSpillCfg {
     static constexpr int kBoxes = D / 64;
     static constexpr int kBoxBytes = kTile * 128;
     static constexpr int kTileBytes = kBoxes * kBoxBytes;
     static constexpr int kDsBytes = 2 * kBoxBytes;
-    static constexpr int kStageBytes = kDsBytes + kTileBytes;
-    static constexpr int kStages = 3;
+    static constexpr int kStageBytes = HEADS * kDsBytes + kTileBytes;
+    static constexpr int kStages = HEADS == 1 ? 3 : 2;
     static constexpr int kBars = 2 * kStages + 1;
     static constexpr int kThreadsDq = 192;
     static constexpr int kSmemBytes = kStages * kStageBytes + kBars * 8 + 16;
 };
 
-template <int D>
-__global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_kernel(const __grid_constant__ BwdKernelParams p) {
-    using C = DqSpillCfg<D>;
+template <int D, int HEADS>
+__global__ void __launch_bounds__(DqSpillCfg<D, HEADS>::kThreadsDq, 1) bwd_dq_spill_kernel(const __grid_constant__ BwdKernelParams p) {
+    using C = DqSpillCfg<D, HEADS>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::kStages * C::kStageBytes);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + C::kBars);
@@ -894,14 +895,14 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
     const uint32_t acc_final = bar0 + 8u * (2 * C::kStages);
     const int warp = warp_index_uniform(), lane = threadIdx.x & 31;
 
-    // block -> (query tile, head, batch); late query tiles see the most keys and go first
-    const int lin = blockIdx.x;
-    const int tile_rank = lin / (p.q_heads * p.batch);
-    const int bh = lin % (p.q_heads * p.batch);
-    const int b = bh / p.q_heads, h = bh % p.q_heads;
+    // block -> (query tile, first head, batch); late query tiles see the most keys and go first
+    const int lin = blockIdx.x, head_groups = p.q_heads / HEADS;
+    const int tile_rank = lin / (head_groups * p.batch);
+    const int bh = lin % (head_groups * p.batch);
+    const int b = bh / head_groups, h = bh % head_groups * HEADS;
     const int t_own = p.causal ? p.n_tiles - 1 - tile_rank : tile_rank;
     const int n_iter = p.causal ? t_own + 1 : p.n_tiles;
-    constexpr uint32_t kTmemCols = D;  // 64 or 128: a power of two >= 32
+    constexpr uint32_t kTmemCols = HEADS * D;  // a power of two >= 32
 
     if (threadIdx.x == 0) {
         *abort_flag = (smem_u32(smem) & 1023u) ? 1 : 0;
@@ -935,9 +936,11 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
             }
             uint8_t *stage = smem + s * C::kStageBytes;
             mbar_expect_tx(rg_full(s), C::kStageBytes);
-            bulk_copy_g2s(smem_u32(stage), p.ds_spill + ds_tile_index(p, b, h, it, t_own) * C::kDsBytes, C::kDsBytes, rg_full(s));
+            for (int x = 0; x < HEADS; ++x)
+                bulk_copy_g2s(smem_u32(stage + x * C::kDsBytes), p.ds_spill + ds_tile_index(p, b, h + x, it, t_own) * C::kDsBytes,
+                              C::kDsBytes, rg_full(s));
             for (int kb = 0; kb < C::kBoxes; ++kb)
-                tma_load_4d(smem_u32(stage + C::kDsBytes + kb * C::kBoxBytes), &p.map_k, kb * 64, it * kTile, kvh, b, rg_full(s));
+                tma_load_4d(smem_u32(stage + HEADS * C::kDsBytes + kb * C::kBoxBytes), &p.map_k, kb * 64, it * kTile, kvh, b, rg_full(s));
         }
     } else if (warp == 5 && !*abort_flag && elect_one()) {
         // ================= MMA issuer =================
@@ -951,11 +954,13 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
             }
             tc_fence_after();
             const uint8_t *stage = smem + s * C::kStageBytes;
-            const uint64_t a_desc = make_smem_desc(smem_u32(stage), C::kBoxBytes, 1024);                // dS^T, M-major
-            const uint64_t b_desc = make_smem_desc(smem_u32(stage + C::kDsBytes), C::kBoxBytes, 1024);  // K_j, N-major
+            const uint64_t b_desc = make_smem_desc(smem_u32(stage + HEADS * C::kDsBytes), C::kBoxBytes, 1024);  // K_j, N-major
 #pragma unroll
-            for (int kk = 0; kk < kTile / 16; ++kk)
-                mma_ss_off(tmem_base, a_desc, b_desc, kk * (16 * 128 >> 4), p.idesc_dq, (it > 0 || kk > 0));
+            for (int i = 0; i < HEADS * (kTile / 16); ++i) {
+                const int x = i / (kTile / 16), kk = i % (kTile / 16);
+                const uint64_t a_desc = make_smem_desc(smem_u32(stage + x * C::kDsBytes), C::kBoxBytes, 1024);  // dS^T, M-major
+                mma_ss_off(tmem_base + x * D, a_desc, b_desc, kk * (16 * 128 >> 4), p.idesc_dq, (it > 0 || kk > 0));
+            }
             tc_commit(rg_empty(s));
         }
         if (ok) tc_commit(acc_final);
@@ -964,17 +969,17 @@ __global__ void __launch_bounds__(DqSpillCfg<D>::kThreadsDq, 1) bwd_dq_spill_ker
         const int row_local = warp * 32 + lane;  // TMEM lane = query row
         if (mbar_wait(acc_final, 0, abort_flag)) {
             tc_fence_after();
-            const long long out_row = ((long long)b * p.q_heads + h) * p.seq_len + (long long)t_own * kTile + row_local;
-            float *op = reinterpret_cast<float *>(p.out0) + out_row * D;
             const bool store = t_own * kTile + row_local < p.seq_len;
             const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
 #pragma unroll
-            for (int c = 0; c < D / 32; ++c) {
+            for (int c = 0; c < HEADS * (D / 32); ++c) {
                 uint32_t r[32];
                 tmem_ld32(t_acc + c * 32, r);
                 tc_wait_ld();
                 if (!store) continue;
-                float4 *dst = reinterpret_cast<float4 *>(op + c * 32);
+                const int x = c / (D / 32);
+                const long long out_row = ((long long)b * p.q_heads + h + x) * p.seq_len + (long long)t_own * kTile + row_local;
+                float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p.out0) + out_row * D + (c % (D / 32)) * 32);
 #pragma unroll
                 for (int q4 = 0; q4 < 8; ++q4)
                     dst[q4] = make_float4(__uint_as_float(r[q4 * 4]) * p.scale, __uint_as_float(r[q4 * 4 + 1]) * p.scale,
@@ -1151,9 +1156,14 @@ int launch_backward_sm100(flat_ctx *ctx, const BwdParams &p) {
     if (st) return st;
     kp.out0 = p.dq;
     kp.out1 = nullptr;
-    if (spill) {
-        if (D == 128) st = run(bwd_dq_spill_kernel<128>, DqSpillCfg<128>::kSmemBytes, grid_q, DqSpillCfg<128>::kThreadsDq);
-        else st = run(bwd_dq_spill_kernel<64>, DqSpillCfg<64>::kSmemBytes, grid_q, DqSpillCfg<64>::kThreadsDq);
+    // two heads to a CTA where that leaves every SM several CTAs
+    const bool pairs = p.group % 2 == 0 && grid_q / 2 >= 4 * (long long)ctx->sm_count;
+    if (spill && pairs) {
+        if (D == 128) st = run(bwd_dq_spill_kernel<128, 2>, DqSpillCfg<128, 2>::kSmemBytes, grid_q / 2, DqSpillCfg<128, 2>::kThreadsDq);
+        else st = run(bwd_dq_spill_kernel<64, 2>, DqSpillCfg<64, 2>::kSmemBytes, grid_q / 2, DqSpillCfg<64, 2>::kThreadsDq);
+    } else if (spill) {
+        if (D == 128) st = run(bwd_dq_spill_kernel<128, 1>, DqSpillCfg<128, 1>::kSmemBytes, grid_q, DqSpillCfg<128, 1>::kThreadsDq);
+        else st = run(bwd_dq_spill_kernel<64, 1>, DqSpillCfg<64, 1>::kSmemBytes, grid_q, DqSpillCfg<64, 1>::kThreadsDq);
     } else if (D == 128) st = run(bwd_dq_sm100_kernel<128>, DqCfg<128>::kSmemBytes, grid_q);
     else st = run(bwd_dq_sm100_kernel<64>, DqCfg<64>::kSmemBytes, grid_q);
     if (st) return st;
