@@ -288,6 +288,10 @@ int forward_common(flat_ctx *ctx, const ForwardCall &call, const flat_attention_
             p.alibi_max_abs_slope = std::max(p.alibi_max_abs_slope, std::fabs(call.alibi_slopes[i]));
         const bool tensor_path = storage16(call.dtype) && forward_sm100_supported(p);
         if ((st = ensure_workspace(ctx, kWorkspaceMeta + (tensor_path ? forward_sm100_workspace_bytes(ctx, p) : 0)))) return st;
+        if (tensor_path && p.q_heads <= kInlineSlopes) {
+            p.alibi_host = call.alibi_slopes;
+            return launch_forward_sm100(ctx, p);
+        }
         FLAT_CUDA_OK(ctx, cudaMemcpyAsync(ctx->workspace, call.alibi_slopes, call.alibi_count * sizeof(float),
                                           cudaMemcpyHostToDevice, ctx->stream));
         p.alibi_slopes = static_cast<const float *>(ctx->workspace);

@@ -145,6 +145,8 @@ __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddep
 // switches plus three position domains, variable-length batches and paged K/V are optional
 // pointers.  (The reference kernels' uniform blocks: src/wgpu_external_asymmetric.rs:319-339,
 // src/wgpu_external_variable.rs:148-171.)
+// Slopes of up to this many heads are arguments of the tensor-core kernel: a copy of their own took 4 us of a call.
+constexpr int kInlineSlopes = 128;
 struct FwdParams {
     const void *q, *k, *v;
     void *o;
@@ -166,7 +168,8 @@ struct FwdParams {
     int64_t page_row_stride;             // elements per physical row (kv_heads*head_dim)
     float inv_freq[kMaxHeadDim / 2];     // theta^(-2j/D), host-computed in f32
     // ALiBi (src/attention_bias.rs:82-95): score += slopes[q_head] * ((kv_off + key) - (q_off + query row))
-    const float *alibi_slopes;           // device, [q_heads] or null
+    const float *alibi_slopes;           // device, [q_heads]; null = no bias
+    const float *alibi_host;             // the same on the host: at most kInlineSlopes of them travel with the tensor-core launch
     int64_t alibi_q_off, alibi_kv_off;
     float alibi_max_abs_slope;           // host-side copy of max |slope|
     int f16_io;                          // 16-bit storage is IEEE binary16 instead of bf16 (forward only)

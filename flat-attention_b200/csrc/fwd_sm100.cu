@@ -173,7 +173,8 @@ struct KernelParams {
     long long rope_table_base;           // varlen: position of the table's first row (the smallest query_rope_offset)
     const float2 *rope_q_table;  // (cos, sin) of row r, pair j at [r * D/2 + j]; null = Q is used as loaded
     float2 rope_step[kMaxHeadDim / 2];  // (cos, sin)(rows_per_step * inv_freq[j]): advances a row's rotation
-    const float *alibi_slopes;  // ALIBI kernels: one slope per query head (device)
+    const float *alibi_slopes;  // ALIBI kernels: one slope per query head (device); null: alibi_inline
+    float alibi_inline[kInlineSlopes];
     int alibi_delta;            // ALIBI kernels: bias position of key 0 minus bias position of query row 0
     float alibi_inv_scale;      // ALIBI kernels: 1 / softmax scale
     long long *trace;
@@ -648,7 +649,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                 // position arithmetic is exact.
                 float slope_rel = 0.f, bias_pos0 = 0.f;
                 if constexpr (ALIBI) {
-                    slope_rel = __ldg(p.alibi_slopes + it.h) * p.alibi_inv_scale;
+                    slope_rel = (p.alibi_slopes ? __ldg(p.alibi_slopes + it.h) : p.alibi_inline[it.h]) * p.alibi_inv_scale;
                     bias_pos0 = (float)(p.alibi_delta + it.j0 * kTileRows - (it.r0 + w * kTileRows + row_in_tile));
                 }
 
@@ -1403,7 +1404,8 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
         }
         return FLAT_OK;
     };
-    kp.alibi_slopes = p.alibi_slopes;
+    if (p.alibi_host) std::copy(p.alibi_host, p.alibi_host + p.q_heads, kp.alibi_inline);
+    else kp.alibi_slopes = p.alibi_slopes;
     kp.alibi_delta = (int)(p.alibi_kv_off - p.alibi_q_off);
     kp.alibi_inv_scale = 1.0f / p.scale;
     // <head_dim, CONVK, ALIBI, F16IO, SPLIT, VARLEN>
