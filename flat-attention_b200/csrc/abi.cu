@@ -274,6 +274,10 @@ int forward_common(flat_ctx *ctx, const ForwardCall &call, const flat_attention_
         p.varlen = reinterpret_cast<const flat_varlen_sequence *>(call.varlen_host);  // non-null for the capability test
         const bool tensor_path = storage16(call.dtype) && forward_sm100_supported(p);
         if ((st = ensure_workspace(ctx, kWorkspaceMeta + (tensor_path ? forward_sm100_workspace_bytes(ctx, p) : 0)))) return st;
+        if (tensor_path && p.batch <= kInlineSequences) {
+            p.varlen_host = call.varlen_host;
+            return launch_forward_sm100(ctx, p);
+        }
         ctx->plan_offsets_at = nullptr;  // the metadata may reach into the part that holds a cached decode plan
         FLAT_CUDA_OK(ctx, cudaMemcpyAsync(ctx->workspace, call.varlen_host, bytes, cudaMemcpyHostToDevice, ctx->stream));
         p.varlen = static_cast<const flat_varlen_sequence *>(ctx->workspace);

@@ -147,6 +147,7 @@ __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddep
 // src/wgpu_external_variable.rs:148-171.)
 // Slopes of up to this many heads are arguments of the tensor-core kernel: a copy of their own took 4 us of a call.
 constexpr int kInlineSlopes = 128;
+constexpr int kInlineSequences = 64;  // the same for the lengths of a padded batch
 struct FwdParams {
     const void *q, *k, *v;
     void *o;
@@ -161,7 +162,8 @@ struct FwdParams {
     float scale;
     int rope_q, rope_k;
     int64_t q_rope_off, k_rope_off;
-    const flat_varlen_sequence *varlen;  // device, [batch] or null
+    const flat_varlen_sequence *varlen;  // device, [batch]; null = uniform lengths
+    const flat_varlen_sequence *varlen_host;  // the same on the host: at most kInlineSequences travel with the tensor-core launch
     int64_t varlen_rope_min, varlen_rope_max;  // smallest / largest query_rope_offset of the batch (host-side copy)
     const int32_t *page_table;           // device, [batch, max_pages] or null
     int page_size, max_pages;

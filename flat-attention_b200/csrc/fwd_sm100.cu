@@ -169,7 +169,8 @@ struct KernelParams {
     float *part_o;    // [rem_items * split][256 rows][D] f32, unnormalised
     float2 *part_ml;  // [rem_items * split][256 rows] (running max in the log2 domain, running sum)
     DeviceStatus *status;
-    const flat_varlen_sequence *varlen;  // per batch element: active lengths, causal and RoPE offsets; null = uniform
+    const flat_varlen_sequence *varlen;  // VARLEN: active lengths, causal and RoPE offsets per batch element; null: varlen_inline
+    flat_varlen_sequence varlen_inline[kInlineSequences];
     long long rope_table_base;           // varlen: position of the table's first row (the smallest query_rope_offset)
     const float2 *rope_q_table;  // (cos, sin) of row r, pair j at [r * D/2 + j]; null = Q is used as loaded
     float2 rope_step[kMaxHeadDim / 2];  // (cos, sin)(rows_per_step * inv_freq[j]): advances a row's rotation
@@ -239,7 +240,7 @@ __device__ __forceinline__ WorkItem make_item_whole(const KernelParams &p, int l
     it.j0 = 0;
     it.part_slot = -1;
     if constexpr (VARLEN) {  // padded batch: src/wgpu_external_variable.rs:21-33
-        const flat_varlen_sequence m = p.varlen[it.b];
+        const flat_varlen_sequence m = p.varlen ? p.varlen[it.b] : p.varlen_inline[it.b];
         it.q_len = (int)m.active_query_len;
         it.kv_len = (int)m.active_kv_len;
         it.causal_off = m.causal_query_offset;
@@ -1359,7 +1360,8 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     kp.q_blocks = (p.q_len + 2 * kTileRows - 1) / (2 * kTileRows);
     kp.status = ctx->dev_status;
     kp.rope_q_table = q_table;
-    kp.varlen = p.varlen;
+    if (p.varlen_host) std::copy(p.varlen_host, p.varlen_host + p.batch, kp.varlen_inline);
+    else kp.varlen = p.varlen;
     kp.rope_table_base = p.varlen ? p.varlen_rope_min : 0;
     if (q_table) {
         const double rows_per_step = 32.0 / (D / 8);
