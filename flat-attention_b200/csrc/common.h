@@ -197,6 +197,8 @@ uint64_t forward_sm100_workspace_bytes(const flat_ctx *ctx, const FwdParams &p);
 int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p);
 
 // ---- decode ----------------------------------------------------------------------------------
+// Tables up to this size are kernel arguments of the tensor-core decode: a copy of its own costs a short context 4 us of 18.
+constexpr int kInlinePages = 256;
 struct DecodeParams {
     const void *q;       // [num_seqs, q_heads*head_dim]
     const void *k, *v;   // paged: [pages, page_size, kv_heads*head_dim]; resident: [batch, capacity, ...]
@@ -206,7 +208,8 @@ struct DecodeParams {
     int page_size, max_pages;            // page_size == 0 -> resident (contiguous) addressing
     int physical_pages;                  // paged: entries outside [0, physical_pages) are masked and flagged, never read
     DeviceStatus *status;                // device status word of the context (page-table range violations)
-    const int32_t *page_table;           // device [num_seqs, max_pages]
+    const int32_t *page_table;           // device [num_seqs, max_pages]; null when host_pages is given
+    const int32_t *host_pages;           // one sequence of up to kInlinePages pages: its table, which travels with the launch
     const int32_t *context_lens;         // device [num_seqs] or null (-> uniform_len)
     const int32_t *q_rope_positions;     // device [num_seqs] or null (-> uniform_q_pos)
     int uniform_len;
