@@ -1,0 +1,142 @@
+"""Sizes at which a launch changes its shape: decode spans and page tables among the kernel arguments, clusters and head pairs
+of the backward, the polynomial exponent of head_dim 64, ALiBi slopes among the kernel arguments."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import binding as ob
+from tests.gpu_util import bf16_round, ctx, dev, fa, run_forward
+from tests.test_gpu_backward_bf16 import randn
+from tests.test_gpu_chunked_backward import run_backward
+from tests.test_gpu_decode_cache import oracle_decode, unpack
+
+pytestmark = pytest.mark.gpu
+
+
+# tokens: one span of one tile, its edges, the largest table that travels with the launch (256 pages) and one page more
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 256 * 16, 256 * 16 + 1])
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 64), (32, 8, 128)])
+def test_paged_decode_spans_and_tables(n, Hq, Hkv, D):
+    c, page = ctx(), 16
+    cache = fa.CudaPagedKvCache(c, fa.BF16, page, (n + page - 1) // page + 1, Hkv, D)
+    g = torch.Generator().manual_seed(n)
+    k, v, q = (torch.randn(r * D, generator=g).bfloat16() for r in (n * Hkv, n * Hkv, Hq))
+    cache.record_append(k.cuda(), v.cuda(), n)
+    out = c.create_decode_output_buffer(fa.BF16, 1, Hq, D)
+    out.fill_(0x7f)
+    c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, n - 1, q.cuda(), cache.k_buffer(), cache.v_buffer(), out)
+    o, l = unpack(out, fa.BF16, Hq, D)
+    eo, el = oracle_decode(q.float().numpy(), k.float().numpy().reshape(n, -1), v.float().numpy().reshape(n, -1), Hq, Hkv, D, 5e5,
+                           n - 1, 0, True)
+    assert np.abs(o.reshape(-1) - eo.reshape(-1)).max() <= 2e-2
+    assert np.abs(l.reshape(-1) - el.reshape(-1)).max() <= 2e-3
+    assert c.device_status() == 0
+
+
+# (B, Hq, Hkv, N, D): clusters of 1, 2, 3 and 8 CTAs per key tile on 148 SMs, key tiles with fewer pairs than CTAs among them
+@pytest.mark.parametrize("B,Hq,Hkv,N,D", [(1, 4, 4, 100, 64), (1, 8, 1, 130, 128), (1, 12, 1, 128, 64), (1, 32, 2, 600, 64),
+                                          (1, 16, 1, 700, 128)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_backward_clusters(B, Hq, Hkv, N, D, causal):
+    q, k, v, do = randn(B * Hq * N * D, 1), randn(B * Hkv * N * D, 2), randn(B * Hkv * N * D, 3), randn(B * Hq * N * D, 4)
+    fo, fl = run_forward("grouped", fa.F32, fa.shape(B, Hq, Hkv, N, N, D), fa.config(causal), q, k, v)
+    fo = bf16_round(fo)
+    got = run_backward(fa.BF16, B, Hq, Hkv, N, D, causal, None, q, k, v, do, fo, fl)
+    exp = run_backward(fa.F32, B, Hq, Hkv, N, D, causal, None, q, k, v, do, fo, fl)
+    for name, a, e in zip(("dQ", "dK", "dV"), got, exp):
+        # P and dS are rounded to bf16 (2^-9) before a sum of N * group terms of mixed sign: 2e-2 holds for the small sums of
+        # the other backward tests, here it grows with the largest gradient
+        assert np.abs(a - e).max() <= 2e-2 + 4e-3 * np.abs(e).max(), (name, float(np.abs(a - e).max()), float(np.abs(e).max()))
+    again = run_backward(fa.BF16, B, Hq, Hkv, N, D, causal, None, q, k, v, do, fo, fl)
+    assert all(np.array_equal(x, y) for x, y in zip(got, again))
+    assert ctx().device_status() == 0
+
+
+@pytest.mark.parametrize("D,causal", [(64, True), (128, False)])
+def test_backward_head_pairs(D, causal):
+    """dQ with two heads to a CTA (4 * 148 pairs of query tiles) equals dQ of the same heads in a batch too small for that."""
+    B, Hq, Hkv, N = 13, 32, 16, 260
+    q, k, v, do = (torch.randn(B, h, N, D, generator=torch.Generator().manual_seed(h + i)).bfloat16().float().numpy()
+                   for i, h in enumerate((Hq, Hkv, Hkv, Hq)))
+    fo, fl = run_forward("grouped", fa.F32, fa.shape(B, Hq, Hkv, N, N, D), fa.config(causal), q.reshape(-1), k.reshape(-1), v.reshape(-1))
+    fo = bf16_round(fo).reshape(B, Hq, N, D)
+    flat = [x.reshape(-1) for x in (q, k, v, do, fo, fl)]
+    dq, _, _ = run_backward(fa.BF16, B, Hq, Hkv, N, D, causal, None, *flat)
+    dq = dq.reshape(B, Hq, N, D)
+    fl = fl.reshape(B, Hq, N)
+    for b in (0, B - 1):
+        one, _, _ = run_backward(fa.BF16, 1, Hq, Hkv, N, D, causal, None, *(x[b].reshape(-1) for x in (q, k, v, do, fo, fl)))
+        assert np.array_equal(dq[b].reshape(-1), one)
+
+
+def test_exponent_of_head_dim_64_keeps_nan_and_zero():
+    """A NaN query row stays NaN in O and LSE and alone; scores far below the row's maximum give exactly nothing."""
+    B, H, N, D = 1, 2, 300, 64
+    q, k, v = randn(B * H * N * D, 5), randn(B * H * N * D, 6), randn(B * H * N * D, 7)
+    q.reshape(H, N, D)[1, 131] = np.nan
+    k.reshape(H, N, D)[0, 7] = 60.0 * np.sign(q.reshape(H, N, D)[0, 9])  # one key far above all others for row 9
+    q.reshape(H, N, D)[0, 9] = 60.0 * np.sign(q.reshape(H, N, D)[0, 9])
+    o, l = run_forward("grouped", fa.BF16, fa.shape(B, H, H, N, N, D), fa.config(False), q, k, v)
+    o, l = o.reshape(H, N, D), l.reshape(H, N)
+    bad = np.zeros((H, N), bool)
+    bad[1, 131] = True
+    assert np.array_equal(np.isnan(l), bad) and np.array_equal(np.isnan(o).all(-1), bad) and np.array_equal(np.isnan(o).any(-1), bad)
+    assert np.array_equal(o[0, 9], v.reshape(H, N, D)[0, 7])
+
+
+@pytest.mark.parametrize("H", [128, 130])
+def test_alibi_slopes_of_many_heads(H):
+    """Up to 128 slopes are kernel arguments, more are copied to the device."""
+    N, D = 40, 64
+    q, k, v = randn(N * H * D, 8), randn(N * H * D, 9), randn(N * H * D, 10)
+    slopes = [float(2.0 ** (-8.0 * (h + 1) / H)) for h in range(H)]
+    shp, c = fa.shape(1, H, H, N, N, D), ctx()
+    out = c.create_output_buffer(fa.BF16, shp)
+    c.forward_projection_rope_asymmetric_alibi(fa.BF16, shp, fa.config(True), fa.rotary(5e5, 0, 0), slopes, 0, 0,
+                                               dev(q, torch.bfloat16), dev(k, torch.bfloat16), dev(v, torch.bfloat16), out)
+    o, l = c.split_output(out, fa.BF16, shp, fa.PROJECTION)
+    eo, el = ob.forward_reference_projection_grouped_rope_asymmetric_biased(q, k, v, ob._shape(1, H, H, N, N, D, 0), 5e5, 0, 0, causal=True,
+                                                                            alibi=(slopes, 0, 0))
+    assert np.abs(o.float().cpu().numpy().reshape(-1) - eo.reshape(-1)).max() <= 2e-2
+    assert np.abs(l.cpu().numpy().reshape(-1) - el.reshape(-1)).max() <= 2e-3
+
+
+def test_captured_calls_replay_to_the_same_bits():
+    """Forward (rotation and attention), backward (three kernels) and decode (two) inside one CUDA graph: the launches that
+    overlap in a stream keep their order in a graph."""
+    B, Hq, Hkv, N, D = 2, 8, 2, 300, 128
+    stream = torch.cuda.Stream()
+    c = fa.Context(0, stream=stream)
+    shp, cfg = fa.shape(B, Hq, Hkv, N, N, D), fa.config(True)
+    q, k, v, do = (dev(randn(B * h * N * D, i), torch.bfloat16) for i, h in enumerate((Hq, Hkv, Hkv, Hq)))
+    out = c.create_output_buffer(fa.BF16, shp)
+    L = fa.backward_layout(fa.BF16, shp)
+    packed, grads = c.empty_bytes(L.input_bytes), c.empty_bytes(L.output_bytes)
+    for at, x in ((L.q_offset, q), (L.k_offset, k), (L.v_offset, v), (L.d_out_offset, do)):
+        packed[at:at + 2 * x.numel()].view(torch.bfloat16).copy_(x.reshape(-1))
+    cache = fa.CudaPagedKvCache(c, fa.BF16, 16, 50, Hkv, D)
+    torch.cuda.synchronize()
+    cache.record_append(k[:600 * Hkv * D], v[:600 * Hkv * D], 600)
+    dec = c.create_decode_output_buffer(fa.BF16, 1, Hq, D)
+
+    def calls():
+        c.forward_grouped_rope(fa.BF16, shp, cfg, fa.rotary(5e5, 0, 0), q, k, v, out)
+        c.forward_grouped(fa.BF16, shp, cfg, q, k, v, packed[L.out_offset:])
+        c.backward_grouped(fa.BF16, shp, cfg, packed, grads)
+        c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, cfg, 5e5, 599, q[:Hq * D], cache.k_buffer(), cache.v_buffer(), dec)
+
+    with torch.cuda.stream(stream):
+        calls()  # tables and scratch
+    torch.cuda.synchronize()
+    want = [x.clone() for x in (out, grads, dec)]
+    for x in (out, grads, dec):
+        x.zero_()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        calls()
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip((out, grads, dec), want))
+    assert c.device_status() == 0
