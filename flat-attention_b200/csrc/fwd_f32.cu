@@ -384,7 +384,9 @@ int cluster_parts(const flat_ctx *ctx, const FwdParams &p) {
 bool forward_f32_supported(const FwdParams &p) {
     if (p.head_dim != 64 && p.head_dim != 128) return false;
     if (p.varlen || p.page_table) return false;
-    if (p.q_len < 16) return false;  // a block has 64 rows: a few rows waste it
+    // a block has 64 rows, most of them idle in a short call; from 16 rows on it is still the faster one (8 / 2 heads: 16 rows
+    // against 16 keys, D = 64 12.3 -> 10.3 us, against 2000 keys 514 -> 33 us)
+    if (p.q_len < 16) return false;
     const void *ptrs[] = {p.q, p.k, p.v, p.o};
     for (const void *x : ptrs)
         if (reinterpret_cast<uintptr_t>(x) & 15) return false;

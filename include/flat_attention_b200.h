@@ -762,7 +762,7 @@ uint64_t flat_device_capabilities_stable(const flat_device_capabilities *caps);
 /* RuntimeKernelId (src/runtime_telemetry.rs:10-20) for this library's kernel families. */
 typedef enum flat_kernel_id {
     FLAT_KERNEL_FORWARD_TCGEN05 = 0,  /* fwd_sm100_kernel: bf16, head_dim 64/128 */
-    FLAT_KERNEL_FORWARD_GENERIC = 1   /* fwd_simt_kernel: f32 arithmetic, any shape */
+    FLAT_KERNEL_FORWARD_GENERIC = 1   /* fwd_f32_kernel / fwd_simt_kernel: f32 arithmetic, any shape */
 } flat_kernel_id;
 
 /* AutotunerCacheStatus (src/runtime_telemetry.rs:138-145). */
