@@ -255,11 +255,9 @@ constexpr int kMergeGroupsWide = 4;  // thread groups of the wide variant; group
 constexpr int kMergeWideFrom = 17;   // rows with this many parts or more are merged by the wide variant
 constexpr int kMergeBatch = 512;   // weights staged per pass
 
-// Merge of the split-KV partials of one row: LSE = log sum exp(LSE_i), O = sum exp(LSE_i - LSE) O_i.  GROUPS = 1: 128
-// threads, the parts are added in order (a batch of many short sequences: few parts per row, thousands of rows).
-// GROUPS = 4: a long context cut into short spans gives a row hundreds of parts and a batch only a few rows, so the
-// parts are spread over four thread groups (the loop is a chain of L2 round trips otherwise) and the groups' sums are
-// added in group order.  Either way eight independent loads are in flight per thread and the result is a fixed
+// Merge of the split-KV partials that ranks exchange, any head dimension and part stride: LSE = log sum exp(LSE_i),
+// O = sum exp(LSE_i - LSE) O_i.  GROUPS = 1: 128 threads, the parts are added in order.  GROUPS = 4: many parts are spread
+// over four thread groups (the loop is a chain of L2 round trips otherwise) and the groups' sums are added in group order.  Either way eight independent loads are in flight per thread and the result is a fixed
 // function of the inputs and of the part count.
 template <typename T, int GROUPS>
 __global__ void __launch_bounds__(kMergeDims * GROUPS) merge_kernel(int parts, int64_t rows, int head_dim,
@@ -327,11 +325,11 @@ __global__ void __launch_bounds__(kMergeDims * GROUPS) merge_kernel(int parts, i
 
 // Merge of one decode row (sequence, q_head), D a multiple of 4.  Fixed-chunk mode: only ceil(ctx/chunk) parts of a row are
 // live.  Balanced mode: one slot per CTA that touched the sequence; a single slot was already written as the final result.
-//  A chain of dependent L2 round trips is all there is to it,
-// so it has as few of them as possible: every warp reads all LSEs itself (no block reduction, no staged weights), a lane
-// then owns four columns, so that 32 / lanes parts go through a warp at a time, eight steps in flight, and the
-// warps' sums are added in warp order.  128 rows of 150 parts (2 sequences of 60001 tokens) take 6.4 us where a
-// block reduction, staged weights and one column per thread took 8.5; a decode step of 700 tokens went from 12.3 to 10.3 us.
+// A chain of dependent L2 round trips is all there is to it, so it has as few of them as possible: every warp reads all
+// LSEs itself (no block reduction, no staged weights), a lane owns four columns, so that 32 / lanes parts go through a warp
+// at a time, eight steps of them requested before the LSEs are reduced, and the warps' sums are added in warp order.  128
+// rows of 150 parts (2 sequences of 60001 tokens) take 6.4 us where a block reduction, staged weights and one column per
+// thread took 8.5; a decode step of 700 tokens went from 12.3 to 10.3 us.
 template <typename T, int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) merge_row_kernel(int parts, int head_dim, const float *__restrict__ partial_o,
                                                                const float *__restrict__ partial_lse, T *__restrict__ o,

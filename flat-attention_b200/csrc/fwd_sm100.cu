@@ -54,7 +54,8 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 domain
 // (16 exponentials per clock and SM) becomes the bound: every kPolyEvery-th pair of scores takes 2^t from the FMA and
 // integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, D = 64: 135 us without, 133 / 129 / 138 us with every 8th /
 // 4th / 8 of 3 pairs.  At D = 128 the same costs time (the tensor pipe and the power limit bound there: a 32768-token
-// chunked prefill 18.5 -> 19.5 ms), so the flag follows D.
+// chunked prefill 18.5 -> 19.5 ms), so the flag follows D; nor where K is converted in shared memory (CONVK): the converting
+// warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads, D = 64 979 -> 995 us).
 constexpr int kPolyEvery = 4;
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -762,7 +763,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                             float t0, t1;
                             asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t2));
                             float p0 = t0, p1 = t1;
-                            if (D == 64 && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
+                            if (D == 64 && !CONVK && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
                                 ex2_poly(p0, p1);
                             } else {
                                 p0 = ex2(t0);
