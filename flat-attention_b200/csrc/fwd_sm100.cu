@@ -55,7 +55,8 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 domain
 // integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, D = 64: 135 us without, 133 / 129 / 138 us with every 8th /
 // 4th / 8 of 3 pairs.  At D = 128 the same costs time (the tensor pipe and the power limit bound there: a 32768-token
 // chunked prefill 18.5 -> 19.5 ms), so the flag follows D; nor where K is converted in shared memory (CONVK): the converting
-// warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads, D = 64 979 -> 995 us).
+// warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads, D = 64 979 -> 995 us), nor for K and V behind a page
+// table (the same call with the binary16 shadow 964 -> 984 us).
 constexpr int kPolyEvery = 4;
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -304,10 +305,11 @@ __device__ __forceinline__ int item_index(const KernelParams &p, int k) {
 // (src/attention_bias.rs:82-95) before the running maximum is taken.
 // F16IO: Q, K, V and O are IEEE binary16 instead of bf16 (P is then written as binary16 too, since one MMA takes A and B
 // of one format); accumulation, softmax and LSE stay f32.
+// POLY: a part of the exponentials leaves the special-function unit (kPolyEvery).
 // VARLEN: a padded variable-length batch (never split).  The rows past a sequence's live ones get O = 0, LSE = -inf
 // (src/asymmetric_grouped.rs:103-104) from the epilogue: filling O and LSE before the launch took 28 us of the 251 us of
 // a padded batch of 16 x 1024 rows, 32 heads, D = 128.
-template <int D, bool CONVK, bool ALIBI, bool F16IO, bool SPLIT, bool VARLEN>
+template <int D, bool CONVK, bool ALIBI, bool F16IO, bool SPLIT, bool VARLEN, bool POLY = D == 64 && !CONVK>
 __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_constant__ KernelParams p) {
     using C = Cfg<D, CONVK>;
     extern __shared__ uint8_t smem_raw[];
@@ -763,7 +765,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                             float t0, t1;
                             asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t2));
                             float p0 = t0, p1 = t1;
-                            if (D == 64 && !CONVK && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
+                            if (POLY && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
                                 ex2_poly(p0, p1);
                             } else {
                                 p0 = ex2(t0);
@@ -1411,13 +1413,17 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     else kp.alibi_slopes = p.alibi_slopes;
     kp.alibi_delta = (int)(p.alibi_kv_off - p.alibi_q_off);
     kp.alibi_inv_scale = 1.0f / p.scale;
-    // <head_dim, CONVK, ALIBI, F16IO, SPLIT, VARLEN>
+    // <head_dim, CONVK, ALIBI, F16IO, SPLIT, VARLEN, POLY>
     auto pick = [&](auto d_tag, auto convk_tag, auto alibi_tag, auto f16_tag) -> int {
         constexpr int kD = decltype(d_tag)::value;
         constexpr bool kConv = decltype(convk_tag)::value, kAlibi = decltype(alibi_tag)::value, kF16 = decltype(f16_tag)::value;
         constexpr int kSmem = Cfg<kD, kConv>::kSmemBytes;
         if constexpr (!kAlibi)
             if (p.varlen) return run(fwd_sm100_kernel<kD, kConv, false, kF16, false, true>, kSmem);
+        if constexpr (kD == 64 && !kConv && !kAlibi && !kF16)
+            if (p.page_table)
+                return plan.split > 1 ? run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, true, false, false>, kSmem)
+                                      : run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, false, false, false>, kSmem);
         if (plan.split > 1) return run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, true, false>, kSmem);
         return run(fwd_sm100_kernel<kD, kConv, kAlibi, kF16, false, false>, kSmem);
     };
