@@ -56,7 +56,8 @@ constexpr float kRescaleThreshold = 8.0f;  // log2 domain
 // 4th / 8 of 3 pairs.  At D = 128 the same costs time (the tensor pipe and the power limit bound there: a 32768-token
 // chunked prefill 18.5 -> 19.5 ms), so the flag follows D; nor where K is converted in shared memory (CONVK): the converting
 // warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads, D = 64 979 -> 995 us), nor for K and V behind a page
-// table (the same call with the binary16 shadow 964 -> 984 us).
+// table (the same call with the binary16 shadow 964 -> 984 us) and for padded batches, whose items are short (16 x 1024 rows,
+// 32 / 8 heads 162 -> 165 us).
 constexpr int kPolyEvery = 4;
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -309,7 +310,7 @@ __device__ __forceinline__ int item_index(const KernelParams &p, int k) {
 // VARLEN: a padded variable-length batch (never split).  The rows past a sequence's live ones get O = 0, LSE = -inf
 // (src/asymmetric_grouped.rs:103-104) from the epilogue: filling O and LSE before the launch took 28 us of the 251 us of
 // a padded batch of 16 x 1024 rows, 32 heads, D = 128.
-template <int D, bool CONVK, bool ALIBI, bool F16IO, bool SPLIT, bool VARLEN, bool POLY = D == 64 && !CONVK>
+template <int D, bool CONVK, bool ALIBI, bool F16IO, bool SPLIT, bool VARLEN, bool POLY = D == 64 && !CONVK && !VARLEN>
 __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_constant__ KernelParams p) {
     using C = Cfg<D, CONVK>;
     extern __shared__ uint8_t smem_raw[];
