@@ -56,3 +56,31 @@ def test_a_call_under_capture_gives_the_same_bits():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+# (Hq, Hkv, Nq, Nkv, D, query offset), causal: one CTA per block, clusters, a diagonal that starts inside a tile
+@pytest.mark.parametrize("Hq,Hkv,Nq,Nkv,D,coff", [(2, 1, 60, 60, 128, 0), (8, 2, 200, 200, 64, 0), (4, 4, 130, 330, 128, 200),
+                                                  (2, 2, 100, 131, 64, 31)])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_non_finite_values_of_unseen_keys_stay_out(Hq, Hkv, Nq, Nkv, D, coff, bad):
+    """A row is a function of the keys it sees: a non-finite V (and K) row changes no bit of the rows before it."""
+    q, k, v = case(1, Hq, Hkv, Nq, Nkv, D)
+    shp, cfg, rot = fa.shape(1, Hq, Hkv, Nq, Nkv, D, coff), fa.config(True), fa.rotary(5e5, coff, 0)
+    o, l = (x.reshape(s) for x, s in zip(run_forward("projection_rope_asymmetric", fa.F32, shp, cfg, q, k, v, rot=rot),
+                                         ((Nq, Hq, D), (Hq, Nq))))
+    for key in (40, 63, 64, Nkv - 1):
+        if key >= Nkv:
+            continue
+        first = max(0, key - coff)  # the first row that sees the key
+        v2 = v.reshape(Nkv, Hkv, D).copy()
+        v2[key] = bad
+        o2, l2 = run_forward("projection_rope_asymmetric", fa.F32, shp, cfg, q, k, v2, rot=rot)
+        o2, l2 = o2.reshape(Nq, Hq, D), l2.reshape(Hq, Nq)
+        assert np.array_equal(o2[:first], o[:first]), (key, int(np.isnan(o2).any((1, 2)).argmax()))
+        assert np.array_equal(l2, l)
+        assert not np.isfinite(o2[first:]).any()
+        k2 = k.reshape(Nkv, Hkv, D).copy()
+        k2[key] = bad
+        o2, l2 = run_forward("projection_rope_asymmetric", fa.F32, shp, cfg, q, k2, v, rot=rot)
+        assert np.array_equal(o2.reshape(Nq, Hq, D)[:first], o[:first])
+        assert np.array_equal(l2.reshape(Hq, Nq)[:, :first], l[:, :first])
