@@ -599,6 +599,12 @@ int32_t flat_ctx_create(int32_t device, void *stream, flat_ctx **out) {
         delete ctx;
         return FLAT_ERR_EXECUTION;
     }
+    if (cudaMalloc(&ctx->f32_table.dev, kF32TableBytes) == cudaSuccess) {
+        ctx->f32_table.bytes = kF32TableBytes;
+    } else {
+        ctx->f32_table.dev = nullptr;
+        cudaGetLastError();
+    }
     *out = ctx;
     return FLAT_OK;
 }
@@ -615,6 +621,7 @@ void flat_ctx_destroy(flat_ctx *ctx) {
     if (ctx->host_stage) cudaFree(ctx->host_stage);
     for (auto &t : ctx->rope_tables)
         if (t.dev) cudaFree(t.dev);
+    if (ctx->f32_table.dev) cudaFree(ctx->f32_table.dev);
     for (cudaEvent_t e : ctx->pipe_events) cudaEventDestroy(e);
     if (ctx->stream_switch) cudaEventDestroy(ctx->stream_switch);
     if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);

@@ -18,6 +18,7 @@
 namespace flat {
 
 constexpr int kMaxHeadDim = 128;  // WGSL_MAX_HEAD_DIM, src/lib.rs:60
+constexpr uint64_t kF32TableBytes = 16ull << 20;  // 32768 positions at head_dim 128
 
 // Device status word written by bounded waits.
 struct DeviceStatus {
@@ -54,9 +55,13 @@ struct flat_ctx {
         int half_dim = 0, rows = 0;
         int64_t pos_off = 0;
         uint64_t last_use = 0;
+        bool replays_write = false;  // a captured launch fills this memory: what it holds depends on replays
     };
     RopeTable rope_tables[2];
     uint64_t rope_clock = 0;
+    // The f32 forward has a table of its own, of kF32TableBytes, allocated with the context (null where the device had no
+    // room): it never allocates, and only reads the tables above, whose addresses captured launches hold.
+    RopeTable f32_table;
     // The tensor-core backward may keep every bf16 dS^T tile in scratch (O(N^2) bytes) so that dQ needs no second score
     // recompute; it does so while that spill fits this budget (flat_ctx_set_backward_scratch_budget).
     uint64_t backward_scratch_budget = 8ull << 30;
@@ -184,8 +189,8 @@ int launch_forward_simt(flat_ctx *ctx, int dtype, const FwdParams &p);
 bool forward_f32_supported(const FwdParams &p);
 void forward_f32_geometry(const flat_ctx *ctx, const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3]);
 int launch_forward_f32(flat_ctx *ctx, const FwdParams &p);
-// (cos, sin) of `rows` positions from pos_off on, [rows][half_dim], from the context's tables or computed now on its stream.
-int rope_table(flat_ctx *ctx, const float *inv_freq, int half_dim, int rows, int64_t pos_off, const float2 **out);
+// Writes (cos, sin) of `rows` positions from pos_off on to dev, [rows][half_dim] float2, on the context's stream.
+int fill_rope_table(flat_ctx *ctx, void *dev, const float *inv_freq, int half_dim, int rows, int64_t pos_off);
 // tile geometry and grid of the forward kernels for a parameter block (telemetry; nothing is launched)
 void forward_simt_geometry(const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3]);
 void forward_sm100_geometry(const flat_ctx *ctx, const FwdParams &p, uint32_t *query_rows, uint32_t *kv_rows, uint32_t grid[3],

@@ -10,10 +10,11 @@
 // dealt to a cluster of up to 8 CTAs, which combine their (max, sum, O) through distributed shared memory in rank
 // order: one launch, no scratch, bitwise repeatable.  8 / 2 heads, 512 rows, D = 128, causal, RoPE: 219 us with the kernel of
 // fwd_simt.cu, 45 us here; 2 x 2048 rows, 16 / 4 heads 3470 us and 1180 us (29 TFLOP/s).
-// RoPE: K and Q are rotated on the way into shared memory with the (cos, sin) table of the call's positions; without a
-// table (a call under stream capture, where none can be allocated) the same sincosf runs here.
+// RoPE: K and Q are rotated on the way into shared memory with the (cos, sin) table of the call's positions (find_tables());
+// without one the same sincosf runs here.
 #include <cooperative_groups.h>
 
+#include <cstring>
 #include <type_traits>
 
 #include "common.h"
@@ -423,6 +424,51 @@ int cluster_parts(const flat_ctx *ctx, const FwdParams &p) {
     return parts;
 }
 
+bool holds(const flat_ctx::RopeTable &t, const FwdParams &p, int64_t first, int64_t rows) {
+    return t.dev && !t.replays_write && t.half_dim == p.head_dim / 2 && t.pos_off <= first && first + rows <= t.pos_off + t.rows &&
+           std::memcmp(t.inv_freq, p.inv_freq, p.head_dim / 2 * sizeof(float)) == 0;
+}
+
+// The (cos, sin) tables of a call.  Those of the tensor-core kernels are read where they hold the positions, and never
+// written; else the context's table of this mode is made to hold one range with the positions of Q and of K, unless it does.
+// Without a table the kernel evaluates the same angles itself, for every tile again (512 rows 61 us instead of 45): under
+// stream capture, where a replay would read what later calls have put there, beyond kF32TableBytes, and where the context
+// got no memory.
+void find_tables(flat_ctx *ctx, F32Params *fp) {
+    const FwdParams &p = fp->f;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusActive;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    if (capture != cudaStreamCaptureStatusNone) return;
+    const int half_dim = p.head_dim / 2;
+    auto at = [&](const flat_ctx::RopeTable &t, int64_t pos) {
+        return static_cast<const float2 *>(t.dev) + (pos - t.pos_off) * half_dim;
+    };
+    for (const auto &t : ctx->rope_tables) {
+        if (p.rope_q && holds(t, p, p.q_rope_off, p.q_len)) fp->q_table = at(t, p.q_rope_off);
+        if (p.rope_k && holds(t, p, p.k_rope_off, p.kv_len)) fp->k_table = at(t, p.k_rope_off);
+    }
+    const bool want_q = p.rope_q && !fp->q_table, want_k = p.rope_k && !fp->k_table;
+    if (!want_q && !want_k) return;
+    int64_t lo = INT64_MAX, hi = 0;
+    if (want_q) lo = p.q_rope_off, hi = lo + p.q_len;
+    if (want_k) lo = std::min(lo, p.k_rope_off), hi = std::max(hi, p.k_rope_off + p.kv_len);
+    flat_ctx::RopeTable &t = ctx->f32_table;
+    if (!holds(t, p, lo, hi - lo)) {
+        if (!t.dev || (uint64_t)(hi - lo) * half_dim * sizeof(float2) > t.bytes) return;
+        t.rows = 0;
+        if (fill_rope_table(ctx, t.dev, p.inv_freq, half_dim, (int)(hi - lo), lo)) return;
+        std::memcpy(t.inv_freq, p.inv_freq, half_dim * sizeof(float));
+        t.half_dim = half_dim;
+        t.pos_off = lo;
+        t.rows = (int)(hi - lo);
+    }
+    if (want_q) fp->q_table = at(t, p.q_rope_off);
+    if (want_k) fp->k_table = at(t, p.k_rope_off);
+}
+
 }  // namespace
 
 bool forward_f32_supported(const FwdParams &p) {
@@ -453,15 +499,7 @@ int launch_forward_f32(flat_ctx *ctx, const FwdParams &p) {
         return fail(ctx, FLAT_ERR_DISPATCH_LIMIT, "grid dimension %d exceeds 65535", p.q_heads > 65535 ? p.q_heads : p.batch);
     F32Params fp{};
     fp.f = p;
-    // where no table is to be had (a capturing stream allows no allocation, the device may be full) or it would be
-    // larger than 64 MiB, the kernel evaluates the angles itself, with the same result
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    FLAT_CUDA_OK(ctx, cudaStreamIsCapturing(ctx->stream, &capture));
-    const int64_t row_bytes = p.head_dim / 2 * (int64_t)sizeof(float2);
-    if (capture == cudaStreamCaptureStatusNone && std::max(p.q_len, p.kv_len) * row_bytes <= (64ll << 20)) {
-        if (p.rope_q && rope_table(ctx, p.inv_freq, p.head_dim / 2, p.q_len, p.q_rope_off, &fp.q_table)) cudaGetLastError();
-        if (p.rope_k && rope_table(ctx, p.inv_freq, p.head_dim / 2, p.kv_len, p.k_rope_off, &fp.k_table)) cudaGetLastError();
-    }
+    if (p.rope_q || p.rope_k) find_tables(ctx, &fp);
     const int parts = cluster_parts(ctx, p);
     return p.head_dim == 128 ? launch<128>(ctx, fp, parts) : launch<64>(ctx, fp, parts);
 }

@@ -1153,6 +1153,19 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 
 
 }  // namespace
 
+int fill_rope_table(flat_ctx *ctx, void *dev, const float *inv_freq, int half_dim, int rows, int64_t pos_off) {
+    const int64_t n = (int64_t)rows * half_dim;
+    InvFreq f{};
+    std::memcpy(f.f, inv_freq, sizeof(float) * half_dim);
+    rope_table_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, ctx->stream>>>(static_cast<float2 *>(dev), rows,
+                                                                                             half_dim, pos_off, f);
+    ctx->launches += 1;
+    FLAT_CUDA_OK(ctx, cudaGetLastError());
+    return FLAT_OK;
+}
+
+namespace {
+
 // (cos, sin) table of `rows` positions starting at pos_off, from the context's cache or computed now on its stream.
 int rope_table(flat_ctx *ctx, const float *inv_freq, int half_dim, int rows, int64_t pos_off, const float2 **out) {
     flat_ctx::RopeTable *slot = nullptr;
@@ -1173,13 +1186,13 @@ int rope_table(flat_ctx *ctx, const float *inv_freq, int half_dim, int rows, int
         slot->bytes = 0;
         FLAT_CUDA_OK(ctx, cudaMalloc(&slot->dev, bytes));
         slot->bytes = bytes;
+        slot->replays_write = false;
     }
-    const int64_t n = (int64_t)rows * half_dim;
-    InvFreq f{};
-    std::memcpy(f.f, inv_freq, sizeof(float) * half_dim);
-    rope_table_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, ctx->stream>>>(
-        static_cast<float2 *>(slot->dev), rows, half_dim, pos_off, f);
-    ctx->launches += 1;
+    slot->rows = 0;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) slot->replays_write = true;
+    if (int st = fill_rope_table(ctx, slot->dev, inv_freq, half_dim, rows, pos_off)) return st;
     std::memcpy(slot->inv_freq, inv_freq, sizeof(float) * half_dim);
     slot->half_dim = half_dim;
     slot->rows = rows;
@@ -1188,6 +1201,8 @@ int rope_table(flat_ctx *ctx, const float *inv_freq, int half_dim, int rows, int
     *out = static_cast<const float2 *>(slot->dev);
     return FLAT_OK;
 }
+
+}  // namespace
 
 bool forward_sm100_supported(const FwdParams &p) {
     if (p.head_dim != 64 && p.head_dim != 128) return false;
