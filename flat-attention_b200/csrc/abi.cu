@@ -429,6 +429,7 @@ uint64_t plan_decode(flat_ctx *ctx, int dtype, DecodeParams &p, const int32_t *h
     p.kv_splits = 1;
     p.chunk_tokens = 0;
     p.balanced = 0;
+    p.short_partials = 0;
     if (!decode_fast_path_ok(dtype, p.head_dim, p.group)) return 0;
     if (kv_splits == 0 && offsets && decode_mma_supported(dtype, p) &&
         (uint64_t)(p.num_seqs + 1) * sizeof(int32_t) <= kWorkspaceMeta - kSeqOffsetsAt) {
@@ -449,17 +450,25 @@ uint64_t plan_decode(flat_ctx *ctx, int dtype, DecodeParams &p, const int32_t *h
             if (ctas < 1) ctas = 1;
             int64_t span = (at + ctas - 1) / ctas;
             span = (span + 15) / 16 * 16;
-            // A span is a chain of tiles for a warp and a part more for the merge.  Shortest spans of 16 / 32 / 64 tokens,
-            // 32 / 8 heads, D = 128: 1000 tokens 10.3 / 12.3 / 14.4 us, 2500 14.4 / 12.3 / 14.4, 3500 16.4 / 14.4 / 16.6,
-            // 6500 20.6 / 20.6 / 20.5, 8000 22.6 / 22.6 / 20.9.
-            const int64_t shortest = max16 <= 2048 ? 16 : max16 <= 6144 ? 32 : 64;
-            if (span < shortest) span = shortest;
-            ctas = (at + span - 1) / span;
             p.balanced = 1;
-            p.span_tokens = (int)span;
-            p.num_ctas = (int)ctas;
-            p.kv_splits = (int)((max16 + span - 1) / span + 1);  // slots per sequence
-            return decode_workspace_bytes(p);
+            // A span is a chain of tiles for a warp and a part more for the merge.  Shortest spans of 16 / 32 / 64 tokens, D =
+            // 128, 32 / 8 heads: 1000 tokens 10.3 / 12.3 / 14.4 us, 2500 14.4 / 12.3 / 14.4, 3500 16.4 / 14.4 / 16.6, 6500 20.6
+            // / 20.6 / 20.5, 8000 22.6 / 22.6 / 20.9; 64 / 8 heads, 1000 11.4 / 12.3 / 14.4, 3000 16.4 / 14.4 / 17.5; 16 / 16
+            // heads, 400 10.3 / 12.3 / 12.6; D = 64, 8 / 2 heads, 1000 8.9 / 8.8 / 10.3, 3000 10.3 / 8.9 / 10.3; four
+            // sequences of 700 tokens 12.4 / 12.4 / 16.5, of 1500 16.4 / 16.4 / 18.6.
+            // Shorter spans are more parts, dense over all sequences: they are taken while the parts fit the context's memory
+            // for them, so that no call asks for more workspace than spans of 64 do.
+            for (int64_t shortest = max16 <= 2048 ? 16 : max16 <= 6144 ? 32 : 64;; shortest *= 2) {
+                const int64_t s = std::max(span, shortest);
+                p.num_ctas = (int)((at + s - 1) / s);
+                p.span_tokens = (int)s;
+                p.kv_splits = (int)((max16 + s - 1) / s + 1);  // slots per sequence
+                if (s >= 64) return decode_workspace_bytes(p);
+                if (ctx->short_partials && decode_workspace_bytes(p) <= kShortPartialBytes) {
+                    p.short_partials = 1;
+                    return 0;
+                }
+            }
         }
     }
     int splits = 1, chunk = 0;
@@ -539,8 +548,9 @@ int run_decode(flat_ctx *ctx, int dtype, DecodeParams &p) {
     if (p.kv_splits > 1) {
         const uint64_t rows = (uint64_t)p.num_seqs * p.q_heads;
         const uint64_t o_bytes = (uint64_t)p.kv_splits * rows * p.head_dim * sizeof(float);
-        p.partial_o = reinterpret_cast<float *>(scratch_ptr(ctx));
-        p.partial_lse = reinterpret_cast<float *>(scratch_ptr(ctx) + o_bytes);
+        char *partials = p.short_partials ? static_cast<char *>(ctx->short_partials) : scratch_ptr(ctx);
+        p.partial_o = reinterpret_cast<float *>(partials);
+        p.partial_lse = reinterpret_cast<float *>(partials + o_bytes);
     }
     return launch_decode(ctx, dtype, p);
 }
@@ -605,6 +615,10 @@ int32_t flat_ctx_create(int32_t device, void *stream, flat_ctx **out) {
         ctx->f32_table.dev = nullptr;
         cudaGetLastError();
     }
+    if (cudaMalloc(&ctx->short_partials, kShortPartialBytes) != cudaSuccess) {
+        ctx->short_partials = nullptr;
+        cudaGetLastError();
+    }
     *out = ctx;
     return FLAT_OK;
 }
@@ -622,6 +636,7 @@ void flat_ctx_destroy(flat_ctx *ctx) {
     for (auto &t : ctx->rope_tables)
         if (t.dev) cudaFree(t.dev);
     if (ctx->f32_table.dev) cudaFree(ctx->f32_table.dev);
+    if (ctx->short_partials) cudaFree(ctx->short_partials);
     for (cudaEvent_t e : ctx->pipe_events) cudaEventDestroy(e);
     if (ctx->stream_switch) cudaEventDestroy(ctx->stream_switch);
     if (ctx->copy_in) cudaStreamDestroy(ctx->copy_in);

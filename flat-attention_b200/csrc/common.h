@@ -18,6 +18,7 @@
 namespace flat {
 
 constexpr int kMaxHeadDim = 128;  // WGSL_MAX_HEAD_DIM, src/lib.rs:60
+constexpr uint64_t kShortPartialBytes = 32ull << 20;  // 508 parts of 32 heads at D = 128
 constexpr uint64_t kF32TableBytes = 16ull << 20;  // 32768 positions at head_dim 128
 
 // Device status word written by bounded waits.
@@ -62,6 +63,9 @@ struct flat_ctx {
     // The f32 forward has a table of its own, of kF32TableBytes, allocated with the context (null where the device had no
     // room): it never allocates, and only reads the tables above, whose addresses captured launches hold.
     RopeTable f32_table;
+    // Partials of decode spans shorter than 64 tokens, kShortPartialBytes, allocated with the context (null where the device
+    // had no room: spans are then 64 tokens or more).  The workspace a decode call asks for is that of spans of 64.
+    void *short_partials = nullptr;
     // The tensor-core backward may keep every bf16 dS^T tile in scratch (O(N^2) bytes) so that dQ needs no second score
     // recompute; it does so while that spill fits this budget (flat_ctx_set_backward_scratch_budget).
     uint64_t backward_scratch_budget = 8ull << 30;
@@ -226,6 +230,7 @@ struct DecodeParams {
     int kv_splits;                       // >= 1
     float *partial_o;                    // [splits, num_seqs*q_heads, head_dim] f32 (splits > 1)
     float *partial_lse;                  // [splits, num_seqs*q_heads]
+    int short_partials;                  // the partials go to the context's memory for short spans, not to its workspace
     int chunk_tokens;                    // tokens per split chunk (splits > 1)
     // Balanced mode (tensor-core decode only): sequences, each padded to a multiple of 16 tokens,
     // are laid end to end and CTA i streams tokens [i*span, (i+1)*span) of that line, whatever

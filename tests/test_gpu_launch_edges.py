@@ -8,7 +8,7 @@ from oracle import binding as ob
 from tests.gpu_util import bf16_round, ctx, dev, fa, run_forward
 from tests.test_gpu_backward_bf16 import randn
 from tests.test_gpu_chunked_backward import run_backward
-from tests.test_gpu_decode_cache import oracle_decode, unpack
+from tests.test_gpu_decode_cache import oracle_decode, run_batched, unpack
 
 pytestmark = pytest.mark.gpu
 
@@ -30,6 +30,31 @@ def test_paged_decode_spans_and_tables(n, Hq, Hkv, D):
                            n - 1, 0, True)
     assert np.abs(o.reshape(-1) - eo.reshape(-1)).max() <= 2e-2
     assert np.abs(l.reshape(-1) - el.reshape(-1)).max() <= 2e-3
+    assert c.device_status() == 0
+
+
+# lengths of the batch: single sequences on either side of the span rule, a full batch of short ones, and one long among many
+# short ones, whose parts (dense over all sequences) would take four times the memory with spans of 16 tokens
+@pytest.mark.parametrize("lens", [[700], [2048], [2064], [6000], [8000], [700] * 16, [100] * 128, [2048] + [16] * 11,
+                                  [2048] + [16] * 127])
+def test_decode_asks_for_no_more_workspace_than_spans_of_64(lens):
+    """Shorter spans keep their parts in memory of the context: the workspace is bounded by the parts of 64-token spans."""
+    Hq, Hkv, D, page, c = 32, 8, 128, 16, fa.Context(0)
+    pages = [-(-n // page) for n in lens]
+    g = torch.Generator().manual_seed(3)
+    Q = torch.randn(len(lens), Hq * D, generator=g).bfloat16()
+    K, V = (torch.randn(sum(pages) * page, Hkv * D, generator=g).bfloat16() for _ in range(2))
+    tables = np.zeros((len(lens), max(pages)), np.int32)
+    for i, n in enumerate(pages):
+        tables[i, :n] = sum(pages[:i]) + np.arange(n)
+    args = (fa.BF16, np.array(lens, np.int32), tables, sum(pages), max(pages), Q, K, V, Hq, Hkv, D, page, 5e5)
+    o, l = run_batched(c, *args)
+    padded = [-(-n // 16) * 16 for n in lens]
+    span = max(64, (-(-sum(padded) // (2 * 148)) + 15) // 16 * 16)
+    parts = -(-max(padded) // span) + 1
+    assert c.workspace_bytes() <= (1 << 16) + parts * len(lens) * Hq * (D + 1) * 4 + 256
+    eo, el = run_batched(ctx(), *args, splits=1)
+    assert np.abs(o - eo).max() <= 2e-2 and np.abs(l - el).max() <= 2e-3
     assert c.device_status() == 0
 
 
