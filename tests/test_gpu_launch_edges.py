@@ -58,7 +58,7 @@ def test_decode_asks_for_no_more_workspace_than_spans_of_64(lens):
     assert c.device_status() == 0
 
 
-# (B, Hq, Hkv, N, D): clusters of 1, 2, 3 and 8 CTAs per key tile on 148 SMs, key tiles with fewer pairs than CTAs among them
+# (B, Hq, Hkv, N, D): clusters of 1, 4, 3, 8 and 8 CTAs per key tile on 148 SMs, with and without a mask
 @pytest.mark.parametrize("B,Hq,Hkv,N,D", [(1, 4, 4, 100, 64), (1, 8, 1, 130, 128), (1, 12, 1, 128, 64), (1, 32, 2, 600, 64),
                                           (1, 16, 1, 700, 128)])
 @pytest.mark.parametrize("causal", [True, False])
@@ -73,6 +73,41 @@ def test_backward_clusters(B, Hq, Hkv, N, D, causal):
         # the other backward tests, here it grows with the largest gradient
         assert np.abs(a - e).max() <= 2e-2 + 4e-3 * np.abs(e).max(), (name, float(np.abs(a - e).max()), float(np.abs(e).max()))
     again = run_backward(fa.BF16, B, Hq, Hkv, N, D, causal, None, q, k, v, do, fo, fl)
+    assert all(np.array_equal(x, y) for x, y in zip(got, again))
+    assert ctx().device_status() == 0
+
+
+def cluster_and_fewest_pairs(B, Hq, Hkv, N, causal, sms=148):
+    """CTAs per key tile as the launch chooses them, and the (head, query tile) pairs of the key tile that has the fewest."""
+    n, group = -(-N // 128), Hq // Hkv
+    pairs, longest = (n * (n + 1) // 2 if causal else n * n) * Hq * B, n * group
+    parts = 1
+    while parts < 8 and (parts + 1) * 4 <= longest and 4 * (-(-longest // parts)) * sms > 5 * pairs:
+        parts += 1
+    return parts, group if causal else longest
+
+
+# the last key tile has 1 pair for 2 CTAs, 4 for 8
+@pytest.mark.parametrize("Hq,Hkv,N,parts", [(16, 16, 1000, 2), (8, 2, 1500, 8)])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("budget", [0, 8 << 30])
+def test_backward_clusters_with_idle_ctas(Hq, Hkv, N, parts, D, budget):
+    """CTAs of a cluster without a pair of their own: they stream nothing and still add their share of the others' sums."""
+    size, fewest = cluster_and_fewest_pairs(1, Hq, Hkv, N, True)
+    assert size == parts and fewest < size
+    q, k, v, do = randn(Hq * N * D, 11), randn(Hkv * N * D, 12), randn(Hkv * N * D, 13), randn(Hq * N * D, 14)
+    fo, fl = run_forward("grouped", fa.F32, fa.shape(1, Hq, Hkv, N, N, D), fa.config(True), q, k, v)
+    fo = bf16_round(fo)
+    exp = run_backward(fa.F32, 1, Hq, Hkv, N, D, True, None, q, k, v, do, fo, fl)
+    ctx().set_backward_scratch_budget(budget)
+    try:
+        got, again = (run_backward(fa.BF16, 1, Hq, Hkv, N, D, True, None, q, k, v, do, fo, fl) for _ in range(2))
+    finally:
+        ctx().set_backward_scratch_budget(8 << 30)
+    for name, a, e in zip(("dQ", "dK", "dV"), got, exp):  # the bound of the test above
+        assert np.abs(a - e).max() <= 2e-2 + 4e-3 * np.abs(e).max(), (name, float(np.abs(a - e).max()), float(np.abs(e).max()))
+        a, e = a.reshape(-1, N, D)[:, -(N % 128):], e.reshape(-1, N, D)[:, -(N % 128):]  # the tile of the idle CTAs
+        assert np.abs(a - e).max() <= 2e-2 + 4e-3 * np.abs(e).max(), name
     assert all(np.array_equal(x, y) for x, y in zip(got, again))
     assert ctx().device_status() == 0
 
@@ -94,6 +129,42 @@ def test_backward_head_pairs(D, causal):
         assert np.array_equal(dq[b].reshape(-1), one)
 
 
+@pytest.mark.parametrize("S", [64, 65])
+@pytest.mark.parametrize("dtype", [fa.BF16, fa.F16])
+def test_padded_batches_around_the_lengths_that_travel_with_the_launch(S, dtype):
+    """64 sequences' lengths and offsets are kernel arguments, 65 are copied to the workspace, where a decode plan that was
+    uploaded before them must not be taken for granted.  Against the f32 kernel on the same rounded inputs."""
+    Hq, Hkv, N, D, c = 4, 2, 70, 64, ctx()
+    td = fa.torch_dtype(dtype)
+    q, k, v = (torch.as_tensor(randn(S * N * h * D, 60 + i)).to(td).float().numpy() for i, h in enumerate((Hq, Hkv, Hkv)))
+    rng = np.random.default_rng(S)
+    lens = rng.integers(1, N + 1, S)
+    lens[0], lens[-1] = N, 33
+    seqs = [fa.VarlenSequence(int(n), int(n), 0, int(rng.integers(0, 3000))) for n in lens]
+    cache = fa.CudaPagedKvCache(c, fa.BF16, 16, 40, Hkv, D)
+    kv = torch.randn(2, 600 * Hkv * D, generator=torch.Generator().manual_seed(S)).bfloat16().cuda()
+    cache.record_append(kv[0], kv[1], 600)
+    dq, decoded = dev(randn(Hq * D, 70), torch.bfloat16), []
+
+    def decode():
+        out = c.create_decode_output_buffer(fa.BF16, 1, Hq, D)
+        c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, 599, dq, cache.k_buffer(), cache.v_buffer(), out)
+        decoded.append(out)
+
+    shp, rot = fa.shape(S, Hq, Hkv, N, N, D), fa.rotary(5e5, 0)
+    decode()
+    o, l = run_forward("projection_rope_varlen", dtype, shp, fa.config(True), q, k, v, rot=rot, sequences=seqs)
+    decode()
+    assert torch.equal(*decoded)
+    eo, el = run_forward("projection_rope_varlen", fa.F32, shp, fa.config(True), q, k, v, rot=rot, sequences=seqs)
+    o, l, eo, el = o.reshape(S, N, Hq * D), l.reshape(S, Hq, N), eo.reshape(S, N, Hq * D), el.reshape(S, Hq, N)
+    for b, n in enumerate(lens):
+        assert np.abs(o[b, :n] - eo[b, :n]).max() <= 2e-2, b
+        assert np.abs(l[b, :, :n] - el[b, :, :n]).max() <= 2e-3, b
+        assert np.all(o[b, n:] == 0.0) and np.all(np.isneginf(l[b, :, n:])), b
+    assert c.device_status() == 0
+
+
 def test_exponent_of_head_dim_64_keeps_nan_and_zero():
     """A NaN query row stays NaN in O and LSE and alone; scores far below the row's maximum give exactly nothing."""
     B, H, N, D = 1, 2, 300, 64
@@ -107,6 +178,30 @@ def test_exponent_of_head_dim_64_keeps_nan_and_zero():
     bad[1, 131] = True
     assert np.array_equal(np.isnan(l), bad) and np.array_equal(np.isnan(o).all(-1), bad) and np.array_equal(np.isnan(o).any(-1), bad)
     assert np.array_equal(o[0, 9], v.reshape(H, N, D)[0, 7])
+
+
+@pytest.mark.parametrize("dtype", [fa.BF16, fa.F16])
+def test_exponent_of_head_dim_64_is_accurate(dtype):
+    """LSE of rows whose visible scores are 0 (key 0) and t (the 32 keys whose exponentials leave the special-function unit):
+    log(1 + 32 e^t) shows an error of 2^t at full size."""
+    H, N, D = 8, 128, 64
+    td = fa.torch_dtype(dtype)
+    a = torch.linspace(0, -64, H * N).to(td).double().reshape(H, N)  # t = a / 8 in the natural log domain: 2^0 to 2^-11.5
+    a[0, :4] = torch.tensor([-704.0, -705.0, -2048.0, -30000.0]).to(td).double()  # below 2^-126.5
+    q, k = torch.zeros(H, N, D), torch.zeros(H, N, D)
+    q[:, :, 0], q[:, :, 1] = a.float(), 1.0
+    k[:, 1:, 1] = -30000.0
+    for j in range(N):
+        if j % 8 >= 6:
+            k[:, j, 0], k[:, j, 1] = 1.0, 0.0
+    v = torch.ones(H, N, D)
+    o, l = run_forward("grouped", dtype, fa.shape(1, H, H, N, N, D), fa.config(False), q.numpy(), k.numpy(), v.numpy())
+    want = torch.log1p(32 * torch.exp(a / 8)).numpy()
+    # 2^-22 for the exponentials, 2^-22 for the sum of 33 numbers, 2^-22 for t (the product of score, scale and log2 e, where the
+    # sum depends on it), 2^-21 for log2 and the product with ln 2 at values up to 3.5
+    assert np.abs(l.reshape(H, N) - want).max() <= 5 * 2.0 ** -22, np.abs(l.reshape(H, N) - want).max()
+    assert np.all(l.reshape(H, N)[0, :4] == 0.0)
+    assert np.all(np.abs(o - 1.0) <= 2.0 ** -8)
 
 
 @pytest.mark.parametrize("H", [128, 130])
