@@ -170,7 +170,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
     const int it0 = part * n_total / p.parts;
     const int n_iter = (part + 1) * n_total / p.parts - it0;
 
-    grid_dependency_launch();  // the dQ kernel
+    // the dQ kernel; its CTAs, which take TMEM before they wait, find no registers on an SM that still runs one of these
+    grid_dependency_launch();
     if (threadIdx.x == 0) {
         *abort_flag = (smem_u32(smem) & 1023u) ? 1 : 0;  // a misplaced shared window would break the swizzle: refuse to run
         if (*abort_flag) timeout(p, 90);

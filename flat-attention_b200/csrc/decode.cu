@@ -246,19 +246,17 @@ __global__ void __launch_bounds__(256) decode_kernel(const __grid_constant__ Dec
     }
 }
 
-// Merge of split-KV partials: one CTA of 128 threads per (sequence, q_head) row.
-//   LSE = log(sum_i exp(LSE_i)),  O = sum_i exp(LSE_i - LSE) O_i
-// Phase 1: the threads reduce max and sum of the parts' LSE; phase 2: thread d accumulates column d
-// over the parts with the weights staged in shared memory (coalesced rows, several loads in flight).
 constexpr int kMergeDims = 128;    // threads along the head dimension (kMaxHeadDim)
 constexpr int kMergeGroupsWide = 4;  // thread groups of the wide variant; group g takes the parts g, g + 4, ... of a batch
 constexpr int kMergeWideFrom = 17;   // rows with this many parts or more are merged by the wide variant
 constexpr int kMergeBatch = 512;   // weights staged per pass
 
-// Merge of the split-KV partials that ranks exchange, any head dimension and part stride: LSE = log sum exp(LSE_i),
-// O = sum exp(LSE_i - LSE) O_i.  GROUPS = 1: 128 threads, the parts are added in order.  GROUPS = 4: many parts are spread
-// over four thread groups (the loop is a chain of L2 round trips otherwise) and the groups' sums are added in group order.  Either way eight independent loads are in flight per thread and the result is a fixed
-// function of the inputs and of the part count.
+// Merge of the split-KV partials that ranks exchange, any head dimension and part stride, one CTA per row: LSE = log sum
+// exp(LSE_i), O = sum exp(LSE_i - LSE) O_i.  The threads reduce maximum and sum of the parts' LSEs, then thread d adds up
+// column d with the weights staged in shared memory.  GROUPS = 1: 128 threads, the parts are added in order.  GROUPS = 4:
+// many parts are spread over four thread groups (the loop is a chain of L2 round trips otherwise) and the groups' sums are
+// added in group order.  Either way eight independent loads are in flight per thread and the result is a fixed function of
+// the inputs and of the part count.
 template <typename T, int GROUPS>
 __global__ void __launch_bounds__(kMergeDims * GROUPS) merge_kernel(int parts, int64_t rows, int head_dim,
                                                               const float *__restrict__ partial_o,

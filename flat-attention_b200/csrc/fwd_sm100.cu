@@ -50,14 +50,15 @@ constexpr int kMmaWarp = 9;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
-// At D = 64 the two products of a score cost the tensor pipe half of what they do at D = 128, and the special-function unit
-// (16 exponentials per clock and SM) becomes the bound: every kPolyEvery-th pair of scores takes 2^t from the FMA and
-// integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, D = 64: 135 us without, 133 / 129 / 138 us with every 8th /
-// 4th / 8 of 3 pairs.  At D = 128 the same costs time (the tensor pipe and the power limit bound there: a 32768-token
-// chunked prefill 18.5 -> 19.5 ms), so the flag follows D; nor where K is converted in shared memory (CONVK): the converting
-// warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads, D = 64 979 -> 995 us), nor for K and V behind a page
-// table (the same call with the binary16 shadow 964 -> 984 us) and for padded batches, whose items are short (16 x 1024 rows,
-// 32 / 8 heads 162 -> 165 us).
+// At D = 64 the two products of a score cost the tensor pipe half of what they do at D = 128, and the exponent pass (16
+// exponentials per clock and SM of the special-function unit) is the longest part of the chain of a tile: every kPolyEvery-th
+// pair of scores takes 2^t from the FMA and integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, no mask: 135.4 us
+// without, 130.9 us with every 4th pair (133 us with every 8th, 138 us with 3 of 8); masked calls are within 1.5% of each
+// other (4 x 2000 rows 77.0 and 78.1 us, 8000 rows 387 us both, the training step of 2 x 1000 rows 66.1 and 65.7 us).  At D =
+// 128 it costs time (a 32768-token chunked prefill 18.5 -> 19.5 ms), so the flag follows D; nor is it used where K is
+// converted in shared memory (CONVK): the converting warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads,
+// D = 64 979 -> 995 us), nor for K and V behind a page table (the same call with the binary16 shadow 964 -> 984 us) and for
+// padded batches, whose items are short (16 x 1024 rows, 32 / 8 heads 162 -> 165 us).
 constexpr int kPolyEvery = 4;
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -66,7 +67,7 @@ __device__ __forceinline__ uint64_t pack2(float a, float b) {
     return r;
 }
 // 2^t of two scores, t <= 100: t = n + f with |f| <= 1/2 (adding 1.5 * 2^23 rounds to an integer), 2^f as the minimax
-// polynomial of degree 5 (relative error 7.5e-8, 2.1e-7 as evaluated: that of ex2.approx), scaled by 2^n.  The
+// polynomial of degree 5 (with f32 coefficients 1.6e-7 relative, 2.2e-7 as evaluated; ex2.approx: 2^-22), scaled by 2^n.  The
 // integer carries the exponent bias, so that its low byte shifted by 23 is 2^n; t below -127 gives exactly 0, NaN stays NaN.
 __device__ __forceinline__ void ex2_poly(float &t0, float &t1) {
     constexpr float kRound = 12582912.f + 127.f;
@@ -336,8 +337,9 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
     auto p_part = [&](int w) { return bar0 + 8u * (12 + 3 * C::kStages + w); };   // the first kEarlyKeys columns of P are written
     // ALiBi's exponent pass is longer (the addend advances with the columns), and the value product of the first 96 keys is
     // issued while the last 32 are still being exponentiated: B = 2, 1000 new rows against 3000 keys, 32 / 8 heads, D = 128,
-    // 118.5 -> 111.0 us.  Without the bias the second wait costs the issuing thread more than the overlap gives (587 -> 606 us
-    // for B = 4, N = 4096).
+    // 115.4 -> 106.8 us, D = 64 93.1 -> 91.1; with pre-rotated K, which is converted in shared memory, 116.6 -> 111.2 and
+    // 93.8 -> 90.5; 64 rows against 5000 keys 56.1 -> 53.2.  Without the bias the second wait costs the issuing thread more
+    // than the overlap gives (587 -> 606 us for B = 4, N = 4096).
     constexpr int kEarlyKeys = ALIBI ? 96 : 0;
 
     const int warp = warp_index_uniform();

@@ -195,7 +195,7 @@ def test_variable_length_projection_bf16(B, Hq, Hkv, Nq, Nkv, D, causal, kvoff, 
     launches = ctx().launch_count()
     o, l = run_forward("projection_rope_varlen", fa.BF16, fa.shape(B, Hq, Hkv, Nq, Nkv, D), fa.config(causal), q, k, v,
                        rot=fa.rotary(theta, 0, kvoff), sequences=seqs)
-    # K rotation, padding fill and the tcgen05 kernel (plus the table kernels): the generic kernel is a single launch
+    # K rotation, the tcgen05 kernel and the table kernels: the generic kernel is a single launch
     assert ctx().launch_count() - launches >= 3
     o, l = o.reshape(B, Nq, Hq, D), l.reshape(B, Hq, Nq)
     for b, (aq, akv, coff, qr) in enumerate(meta):
