@@ -82,7 +82,7 @@ template <int D>
 __device__ __forceinline__ bool copied_non_finite(const float *src) {
     constexpr int kVec = D / 4;
     uint64_t zero[4] = {};
-#pragma unroll
+#pragma unroll 2
     for (int u = 0; u < 64 * kVec / kThreads; ++u) {
         const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(src + 4 * (u * kThreads + threadIdx.x));
         fma2(zero[2 * u & 3], x.x, 0);
@@ -131,6 +131,22 @@ __device__ __forceinline__ void load_rotated_rows(float *dst, int stride, const 
                          : make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
+}
+
+// O += P V of a tile of which row r of the thread sees the first `seen` + 16 r keys.  Not inlined: a call of it is rare, and
+// its code beside the plain loop costs that one registers.
+template <int D>
+__device__ __noinline__ void accumulate_seen(uint64_t *o, const float *ps, const float *vs, int seen) {
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    for (int r = 0; r < kRowsPerThread; ++r)
+        for (int k = 0; k < min(kKeys, seen + 16 * r); ++k) {
+            const float x = ps[(ty + 16 * r) * Tile<D>::kPStride + k];
+            for (int c = 0; c < D / 32; ++c) {
+                const ulonglong2 vv = *reinterpret_cast<const ulonglong2 *>(vs + k * D + 4 * tx + 32 * c);
+                fma2(o[(r * (D / 32) + c) * 2], pack2(x, x), vv.x);
+                fma2(o[(r * (D / 32) + c) * 2 + 1], pack2(x, x), vv.y);
+            }
+        }
 }
 
 template <int D, bool ALIBI>
@@ -258,10 +274,10 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
         }
         cp_async_wait_all();
         // On the causal diagonal a row does not see all keys of the tile: their probability is 0, which keeps a finite V out
-        // of the row and a non-finite one not.  Each thread looks through the V it copied itself (8 heads, D = 128:
-        // 45.1 us for 512 rows with and without, 403 -> 408 us for 2048; D = 64, 300 rows 17.8 -> 18.3 us), and only a tile
-        // that does hold a non-finite value takes the loop that leaves keys out row by row (in every diagonal tile the
-        // comparison costs a short call a fifth: 64 rows 16.4 -> 20.5 us).
+        // of the row and a non-finite one not.  Each thread looks through the V it copied itself, and only a tile that does
+        // hold a non-finite value takes the loop that leaves keys out row by row.  Kernel times without / with the search, 8 / 2
+        // heads, D = 128: 512 rows 43.6 / 43.9 us, 356 rows 37.9 / 38.7, 2048 rows 393 / 391; D = 64, 300 rows 15.9 / 16.1
+        // (that loop in every diagonal tile: 64 rows 16.4 -> 20.5 us; inlined for the rare case, 2048 rows 403).
         const bool diagonal = p.causal && k0 + kKeys > p.causal_off + r0 + 1;
         bool by_row = false;
         if (diagonal) by_row = __syncthreads_or(copied_non_finite<D>(vs));
@@ -294,22 +310,12 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
                 }
             }
         } else {
-#pragma unroll 1
-            for (int k = 0; k < kKeys; ++k) {
+            uint64_t copy[kRowsPerThread * 2 * kCols];
 #pragma unroll
-                for (int r = 0; r < kRowsPerThread; ++r) {
-                    const int row = ty + 16 * r;
-                    if (k0 + k > p.causal_off + r0 + row) continue;
-                    const float x = ps[row * T::kPStride + k];
-                    const uint64_t x2 = pack2(x, x);
+            for (int i = 0; i < kRowsPerThread * 2 * kCols; ++i) copy[i] = o[i / (2 * kCols)][i % (2 * kCols)];
+            accumulate_seen<D>(copy, ps, vs, (int)(p.causal_off + r0 + ty + 1 - k0));
 #pragma unroll
-                    for (int c = 0; c < kCols; ++c) {
-                        const ulonglong2 vv = *reinterpret_cast<const ulonglong2 *>(vs + k * D + 4 * tx + 32 * c);
-                        fma2(o[r][2 * c], x2, vv.x);
-                        fma2(o[r][2 * c + 1], x2, vv.y);
-                    }
-                }
-            }
+            for (int i = 0; i < kRowsPerThread * 2 * kCols; ++i) o[i / (2 * kCols)][i % (2 * kCols)] = copy[i];
         }
         __syncthreads();  // the next tile overwrites P and V
     }
