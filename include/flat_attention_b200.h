@@ -181,7 +181,9 @@ typedef struct flat_resident_kv_cache flat_resident_kv_cache;
 /* ---- context ------------------------------------------------------------------------- */
 
 /* WgpuFlatAttention::new (src/wgpu_backend.rs:177-255): bind to one device.  `stream` is a
- * cudaStream_t (NULL = legacy default stream); the caller owns it, like the wgpu queue. */
+ * cudaStream_t (NULL = legacy default stream); the caller owns it, like the wgpu queue.  48 MiB of
+ * device memory come with the context (f32 rotation angles, partial results of short decode spans);
+ * where the device has no room for them the calls do without. */
 int32_t flat_ctx_create(int32_t device, void *stream, flat_ctx **out);
 void flat_ctx_destroy(flat_ctx *ctx);
 /* Replace the stream later launches are enqueued on.  The new stream is made to wait (on the
