@@ -1,18 +1,28 @@
 // tcgen05 forward: causal / non-causal online-softmax attention for bf16 storage, head_dim 64 or
 // 128, GQA by head mapping, RoPE, rectangular shapes, K/V contiguous or read through a page table.
 //
-// One CTA owns 256 consecutive query rows of one (batch, q_head) as two 128-row tiles that
-// ping-pong on the tensor core.  Warp roles (384 threads):
-//   warps 0-3  softmax of Q tile 0 : thread t owns query row t (TMEM lane t), no shuffles
-//   warps 4-7  softmax of Q tile 1
-//   warp  8    TMA producer        : Q tiles once, then K_j, V_j through an mbarrier ring
-//   warp  9    MMA issuer          : one thread issues every tcgen05.mma and tcgen05.commit
-//   warps 10-11 K converters       : bf16 -> fp16 of each K tile in place (only when Q is rotated against bf16 K)
-// Per KV tile j and Q tile w:  S_w = Q_w K_j^T (SS MMA, f32 in TMEM)  ->  softmax warps read S_w
-// from TMEM, track the running max (rescaling O_w in TMEM only when the max grows by more than
-// 2^8), write P_w = exp2(S_w*c - m) as bf16 over S_w  ->  O_w += P_w V_j (A operand from TMEM).
-// The N x N matrix never leaves TMEM.  Tensor-core order S0 S1 | PV0 S0' PV1 S1' | ... keeps the
-// pipe busy with one tile's MMAs while the other tile is in softmax.
+// One CTA owns 256 consecutive query rows of one (batch, q_head) as two 128-row tiles ("slots") that
+// share the tensor core.  Warp roles (512 threads):
+//   warps 0-3   softmax of slot 0 : thread t owns query row t (TMEM lane t), no shuffles
+//   warps 4-7   softmax of slot 1
+//   warps 8-11  rotate the Q tiles of the next work item, store the O tiles of the finished one
+//   warp  12    TMA producer      : Q tiles, K_j and V_j through mbarrier rings
+//   warp  13    one thread issues the score products, one of warp 14 the value products
+//   warps 14-15 K converters      : bf16 -> fp16 of each K tile in place (only when Q is rotated against bf16 K; the value
+//                                   products are then issued by warp 13 too)
+// Per KV tile j and slot w:  S_w = Q_w K_j^T (SS MMA, f32 in TMEM)  ->  softmax warps load S_w into registers and free the
+// score tile, track the running max (rescaling O_w in TMEM only when the max grows by more than 2^8), write
+// P_w = exp2(S_w*c - m) as bf16 to TMEM columns of its own  ->  O_w += P_w V_j (A operand from TMEM).
+// The N x N matrix never leaves TMEM.  Since P does not lie over S, the next scores are formed while the softmax warps work:
+// at D = 64 each slot has a score tile of its own, at D = 128 (512 columns: O 2 x 128, P 2 x 64, S 128) both slots take one
+// in turn, which also keeps them half a period apart.  While P lay over S a slot's chain was softmax, value product, next
+// scores, one after another: B=4, 32/8 heads, N=4096, D=128, causal, RoPE 597 us a pass, 514 now; a 32768-token chunked
+// prefill 18.6 ms, 15.1 now; binary16 encoder 8 x 1500, 16 heads, D=64 131 us, 119 now; 16 padded prompts of 1024 rows 223
+// and 195 us.
+// The softmax warps hold a whole score row (128 registers) and must not spill: a spilled register is a store that the next
+// mbarrier arrival has to wait for (the period of a tile pair went from 4.7k to 3.4k clk when the spills went).  The code is
+// kept small for the same reason: ten warps run five different loops, and 86 KB of instructions missed the instruction
+// cache 78 times per tile pair.
 //
 // RoPE: Q is rotated inside this kernel.  The raw bf16 Q tile lands in shared memory by TMA, the
 // softmax thread that owns a row rotates it in place with a (cos, sin) table of the call's
@@ -23,7 +33,7 @@
 // holds rotated bf16 K (rotate_k = 0) only Q is rotated; tcgen05.mma kind::f16 takes A and B of
 // one format only, so each bf16 K tile is then converted to fp16 in place in shared memory by two
 // otherwise idle warps (CONVK; exact for |k| in the normal fp16 range, saturating beyond 65504)
-// before the MMA warp may use it.
+// before the score products may use it.
 // Semantics: Appendix of the forward contract (src/projection_asymmetric.rs:97-238): key k is
 // visible to local row q iff !causal || k <= query_position_offset + q; LSE = max + ln(sum).
 #include <cuda.h>
@@ -44,9 +54,13 @@ namespace {
 using namespace sm100;
 
 constexpr int kTileRows = 128;
-constexpr int kThreads = 384;
-constexpr int kProducerWarp = 8;
-constexpr int kMmaWarp = 9;
+constexpr int kThreads = 512;
+constexpr int kStoreWarp = 8;
+constexpr int kProducerWarp = 12;
+constexpr int kMmaWarp = 13;  // ... and the one after it, or two that convert K tiles
+// Registers of the softmax, the rotating and storing, and the issuing warps.  setmaxnreg.inc draws on what the CTA was
+// launched with (128 registers x 512 threads); a split whose sum is above that would wait for ever.
+constexpr int kRegsSoftmax = 184, kRegsStore = 80, kRegsIssue = 64;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
@@ -93,7 +107,7 @@ __device__ __forceinline__ void ex2_poly(float &t0, float &t1) {
 }
 
 // Debug timeline (compiled in with -DFLAT_TRACE): clock64 stamps of CTA FLAT_TRACE_BLOCK (default 0), written to the buffer whose
-// address is given in the environment variable FLAT_TRACE_PTR.  Layout [role 0..2][iteration 0..63][slot 0..7].
+// address is given in the environment variable FLAT_TRACE_PTR.  Layout [softmax warp 0..7, issuing warps][iteration 0..63][slot 0..7].
 #ifndef FLAT_TRACE_ITEM
 #define FLAT_TRACE_ITEM 0  // the item of the CTA whose KV loop is stamped
 #endif
@@ -101,14 +115,11 @@ __device__ __forceinline__ void ex2_poly(float &t0, float &t1) {
 #ifndef FLAT_TRACE_BLOCK
 #define FLAT_TRACE_BLOCK 0
 #endif
-#define TRACE(role, it, slot)                                                                          \
+#define TRACE_VARS bool tr_on = false; int tr_j = 0
+#define TRACE_STEP(k, j) tr_on = (k) == FLAT_TRACE_ITEM, tr_j = (j)
+#define TRACE_MMA(slot)                                                                                \
     do {                                                                                               \
-        if (p.trace && trace_item && blockIdx.x == FLAT_TRACE_BLOCK && (it) < 64) p.trace[((role) * 64 + (it)) * 8 + (slot)] = clock64(); \
-    } while (0)
-#define TRACEB(k, role, slot)                                                                                \
-    do {                                                                                                     \
-        if (p.trace && blockIdx.x == FLAT_TRACE_BLOCK && (k) >= 0 && (k) < 4)                                 \
-            p.trace[((role) * 64 + 56 + (k)) * 8 + (slot)] = clock64();                                      \
+        if (p.trace && tr_on && blockIdx.x == FLAT_TRACE_BLOCK && tr_j < 64) p.trace[(8 * 64 + tr_j) * 8 + (slot)] = clock64(); \
     } while (0)
 // Stamps of the softmax loop are kept in registers and written one iteration later, so that no global store is
 // outstanding when the thread signals the MMA warp.
@@ -120,11 +131,12 @@ __device__ __forceinline__ void ex2_poly(float &t0, float &t1) {
             for (int s_ = 0; s_ < 5; ++s_) p.trace[((role) * 64 + (it)) * 8 + s_] = tr_[s_];                   \
     } while (0)
 #else
-#define TRACE(role, it, slot) do { } while (0)
+#define TRACE_VARS do { } while (0)
+#define TRACE_STEP(k, j) do { } while (0)
+#define TRACE_MMA(slot) do { } while (0)
 #define TRACE_LOCAL do { } while (0)
 #define TRACE_STAMP(slot) do { } while (0)
 #define TRACE_FLUSH(role, it) do { } while (0)
-#define TRACEB(k, role, slot) do { } while (0)
 #endif
 
 // Division of a non-negative int by a divisor fixed for the launch, as a multiply-high and a shift (the work-item
@@ -157,7 +169,7 @@ struct KernelParams {
     int batch, q_heads, kv_heads, q_len, kv_len, group;
     FastDiv div_bh, div_heads, div_group;  // by batch * q_heads, by q_heads, by group
     int causal;
-    long long causal_off;
+    int causal_off;  // clamped to the keys and rows a call can have
     float scale_log2;
     uint32_t idesc_qk, idesc_pv;
     const int32_t *page_table;
@@ -190,11 +202,13 @@ template <int D, bool CONVK> struct Cfg {
     static constexpr int kBoxes = D / 64;                  // 64-element (128-byte) column boxes per row
     static constexpr int kBoxBytes = kTileRows * 128;      // 128 rows x 128 B
     static constexpr int kTileBytes = kBoxes * kBoxBytes;  // one Q / K / V tile
-    static constexpr int kStages = D == 128 ? 4 : 8;  // K/V ring entries
-    static constexpr int kOutStageBytes = kTileRows * 128;  // one box of the O tile: 128 rows x 64 columns of 16 bits
-    static constexpr int kBars = 2 + 3 * kStages + 12;
-    static constexpr int kSmemBytes = (2 + kStages) * kTileBytes + 2 * kOutStageBytes + kBars * 8 + 16 + 32 + 1024;
-    static_assert(kSmemBytes <= 232448, "shared memory of one CTA");
+    static constexpr int kStages = D == 128 ? 2 : 4;       // entries of the K ring, and of the V ring
+    static constexpr int kOutStageBytes = kTileRows * 128; // one box of the O tile: 128 rows x 64 columns of 16 bits
+    static constexpr int kMlBytes = 2 * kTileRows * 8;     // (max, sum) of the finished rows, per slot
+    static constexpr int kSBufs = D == 128 ? 1 : 2;        // score tiles in TMEM
+    static constexpr int kBars = 20 + 5 * kStages;
+    static constexpr int kSmemBytes = (2 + 2 * kStages) * kTileBytes + kOutStageBytes + kMlBytes + 1024;
+    static_assert(kSmemBytes + kBars * 8 + 64 <= 232448, "shared memory of one CTA");
 };
 
 __device__ __forceinline__ void record_timeout(const KernelParams &p, int where) {
@@ -212,7 +226,7 @@ struct WorkItem {
     int j0;          // first KV tile of the item (0 unless it is a part of a split item)
     int part_slot;   // split items: index of this part's partial record; -1 = the item writes the final result
     int q_len, kv_len;     // this batch element's live rows (the call's lengths unless it is a variable-length batch)
-    long long causal_off;  // key k is visible to local row q iff k <= causal_off + q
+    int causal_off;        // key k is visible to local row q iff k <= causal_off + q
     int table_row0;        // row of the (cos, sin) table that belongs to local query row 0
 };
 
@@ -247,18 +261,15 @@ __device__ __forceinline__ WorkItem make_item_whole(const KernelParams &p, int l
         const flat_varlen_sequence m = p.varlen ? p.varlen[it.b] : p.varlen_inline[it.b];
         it.q_len = (int)m.active_query_len;
         it.kv_len = (int)m.active_kv_len;
-        it.causal_off = m.causal_query_offset;
+        it.causal_off = (int)min(m.causal_query_offset, 1u << 30);
         it.table_row0 = (int)((long long)m.query_rope_offset - p.rope_table_base);
     }
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
         const int first = it.r0 + w * kTileRows;
-        long long visible = it.kv_len;
-        if (p.causal) {
-            const long long last_row = min(first + kTileRows - 1, it.q_len - 1);
-            visible = min((long long)it.kv_len, it.causal_off + last_row + 1);
-        }
-        it.n_tiles[w] = first < it.q_len ? (int)((visible + kTileRows - 1) / kTileRows) : 0;
+        int visible = it.kv_len;
+        if (p.causal) visible = min(visible, it.causal_off + min(first + kTileRows, it.q_len));
+        it.n_tiles[w] = first < it.q_len ? (visible + kTileRows - 1) / kTileRows : 0;
     }
     return it;
 }
@@ -303,6 +314,79 @@ __device__ __forceinline__ int item_index(const KernelParams &p, int k) {
     return idx < p.total_items ? (int)idx : -1;
 }
 
+// Rotates a slot's Q tile in place (bf16 or binary16 in, fp16 out).  A warp rotates its 32 rows; lane l takes the 16-byte
+// chunk (l mod CH) of row (step * RPS + l / CH), so that the (cos, sin) table is read in contiguous row segments.
+// Four chunks are fetched before any of them is written back: the loads are then in flight together instead of each waiting
+// behind the previous step's store.  (Not all of them: the code would be four times as long, see fwd_sm100_kernel.)
+template <int D, bool F16IO>
+__device__ __forceinline__ void rotate_q_tile(const KernelParams &p, const WorkItem &nx, int w, uint8_t *tile, int lane_base, int lane) {
+    constexpr int kBatch = 4;
+    constexpr int kBoxBytes = kTileRows * 128;
+    constexpr int CH = D / 8;     // 16-byte chunks (8 elements, 4 pairs) per row
+    constexpr int RPS = 32 / CH;  // rows per step of one warp
+    static_assert(CH % kBatch == 0, "whole batches");
+    const int ch = lane % CH;
+    const int first_row = nx.r0 + w * kTileRows;
+    // (cos, sin) of the lane's first row come from the table; each further step advances the angle by
+    // RPS positions with the rotation (cos, sin)(RPS * inv_freq), which keeps the table traffic at two
+    // 16-byte loads per thread.  The recurrence error (a few 1e-7 over CH steps) is far below the
+    // rounding of the fp16 result.
+    float cc[4], ss[4], cstep[4], sstep[4];
+    {
+        const int rr = nx.table_row0 + min(first_row + lane_base + lane / CH, nx.q_len - 1);
+        const float4 *tp = reinterpret_cast<const float4 *>(p.rope_q_table + (long long)rr * (D / 2)) + 2 * ch;
+        const float4 cs0 = __ldg(tp), cs1 = __ldg(tp + 1);  // (c, s, c, s) x 2
+        cc[0] = cs0.x; ss[0] = cs0.y; cc[1] = cs0.z; ss[1] = cs0.w;
+        cc[2] = cs1.x; ss[2] = cs1.y; cc[3] = cs1.z; ss[3] = cs1.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 stp = p.rope_step[ch * 4 + e];
+            cstep[e] = stp.x;
+            sstep[e] = stp.y;
+        }
+    }
+#pragma unroll 1
+    for (int s0 = 0; s0 < CH; s0 += kBatch) {
+        uint4 raw[kBatch];
+#pragma unroll
+        for (int st = 0; st < kBatch; ++st) {
+            const int rt = lane_base + (s0 + st) * RPS + lane / CH;  // row in tile
+            raw[st] = *reinterpret_cast<const uint4 *>(tile + (ch >> 3) * kBoxBytes + rt * 128 + (((ch & 7) ^ (rt & 7)) << 4));
+        }
+#pragma unroll
+        for (int st = 0; st < kBatch; ++st) {
+            const int rt = lane_base + (s0 + st) * RPS + lane / CH;  // row in tile
+            const int off = (ch >> 3) * kBoxBytes + rt * 128 + (((ch & 7) ^ (rt & 7)) << 4);
+            if (first_row + rt < nx.q_len) {  // rows past q_len are not used
+                const uint32_t in[4] = {raw[st].x, raw[st].y, raw[st].z, raw[st].w};
+                uint32_t hi[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    float x, y;
+                    if constexpr (F16IO) {
+                        const float2 xy = __half22float2(*reinterpret_cast<const __half2 *>(&in[e]));
+                        x = xy.x;
+                        y = xy.y;
+                    } else {
+                        x = __uint_as_float(in[e] << 16);
+                        y = __uint_as_float(in[e] & 0xffff0000u);
+                    }
+                    const float rx = x * cc[e] - y * ss[e], ry = x * ss[e] + y * cc[e];
+                    const __half2 h2 = __floats2half2_rn(rx, ry);
+                    hi[e] = *reinterpret_cast<const uint32_t *>(&h2);
+                }
+                *reinterpret_cast<uint4 *>(tile + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float c1 = cc[e] * cstep[e] - ss[e] * sstep[e];
+                ss[e] = ss[e] * cstep[e] + cc[e] * sstep[e];
+                cc[e] = c1;
+            }
+        }
+    }
+}
+
 // ALIBI: the softmax warps add slope[q_head] * (key position - query position) to every scaled score
 // (src/attention_bias.rs:82-95) before the running maximum is taken.
 // F16IO: Q, K, V and O are IEEE binary16 instead of bf16 (P is then written as binary16 too, since one MMA takes A and B
@@ -317,30 +401,34 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *q_s = smem;
-    uint8_t *kv_s = smem + 2 * C::kTileBytes;
-    uint8_t *o_stage = kv_s + C::kStages * C::kTileBytes;  // per slot: staging of one 64-column box of the O tile
-    uint64_t *bars = reinterpret_cast<uint64_t *>(o_stage + 2 * C::kOutStageBytes);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + C::kBars);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    volatile SplitRecord *split_rec = reinterpret_cast<volatile SplitRecord *>(tmem_slot + 2);
+    uint8_t *k_s = smem + 2 * C::kTileBytes;
+    uint8_t *v_s = k_s + C::kStages * C::kTileBytes;
+    uint8_t *o_stage = v_s + C::kStages * C::kTileBytes;  // per storing warp: 32 rows of a 64-column box of the O tile
+    float2 *ml_s = reinterpret_cast<float2 *>(o_stage + C::kOutStageBytes);  // per slot: (max, sum) of the finished item's rows
+    // (statically allocated: their addresses are constants, which the issuing threads need not keep in registers)
+    __shared__ uint64_t bars[C::kBars];
+    __shared__ uint32_t tmem_slot[1];
+    __shared__ int abort_word;
+    __shared__ SplitRecord split_record;
+    volatile int *abort_flag = &abort_word;
+    volatile SplitRecord *split_rec = &split_record;
 
     const uint32_t bar0 = smem_u32(bars);
-    auto q_full = [&](int w) { return bar0 + 8u * w; };
-    auto kv_full = [&](int s) { return bar0 + 8u * (2 + s); };
-    auto kv_empty = [&](int s) { return bar0 + 8u * (2 + C::kStages + s); };
-    auto s_full = [&](int w) { return bar0 + 8u * (2 + 2 * C::kStages + w); };
-    auto p_full = [&](int w) { return bar0 + 8u * (4 + 2 * C::kStages + w); };
-    auto o_final = [&](int w) { return bar0 + 8u * (6 + 2 * C::kStages + w); };
-    auto q_ready = [&](int w) { return bar0 + 8u * (8 + 2 * C::kStages + w); };
-    auto q_empty = [&](int w) { return bar0 + 8u * (10 + 2 * C::kStages + w); };
-    auto k_ready = [&](int s) { return bar0 + 8u * (12 + 2 * C::kStages + s); };  // K tile converted (CONVK)
-    auto p_part = [&](int w) { return bar0 + 8u * (12 + 3 * C::kStages + w); };   // the first kEarlyKeys columns of P are written
-    // ALiBi's exponent pass is longer (the addend advances with the columns), and the value product of the first 96 keys is
-    // issued while the last 32 are still being exponentiated: B = 2, 1000 new rows against 3000 keys, 32 / 8 heads, D = 128,
-    // 115.4 -> 106.8 us, D = 64 93.1 -> 91.1; with pre-rotated K, which is converted in shared memory, 116.6 -> 111.2 and
-    // 93.8 -> 90.5; 64 rows against 5000 keys 56.1 -> 53.2.  Without the bias the second wait costs the issuing thread more
-    // than the overlap gives (587 -> 606 us for B = 4, N = 4096).
-    constexpr int kEarlyKeys = ALIBI ? 96 : 0;
+    auto q_full = [&](int w) { return bar0 + 8u * w; };         // Q tile landed
+    auto q_ready = [&](int w) { return bar0 + 8u * (2 + w); };  // Q tile rotated
+    auto q_empty = [&](int w) { return bar0 + 8u * (4 + w); };  // last score product of the slot's tile done
+    auto s_full = [&](int w) { return bar0 + 8u * (6 + w); };   // score product of the slot done
+    auto s_free = [&](int b) { return bar0 + 8u * (8 + b); };   // score tile b is in registers
+    auto p_full = [&](int w) { return bar0 + 8u * (10 + w); };  // P of the slot written
+    auto pv_done = [&](int w) { return bar0 + 8u * (12 + w); }; // value product of the slot done
+    auto o_final = [&](int w) { return bar0 + 8u * (14 + w); }; // last value product of the slot's item done
+    auto o_free = [&](int w) { return bar0 + 8u * (16 + w); };  // the slot's O and (max, sum) have been read
+    auto ml_full = [&](int w) { return bar0 + 8u * (18 + w); }; // (max, sum) of the slot's item written
+    auto k_full = [&](int s) { return bar0 + 8u * (20 + s); };
+    auto k_empty = [&](int s) { return bar0 + 8u * (20 + C::kStages + s); };
+    auto v_full = [&](int s) { return bar0 + 8u * (20 + 2 * C::kStages + s); };
+    auto v_empty = [&](int s) { return bar0 + 8u * (20 + 3 * C::kStages + s); };
+    auto k_ready = [&](int s) { return bar0 + 8u * (20 + 4 * C::kStages + s); };  // K tile converted (CONVK)
 
     const int warp = warp_index_uniform();
     const int lane = threadIdx.x & 31;
@@ -350,16 +438,21 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
         *abort_flag = 0;
         for (int w = 0; w < 2; ++w) {
             mbar_init(q_full(w), 1);
-            mbar_init(s_full(w), 1);
-            mbar_init(p_full(w), 4);
-            mbar_init(p_part(w), 4);
-            mbar_init(o_final(w), 1);
             mbar_init(q_ready(w), 4);
             mbar_init(q_empty(w), 1);
+            mbar_init(s_full(w), 1);
+            mbar_init(s_free(w), 4);
+            mbar_init(p_full(w), 4);
+            mbar_init(pv_done(w), 1);
+            mbar_init(o_final(w), 1);
+            mbar_init(o_free(w), 4);
+            mbar_init(ml_full(w), 4);
         }
         for (int s = 0; s < C::kStages; ++s) {
-            mbar_init(kv_full(s), 1);
-            mbar_init(kv_empty(s), 1);
+            mbar_init(k_full(s), 1);
+            mbar_init(k_empty(s), 1);
+            mbar_init(v_full(s), 1);
+            mbar_init(v_empty(s), 1);
             mbar_init(k_ready(s), 2);  // one arrival per converter warp
         }
         mbar_fence_init();
@@ -390,193 +483,240 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t col_s[2] = {0u, 128u};
-    const uint32_t col_o[2] = {256u, 256u + D};
+    // TMEM columns: O of both slots, P of both slots, and behind them one score tile (D = 128) or one per slot (D = 64)
+    auto col_o = [](int w) { return (uint32_t)(w * D); };
+    auto col_p = [](int w) { return (uint32_t)(2 * D + w * 64); };
+    auto col_s = [](int w) { return (uint32_t)(2 * D + 128 + (C::kSBufs == 2 ? w * 128 : 0)); };
 
-    // Register rebalancing: a softmax thread holds a whole 128-column score row in registers.  The pool that
-    // setmaxnreg.inc draws from is what the CTA was launched with (168 registers x 384 threads), not the whole
-    // register file: 56 x 128 + 224 x 256 uses exactly that, and a larger request would block for ever.
-    static_assert(56 * 128 + 224 * 256 <= 168 * kThreads, "setmaxnreg split exceeds the CTA's register allocation");
-    if (warp >= 8) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    static_assert(kRegsSoftmax * 256 + kRegsStore * 128 + kRegsIssue * 128 <= 128 * kThreads,
+                  "setmaxnreg split exceeds the CTA's register allocation");
+    if (warp >= kProducerWarp) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == kProducerWarp) {
         // ================= TMA producer =================
         // The whole warp walks the loop (waits are uniform); lane 0 issues the contiguous loads, and with a page
-        // table lane i fetches the id of page i of the tile and issues that page's boxes, so that the page-table
-        // reads of a tile are one parallel access instead of a chain of dependent loads in one thread.
-        {
-            bool ok = true;
-            uint32_t ring = 0;             // K/V ring entries requested so far
-            uint32_t q_loads[2] = {0, 0};  // Q tiles requested so far, per slot
-            for (int k = 0; ok; ++k) {
-                const int lin = item_index(p, k);
-                if (lin < 0) break;
-                const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
-                const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
-                for (int w = 0; w < 2 && ok; ++w) {
-                    if (it.n_tiles[w] == 0) continue;
-                    // the slot is free once every S MMA of its previous tile has completed
-                    if (q_loads[w] > 0 && !mbar_wait(q_empty(w), (q_loads[w] - 1) & 1, abort_flag)) {
-                        if (lane == 0) record_timeout(p, 110 + w);
-                        ok = false;
-                    }
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    ++q_loads[w];
-                    if (lane == 0) {
-                        mbar_expect_tx(q_full(w), C::kTileBytes);
-                        for (int kb = 0; kb < C::kBoxes; ++kb)
-                            tma_load_4d(smem_u32(q_s + w * C::kTileBytes + kb * C::kBoxBytes), &p.map_q, kb * 64,
-                                        it.r0 + w * kTileRows, it.h, it.b, q_full(w));
-                    }
+        // table lane i fetches the id of page i of a tile, one tile ahead of its load, and issues that page's boxes, so
+        // that the page-table reads of a tile are one parallel access instead of a chain of dependent loads in one thread.
+        bool ok = true;
+        uint32_t k_cnt = 0, v_cnt = 0;  // K / V tiles requested so far
+        uint32_t q_loads[2] = {0, 0};   // Q tiles requested so far, per slot
+        WorkItem it{};
+        int page_k = 0, page_v = 0, page_next = 0;  // this lane's page of the next K tile, of the next V tile, of the K tile after
+        const int pages_per_tile = p.page_table ? kTileRows / p.page_size : 0;
+        auto fetch_page = [&](int j) {
+            const int tok = (it.j0 + j) * kTileRows + lane * p.page_size;
+            return lane < pages_per_tile && tok < p.kv_len ? p.page_table[(long long)it.b * p.max_pages + tok / p.page_size]
+                                                           : p.physical_pages;  // out of range: zero fill
+        };
+        auto load_q = [&](int w) {
+            if ((w ? it.n_tiles[1] : it.n_tiles[0]) == 0 || !ok) return;
+            // the slot is free once every S MMA of its previous tile has completed
+            if (q_loads[w] > 0 && !mbar_wait(q_empty(w), (q_loads[w] - 1) & 1, abort_flag)) {
+                if (lane == 0) record_timeout(p, 110 + w);
+                ok = false;
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            ++q_loads[w];
+            if (lane == 0) {
+                mbar_expect_tx(q_full(w), C::kTileBytes);
+                for (int kb = 0; kb < C::kBoxes; ++kb)
+                    tma_load_4d(smem_u32(q_s + w * C::kTileBytes + kb * C::kBoxBytes), &p.map_q, kb * 64, it.r0 + w * kTileRows,
+                                it.h, it.b, q_full(w));
+            }
+        };
+        auto load_kv = [&](bool is_k, int j) {
+            if (!ok) return;
+            uint32_t &cnt = is_k ? k_cnt : v_cnt;
+            const int s = cnt % C::kStages;
+            const uint32_t phase = (cnt / C::kStages) & 1;
+            if (!mbar_wait(is_k ? k_empty(s) : v_empty(s), phase ^ 1, abort_flag)) {
+                if (lane == 0) record_timeout(p, 100 + s);
+                ok = false;
+            }
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) return;
+            ++cnt;
+            const CUtensorMap *map = is_k ? &p.map_k : &p.map_v;
+            const uint32_t dst = smem_u32((is_k ? k_s : v_s) + s * C::kTileBytes);
+            const uint32_t full = is_k ? k_full(s) : v_full(s);
+            if (lane == 0) mbar_expect_tx(full, C::kTileBytes);
+            if (p.page_table) {
+                const int page = is_k ? page_k : page_v;
+                __syncwarp();  // the expect_tx above precedes every load of the entry
+                if (lane < pages_per_tile) {
+                    for (int kb = 0; kb < C::kBoxes; ++kb)
+                        tma_load_4d(dst + kb * C::kBoxBytes + lane * p.page_size * 128, map, kb * 64, 0, it.kvh, page, full);
                 }
-                if (k == 0) grid_dependency_wait();  // K may come from the rotation kernel before this one; Q does not
-                int page = 0;  // this lane's page of the current KV tile (paged mode), fetched with the K entry
-                for (int i = 0; ok && i < 2 * n_max; ++i, ++ring) {
-                    const int s = ring % C::kStages;
-                    const uint32_t phase = (ring / C::kStages) & 1;
-                    if (!mbar_wait(kv_empty(s), phase ^ 1, abort_flag)) {
-                        if (lane == 0) record_timeout(p, 100 + s);
-                        ok = false;
-                    }
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    const int j = i >> 1;
-                    const CUtensorMap *map = (i & 1) ? &p.map_v : &p.map_k;
-                    const uint32_t dst = smem_u32(kv_s + s * C::kTileBytes);
-                    if (lane == 0) mbar_expect_tx(kv_full(s), C::kTileBytes);
-                    if (p.page_table) {
-                        const int pages_per_tile = kTileRows / p.page_size;
-                        if ((i & 1) == 0 && lane < pages_per_tile) {
-                            const int tok = (it.j0 + j) * kTileRows + lane * p.page_size;
-                            page = tok < p.kv_len ? p.page_table[(long long)it.b * p.max_pages + tok / p.page_size]
-                                                  : p.physical_pages;  // out of range: zero fill
-                        }
-                        __syncwarp();  // the expect_tx above precedes every load of the entry
-                        if (lane < pages_per_tile) {
-                            for (int kb = 0; kb < C::kBoxes; ++kb)
-                                tma_load_4d(dst + kb * C::kBoxBytes + lane * p.page_size * 128, map, kb * 64, 0, it.kvh, page,
-                                            kv_full(s));
-                        }
-                    } else if (lane == 0) {
-                        for (int kb = 0; kb < C::kBoxes; ++kb)
-                            tma_load_4d(dst + kb * C::kBoxBytes, map, kb * 64, (it.j0 + j) * kTileRows, it.kvh, it.b, kv_full(s));
-                    }
+            } else if (lane == 0) {
+                for (int kb = 0; kb < C::kBoxes; ++kb)
+                    tma_load_4d(dst + kb * C::kBoxBytes, map, kb * 64, (it.j0 + j) * kTileRows, it.kvh, it.b, full);
+            }
+        };
+        for (int k = 0; ok; ++k) {
+            const int lin = item_index(p, k);
+            if (lin < 0) break;
+            it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
+            const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
+            if (p.page_table && n_max > 0) {
+                page_k = fetch_page(0);
+                page_next = fetch_page(1);
+            }
+            load_q(0);
+            if (k == 0) grid_dependency_wait();  // K may come from the rotation kernel before this one; Q does not
+            if (n_max > 0) load_kv(true, 0);
+            load_q(1);
+            for (int j = 0; ok && j < n_max; ++j) {  // the scores of tile j + 1 are formed before the values of tile j
+                if (p.page_table) {
+                    page_v = page_k;
+                    page_k = page_next;
+                    page_next = fetch_page(j + 2);
                 }
+                if (j + 1 < n_max) load_kv(true, j + 1);
+                load_kv(false, j);
             }
         }
-    } else if (warp == kMmaWarp) {
-        // ================= MMA issuer =================
+    } else if (warp == kMmaWarp || (!CONVK && warp == kMmaWarp + 1)) {
+        // ================= MMA issuers =================
+        // One thread issues the score products, another, of the next warp, the value products: each waits only for what its
+        // own products need, and what one does between two products does not hold up the other.  (Where two warps convert K
+        // tiles, one thread does both, in the order S_0(j+1) PV_0(j) S_1(j+1) PV_1(j).)
         if (elect_one()) {
-            bool ok = true;
+            int failed = 0;  // which wait gave up
             auto wait = [&](uint32_t bar, uint32_t parity, int where) {
-                if (!ok) return;
-                if (!mbar_wait(bar, parity, abort_flag)) {
-                    record_timeout(p, where);
-                    ok = false;
-                }
+                if (!mbar_wait(bar, parity, abort_flag)) failed = where;
             };
-            // The issue loops are unrolled (a rolled loop's dependent instructions cost 100+ cycles per MMA on this
-            // single thread, more than the tensor pipe needs), and each descriptor is the tile's base descriptor plus
-            // a compile-time constant, which keeps the thread inside its small register budget.
-            auto issue_s = [&](int w, int stage) {
-                const uint64_t b_desc = make_smem_desc(smem_u32(kv_s + stage * C::kTileBytes), 0, 1024);
-                const uint64_t a_desc = make_smem_desc(smem_u32(q_s + w * C::kTileBytes), 0, 1024);
+            const uint32_t q_desc = (uint32_t)make_smem_desc(smem_u32(q_s), 0, 1024);  // low words
+            const uint32_t k_desc = (uint32_t)make_smem_desc(smem_u32(k_s), 0, 1024);
+            const uint32_t v_desc = (uint32_t)make_smem_desc(smem_u32(v_s), C::kBoxBytes, 1024);
+            constexpr uint32_t kTile16 = C::kTileBytes >> 4;
+            TRACE_VARS;
+            uint32_t k_stage = 0, k_phase = 0, v_stage = 0, v_phase = 0;
+            // phase bits per slot or score tile of the barriers that are waited for once per use, flipped at each;
+            // s_used, o_used: the score tile (the slot's O) has been written before
+            uint32_t q_phase = 0, s_phase = 0, p_phase = 0, o_phase = 0, s_used = 0, o_used = 0;
+            // The issue sequences are unrolled (a rolled loop's dependent instructions cost 100+ cycles per MMA on a single
+            // thread, more than the tensor pipe needs); descriptors are the tile's plus a constant.
+            auto scores = [&](int w, int j, int n, bool last_reader) {
+                wait(CONVK ? k_ready(k_stage) : k_full(k_stage), k_phase, 240);
+                if (j == 0) {
+                    wait(p.rope_q_table ? q_ready(w) : q_full(w), (q_phase >> w) & 1, 200 + w);
+                    q_phase ^= 1u << w;
+                }
+                const int buf = C::kSBufs == 2 ? w : 0;
+                if ((s_used >> buf) & 1) {
+                    wait(s_free(buf), (s_phase >> buf) & 1, 250 + w);
+                    s_phase ^= 1u << buf;
+                }
+                s_used |= 1u << buf;
+                if (failed) return;
+                TRACE_MMA(w * 4 + 3);
+                tc_fence_after();
 #pragma unroll
                 for (int kk = 0; kk < D / 16; ++kk) {
                     const uint32_t off16 = (kk >> 2) * (C::kBoxBytes >> 4) + (kk & 3) * 2;  // byte offset / 16
-                    mma_ss_off(tmem_base + col_s[w], a_desc, b_desc, off16, p.idesc_qk, kk > 0);
+                    mma_ss_lo(tmem_base + col_s(w), q_desc + w * kTile16, k_desc + k_stage * kTile16, off16, p.idesc_qk, kk > 0);
+                }
+                tc_commit(s_full(w));
+                TRACE_MMA(w * 4 + 0);
+                if (j + 1 == n) tc_commit(q_empty(w));  // the slot's last S of this item
+                if (last_reader) {
+                    tc_commit(k_empty(k_stage));
+                    if (++k_stage == C::kStages) {
+                        k_stage = 0;
+                        k_phase ^= 1;
+                    }
                 }
             };
-            auto issue_pv = [&](int w, int stage, int j, int first, int last) {  // 16-key steps [first, last)
-                const uint64_t b_desc = make_smem_desc(smem_u32(kv_s + stage * C::kTileBytes), C::kBoxBytes, 1024);
+            auto values = [&](int w, int j, int n, bool last_reader) {
+                wait(v_full(v_stage), v_phase, 220);
+                if (j == 0) {
+                    if ((o_used >> w) & 1) {
+                        wait(o_free(w), (o_phase >> w) & 1, 260 + w);
+                        o_phase ^= 1u << w;
+                    }
+                    o_used |= 1u << w;
+                }
+                wait(p_full(w), (p_phase >> w) & 1, 230 + w);
+                p_phase ^= 1u << w;
+                if (failed) return;
+                TRACE_MMA(w * 4 + 1);
+                tc_fence_after();
 #pragma unroll
-                for (int kk = first; kk < last; ++kk)
-                    mma_ts_off(tmem_base + col_o[w], tmem_base + col_s[w] + kk * 8, b_desc, kk * (16 * 128 >> 4), p.idesc_pv,
-                               (j > 0 || kk > 0));
+                for (int kk = 0; kk < kTileRows / 16; ++kk)
+                    mma_ts_lo(tmem_base + col_o(w), tmem_base + col_p(w) + kk * 8, v_desc + v_stage * kTile16, kk * (16 * 128 >> 4),
+                              p.idesc_pv, j > 0 || kk > 0);
+                tc_commit(pv_done(w));
+                TRACE_MMA(w * 4 + 2);
+                if (j + 1 == n) tc_commit(o_final(w));
+                if (last_reader) {
+                    tc_commit(v_empty(v_stage));
+                    if (++v_stage == C::kStages) {
+                        v_stage = 0;
+                        v_phase ^= 1;
+                    }
+                }
             };
-            uint32_t ring0 = 0;           // ring entry of K_0 of the current item
-            uint32_t q_uses[2] = {0, 0};  // Q tiles consumed so far, per slot
-            uint32_t p_waits[2] = {0, 0}; // P hand-overs consumed so far, per slot
-            auto stage_of = [&](uint32_t i) { return (int)((ring0 + i) % C::kStages); };
-            auto phase_of = [&](uint32_t i) { return (uint32_t)(((ring0 + i) / C::kStages) & 1); };
-
-            for (int k = 0; ok; ++k) {
-                const int lin = item_index(p, k);
-                if (lin < 0) break;
-                const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
-                const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
-                const bool trace_item = k == FLAT_TRACE_ITEM;
-                (void)trace_item;
-                TRACEB(k, 2, 0);
-                // prologue: S_w(0) as soon as the slot's Q tile is ready (the other slot may still be finishing the
-                // previous item)
-                bool k0_ready = false;
-                for (int w = 0; w < 2 && ok; ++w) {
-                    if (it.n_tiles[w] == 0) continue;
-                    wait(p.rope_q_table ? q_ready(w) : q_full(w), q_uses[w] & 1, 200 + w);
-                    ++q_uses[w];
-                    TRACEB(k, 2, 1 + w);
-                    if (!k0_ready) {
-                        wait(CONVK ? k_ready(stage_of(0)) : kv_full(stage_of(0)), phase_of(0), 210);
-                        k0_ready = true;
-                    }
-                    if (!ok) break;
-                    tc_fence_after();
-                    issue_s(w, stage_of(0));
-                    tc_commit(s_full(w));
-                    if (it.n_tiles[w] == 1) tc_commit(q_empty(w));  // the slot's last S of this item
-                }
-                // (an item past its sequence's live rows has no KV tile and takes no ring entry: nothing is released)
-                if (ok && n_max > 0) {
-                    tc_commit(kv_empty(stage_of(0)));
-                    TRACEB(k, 2, 3);
-                }
-                for (int j = 0; ok && j < n_max; ++j) {
-                    const uint32_t iv = 2 * j + 1, ik = 2 * j + 2;
-                    wait(kv_full(stage_of(iv)), phase_of(iv), 220);
-                    bool k_next = false;
-                    for (int w = 0; w < 2 && ok; ++w) {
-                        if (j >= it.n_tiles[w]) continue;
-                        if constexpr (kEarlyKeys > 0) {
-                            wait(p_part(w), p_waits[w] & 1, 235 + w);
-                            if (!ok) break;
-                            tc_fence_after();
-                            issue_pv(w, stage_of(iv), j, 0, kEarlyKeys / 16);
+            if constexpr (!CONVK) {
+                for (int k = 0; !failed; ++k) {
+                    const int lin = item_index(p, k);
+                    if (lin < 0) break;
+                    const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
+                    const int n0 = it.n_tiles[0], n1 = it.n_tiles[1], n = max(n0, n1);
+                    if (warp == kMmaWarp) {
+                        for (int j = 0; j < n && !failed; ++j) {
+                            TRACE_STEP(k, j);
+                            if (j < n0) scores(0, j, n0, j >= n1);
+                            if (j < n1) scores(1, j, n1, true);
                         }
-                        wait(p_full(w), p_waits[w] & 1, 230 + w);
-                        if (!ok) break;
-                        ++p_waits[w];
-                        TRACE(2, j, w * 4 + 0);
-                        tc_fence_after();
-                        issue_pv(w, stage_of(iv), j, kEarlyKeys / 16, kTileRows / 16);
-                        TRACE(2, j, w * 4 + 1);
-                        if (w == 1 || j >= it.n_tiles[1]) tc_commit(kv_empty(stage_of(iv)));  // last reader of V_j
-                        if (j + 1 < it.n_tiles[w]) {
-                            if (!k_next) {
-                                wait(CONVK ? k_ready(stage_of(ik)) : kv_full(stage_of(ik)), phase_of(ik), 240);
-                                if (!ok) break;
-                                tc_fence_after();
-                                k_next = true;
-                            }
-                            issue_s(w, stage_of(ik));
-                            tc_commit(s_full(w));
-                            if (j + 2 == it.n_tiles[w]) tc_commit(q_empty(w));  // the slot's last S of this item
-                            TRACE(2, j, w * 4 + 2);
-                            if (w == 1 || j + 1 >= it.n_tiles[1]) tc_commit(kv_empty(stage_of(ik)));  // last reader of K_{j+1}
+                    } else {
+                        for (int j = 0; j < n && !failed; ++j) {
+                            TRACE_STEP(k, j);
+                            if (j < n0) values(0, j, n0, j >= n1);
+                            if (j < n1) values(1, j, n1, true);
+                        }
+                    }
+                }
+            } else {
+                // a step is one KV tile of an item, taken by both slots; sj: the step whose scores come next
+                int k_item = -1, sj = 0, sn0 = 0, sn1 = 0, sn = 0;
+                bool live = true;
+                do {
+                    const int pj = sj, pn0 = sn0, pn1 = sn1;  // the step whose value products come now
+                    TRACE_STEP(k_item, pj);
+                    ++sj;
+                    while (live && sj >= sn) {
+                        const int lin = item_index(p, ++k_item);
+                        live = lin >= 0;
+                        if (!live) break;
+                        const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
+                        sn0 = it.n_tiles[0];
+                        sn1 = it.n_tiles[1];
+                        sn = max(sn0, sn1);  // (0: an item past its sequence's live rows)
+                        sj = 0;
+                    }
+                    // the first scores of an item wait for a Q tile: the values go before them
+                    const int values_first = live && sj == 0 ? 1 : 0;
+#pragma unroll 1
+                    for (int op = 0; op < 4 && !failed; ++op) {
+                        const int w = op >> 1;
+                        if ((op ^ values_first) & 1) {
+                            const int n = w ? pn1 : pn0;
+                            if (pj < n) values(w, pj, n, w == 1 || pj >= pn1);
                         } else {
-                            tc_commit(o_final(w));
+                            const int n = w ? sn1 : sn0;
+                            if (live && sj < n) scores(w, sj, n, w == 1 || sj >= sn1);
                         }
                     }
-                }
-                ring0 += 2 * n_max;
+                } while (live && !failed);
             }
+            if (failed) record_timeout(p, failed);
         }
     } else if (CONVK) {
-        // ================= K converters (warps 10, 11) =================
+        // ================= K converters (the last two warps) =================
         // Each K tile of the ring is rewritten in place from bf16 to fp16 (the values are bf16 numbers, so the
-        // conversion is exact inside the normal fp16 range and saturates beyond it); warp 10 takes rows 0-63,
-        // warp 11 rows 64-127.  K tiles sit at the even ring entries.
+        // conversion is exact inside the normal fp16 range and saturates beyond it); one warp takes rows 0-63, the other
+        // rows 64-127.
         const int cw = warp - (kMmaWarp + 1);
         bool ok = true;
         uint32_t ring = 0;
@@ -585,14 +725,14 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             if (lin < 0) break;
             const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
             const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
-            for (int j = 0; ok && j < n_max; ++j, ring += 2) {
+            for (int j = 0; ok && j < n_max; ++j, ++ring) {
                 const int s = ring % C::kStages;
-                if (!mbar_wait(kv_full(s), (ring / C::kStages) & 1, abort_flag)) {
+                if (!mbar_wait(k_full(s), (ring / C::kStages) & 1, abort_flag)) {
                     record_timeout(p, 400 + s);
                     ok = false;
                     break;
                 }
-                uint8_t *tile = kv_s + s * C::kTileBytes;
+                uint8_t *tile = k_s + s * C::kTileBytes;
                 // a warp covers 64 rows x (D / 8) 16-byte chunks; consecutive lanes take consecutive chunks of a row
                 constexpr int kChunks = 64 * (D / 8);
 #pragma unroll 4
@@ -614,404 +754,375 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             }
         }
     }
+    } else if (warp >= kStoreWarp) {
+        // ================= Q rotation, O store =================
+        // These four warps take from the softmax warps what an item needs at its ends: the Q tiles of the next item are
+        // rotated and the O tiles of the finished one stored while both slots work on.  (The very first Q tile of a slot is
+        // rotated by its softmax warps, which have nothing else to do yet.)
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsStore));
+        const int lane_base = (warp & 3) * 32;
+        const int row_in_tile = lane_base + lane;
+        uint8_t *stg = o_stage + lane_base * 128;  // this warp's 32 rows
+        bool ok = true;
+        uint32_t phases = 0;           // bit w: parity of the slot's next Q tile, bit 2 + w: ... of its next finished item
+        uint32_t rotated = 0;          // bit w: the slot has had a Q tile
+        bool store_pending = false;    // (lane 0) a bulk store of the staging rows has not been waited for
+        auto staging_free = [&]() {
+            if (lane == 0 && store_pending) {
+                bulk_wait_group_read0();
+                store_pending = false;
+            }
+            __syncwarp();
+        };
+        auto send_box = [&](const WorkItem &it, int w, int hf) {  // (rows past q_len are clipped by the tensor map)
+            if (lane == 0 && it.r0 + w * kTileRows + lane_base < p.q_len) {
+                tma_store_4d(&p.map_o, hf * 64, it.r0 + w * kTileRows + lane_base, it.h, it.b, smem_u32(stg));
+                bulk_commit_group();
+                store_pending = true;
+            }
+        };
+        for (int k = -1; ok; ++k) {
+            const int next_lin = item_index(p, k + 1);
+#pragma unroll 1
+            for (int w = 0; w < 2 && ok; ++w) {
+                if (p.rope_q_table && next_lin >= 0) {
+                    const WorkItem nx = make_item<SPLIT, VARLEN>(p, next_lin, split_rec);
+                    if ((w ? nx.n_tiles[1] : nx.n_tiles[0]) > 0) {
+                        if ((rotated >> w) & 1) {
+                            // The tile before has been rotated: only then does the parity of q_full tell this tile's arrival
+                            // (the first one is the softmax warps', and may be gone by the time these look).
+                            const uint32_t parity = (phases >> w) & 1;
+                            if (!mbar_wait(q_ready(w), parity ^ 1, abort_flag) || !mbar_wait(q_full(w), parity, abort_flag)) {
+                                record_timeout(p, 290 + w);
+                                ok = false;
+                            }
+                            if (ok) rotate_q_tile<D, F16IO>(p, nx, w, q_s + w * C::kTileBytes, lane_base, lane);
+                            fence_proxy_async();  // generic-proxy writes -> visible to the tensor core's async proxy
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(q_ready(w));
+                        }
+                        rotated |= 1u << w;
+                        phases ^= 1u << w;
+                    }
+                }
+                if (k < 0 || !ok) continue;
+                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
+                const int row = it.r0 + w * kTileRows + row_in_tile;
+                const bool run = (w ? it.n_tiles[1] : it.n_tiles[0]) > 0;
+                if (run) {
+                    const uint32_t parity = (phases >> (2 + w)) & 1;
+                    const bool got = mbar_wait(ml_full(w), parity, abort_flag) && mbar_wait(o_final(w), parity, abort_flag);
+                    if (!got) {
+                        record_timeout(p, 310 + w);
+                        ok = false;
+                    }
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    phases ^= 4u << w;
+                    tc_fence_after();
+                    const float2 ml = ml_s[w * kTileRows + row_in_tile];
+                    const float m = ml.x, l = ml.y;
+                    const uint32_t t_o = tmem_base + (static_cast<uint32_t>(lane_base) << 16) + col_o(w);
+                    if (SPLIT && it.part_slot >= 0) {
+                        // a part of a split item: unnormalised O, running max and sum go to the partial record
+                        const long long prow = (long long)it.part_slot * (2 * kTileRows) + w * kTileRows + row_in_tile;
+                        float4 *po = reinterpret_cast<float4 *>(p.part_o + prow * D);
+                        uint32_t r[32];
+#pragma unroll 1
+                        for (int c = 0; c < D / 32; ++c) {
+                            tmem_ld32(t_o + c * 32, r);
+                            tc_wait_ld();
+#pragma unroll
+                            for (int q4 = 0; q4 < 8; ++q4)
+                                po[c * 8 + q4] = make_float4(__uint_as_float(r[q4 * 4]), __uint_as_float(r[q4 * 4 + 1]),
+                                                             __uint_as_float(r[q4 * 4 + 2]), __uint_as_float(r[q4 * 4 + 3]));
+                        }
+                        p.part_ml[prow] = ml;
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(o_free(w));
+                    } else {
+                        // O leaves through shared memory: every thread writes its row's 128 bytes of a 64-column box in the
+                        // swizzled box layout and each warp sends its 32 rows with one bulk store (whole lines), instead of
+                        // 32-byte stores 256 bytes apart per thread
+                        const float inv = 1.0f / l;
+                        const bool live_row = !VARLEN || row < it.q_len;  // a padded row of a variable-length batch: O = 0
+#pragma unroll 1
+                        for (int c = 0; c < D / 32; ++c) {
+                            uint32_t r[32];
+                            tmem_ld32(t_o + c * 32, r);
+                            tc_wait_ld();
+                            if (c == D / 32 - 1) {  // O and (max, sum) have been read: the next item may overwrite them
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) mbar_arrive(o_free(w));
+                            }
+                            if ((c & 1) == 0) staging_free();
+#pragma unroll
+                            for (int q8 = 0; q8 < 4; ++q8) {
+                                uint32_t v[4];
+#pragma unroll
+                                for (int e = 0; e < 4; ++e) {
+                                    const float x = __uint_as_float(r[q8 * 8 + 2 * e]) * inv, y = __uint_as_float(r[q8 * 8 + 2 * e + 1]) * inv;
+                                    if constexpr (F16IO) {
+                                        const __half2 h2 = __floats2half2_rn(x, y);
+                                        v[e] = *reinterpret_cast<const uint32_t *>(&h2);
+                                    } else {
+                                        const __nv_bfloat162 h2 = __floats2bfloat162_rn(x, y);
+                                        v[e] = *reinterpret_cast<const uint32_t *>(&h2);
+                                    }
+                                    if (VARLEN && !live_row) v[e] = 0;
+                                }
+                                *reinterpret_cast<uint4 *>(stg + lane * 128 + (((((c & 1) << 2) + q8) ^ (lane & 7)) << 4)) =
+                                    make_uint4(v[0], v[1], v[2], v[3]);
+                            }
+                            if (c & 1) {
+                                fence_proxy_async();  // generic-proxy writes -> visible to the bulk copy's async proxy
+                                __syncwarp();
+                                send_box(it, w, c >> 1);
+                            }
+                        }
+                        if (row < p.q_len)
+                            p.lse[((long long)it.b * p.q_heads + it.h) * p.lse_hs + row] = live_row ? (m + log2f(l)) * kLn2 : -INFINITY;
+                    }
+                } else if (SPLIT && it.part_slot >= 0) {
+                    // a part in which this Q tile has no KV tile at all still owns a partial record: an empty one
+                    p.part_ml[(long long)it.part_slot * (2 * kTileRows) + w * kTileRows + row_in_tile] = make_float2(-INFINITY, 0.f);
+                } else if (VARLEN) {
+                    // a tile past its sequence's live rows: O = 0, LSE = -inf (src/asymmetric_grouped.rs:103-104)
+                    staging_free();
+#pragma unroll
+                    for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<uint4 *>(stg + lane * 128 + (ch << 4)) = make_uint4(0, 0, 0, 0);
+                    fence_proxy_async();
+                    __syncwarp();
+                    for (int hf = 0; hf < D / 64; ++hf) send_box(it, w, hf);
+                    if (row < p.q_len) p.lse[((long long)it.b * p.q_heads + it.h) * p.lse_hs + row] = -INFINITY;
+                }
+            }
+            if (next_lin < 0) break;
+        }
+        if (lane == 0 && store_pending) bulk_wait_group_read0();  // the staging space must outlive the last store's read
     } else {
-        // ================= softmax + epilogue =================
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
+        // ================= softmax =================
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsSoftmax));
         const int w = warp >> 2;
         const int lane_base = (warp & 3) * 32;
         const int row_in_tile = lane_base + lane;
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(lane_base) << 16);
-        const uint32_t t_s = t_lane + col_s[w];
-        const uint32_t t_o = t_lane + col_o[w];
+        const uint32_t t_s = t_lane + col_s(w);
+        const uint32_t t_p = t_lane + col_p(w);
+        const uint32_t t_o = t_lane + col_o(w);
+        const int buf = C::kSBufs == 2 ? w : 0;
         bool ok = true;
-        uint32_t done = 0;     // finished items of this slot (its tile was inside q_len)
-        uint32_t s_waits = 0;  // score tiles of this slot consumed so far
-        bool store_pending = false;  // (lane 0) a bulk store of this warp's staging rows has not been waited for
+        uint32_t done = 0;   // finished items of this slot (its tile was inside q_len)
+        uint32_t tiles = 0;  // score tiles of this slot consumed so far
 
-        // Iteration k runs the KV loop of item k, then rotates the Q tile of item k + 1 (its TMA was issued as soon as
-        // the slot's last S MMA had completed), then stores item k: the next item's first S MMA runs during the
-        // epilogue.  k = -1 only rotates the first tile.
-        for (int k = -1; ok; ++k) {
-            // (item indices are recomputed where they are needed rather than kept in registers across the KV loop)
+        for (int k = 0; ok; ++k) {
+            const int lin = item_index(p, k);
+            if (lin < 0) break;
             const bool trace_item = k == FLAT_TRACE_ITEM;
             (void)trace_item;
+            const WorkItem it = make_item<SPLIT, VARLEN>(p, lin, split_rec);
+            const int n = w ? it.n_tiles[1] : it.n_tiles[0];
+            if (n <= 0) continue;
+            if (done == 0 && p.rope_q_table) {  // the slot's first Q tile
+                if (!mbar_wait(q_full(w), 0, abort_flag)) {
+                    record_timeout(p, 280 + w);
+                    ok = false;
+                } else {
+                    rotate_q_tile<D, F16IO>(p, it, w, q_s + w * C::kTileBytes, lane_base, lane);
+                }
+                fence_proxy_async();  // generic-proxy writes -> visible to the tensor core's async proxy
+                __syncwarp();
+                if (lane == 0) mbar_arrive(q_ready(w));
+            }
             float m = -INFINITY, l = 0.f;
-            bool run = false;
-            if (k >= 0) {
-                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
-                run = it.n_tiles[w] > 0;
-                const int n = it.n_tiles[w];
-                int lim = it.kv_len - 1;  // last visible key of this row
-                int lim_first = lim;     // ... and of the tile's first row: tiles below it need no mask at all
-                if (p.causal) {
-                    const int first = it.r0 + w * kTileRows;
-                    lim = (int)min((long long)lim, it.causal_off + first + row_in_tile);
-                    lim_first = (int)min((long long)lim_first, it.causal_off + first);
-                }
-                // keys are counted from the item's first KV tile below (a part of a split item starts at tile j0)
-                lim -= it.j0 * kTileRows;
-                lim_first -= it.j0 * kTileRows;
-                // ALiBi is added to the raw score as (slope / scale) * position difference, so that the scaling of the
-                // softmax passes covers it.  Positions stay below 2^24 in magnitude (checked on the host): the float
-                // position arithmetic is exact.
-                float slope_rel = 0.f, bias_pos0 = 0.f;
-                if constexpr (ALIBI) {
-                    slope_rel = (p.alibi_slopes ? __ldg(p.alibi_slopes + it.h) : p.alibi_inline[it.h]) * p.alibi_inv_scale;
-                    bias_pos0 = (float)(p.alibi_delta + it.j0 * kTileRows - (it.r0 + w * kTileRows + row_in_tile));
-                }
+            int lim = it.kv_len - 1;  // last visible key of this row
+            int lim_first = lim;     // ... and of the tile's first row: tiles below it need no mask at all
+            if (p.causal) {
+                const int first = it.r0 + w * kTileRows;
+                lim = min(lim, it.causal_off + first + row_in_tile);
+                lim_first = min(lim_first, it.causal_off + first);
+            }
+            // keys are counted from the item's first KV tile below (a part of a split item starts at tile j0)
+            lim -= it.j0 * kTileRows;
+            lim_first -= it.j0 * kTileRows;
+            // ALiBi is added to the raw score as (slope / scale) * position difference, so that the scaling of the
+            // softmax passes covers it.  Positions stay below 2^24 in magnitude (checked on the host): the float
+            // position arithmetic is exact.
+            float slope_rel = 0.f, bias_pos0 = 0.f;
+            if constexpr (ALIBI) {
+                slope_rel = (p.alibi_slopes ? __ldg(p.alibi_slopes + it.h) : p.alibi_inline[it.h]) * p.alibi_inv_scale;
+                bias_pos0 = (float)(p.alibi_delta + it.j0 * kTileRows - (it.r0 + w * kTileRows + row_in_tile));
+            }
 
-                // Online softmax, log2 domain, one thread per row; the whole 128-column score row sits in
-                // registers.  O in TMEM is rescaled only when the running max grew by more than 2^8.
-                TRACE_LOCAL;
-                for (int j = 0; ok && j < n; ++j) {
-                    if (!mbar_wait(s_full(w), s_waits & 1, abort_flag)) {
-                        record_timeout(p, 300 + w);
-                        ok = false;
-                        break;
-                    }
-                    ++s_waits;
-                    tc_fence_after();
-                    if ((warp & 3) == 0 && lane == 0) {
-                        TRACE_FLUSH(w, j - 1);
-                        TRACE_STAMP(0);
-                    }
-                    const int key0 = j * kTileRows;
-                    const bool tile_masked = key0 + kTileRows - 1 > lim_first;  // uniform over the Q tile
-                    const int vis = min(kTileRows, lim - key0 + 1);             // visible columns of this row
-                    const float c_log2 = p.scale_log2;
-                    uint32_t r[128];  // four loads in flight, one wait
+            // Online softmax, log2 domain, one thread per row; the whole 128-column score row sits in
+            // registers.  O in TMEM is rescaled only when the running max grew by more than 2^8.
+            TRACE_LOCAL;
+            for (int j = 0; ok && j < n; ++j) {
+                if (!mbar_wait(s_full(w), tiles & 1, abort_flag)) {
+                    record_timeout(p, 300 + w);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                if (lane == 0) {
+                    TRACE_FLUSH(warp, j - 1);
+                    TRACE_STAMP(0);
+                }
+                const int key0 = j * kTileRows;
+                const bool tile_masked = key0 + kTileRows - 1 > lim_first;  // uniform over the Q tile
+                const int vis = min(kTileRows, lim - key0 + 1);             // visible columns of this row
+                const float c_log2 = p.scale_log2;
+                uint32_t r[128];  // four loads in flight, one wait
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, r + c * 32);
-                    tc_wait_ld();
-                    if ((warp & 3) == 0 && lane == 0) TRACE_STAMP(1);
-                    // ALiBi: the bias of column i is (slope / c) * i on top of a part that is the same for the whole tile
-                    // row (bias_base).  It is never added to the scores in a pass of its own: the exponent pass below
-                    // folds it into the addend of its FMA (a running pair that advances by two columns per step), and
-                    // the maximum is taken per 32-column chunk of raw scores plus the chunk's largest bias, which bounds
-                    // the true maximum from above by at most 31 columns' worth of slope (any reference point at or above
-                    // the maximum serves the online softmax: P only gets smaller, O and the row sum with it).
-                    float bias_base = 0.f;
-                    if constexpr (ALIBI) bias_base = slope_rel * (bias_pos0 + (float)key0);
-                    if (tile_masked) {
-#pragma unroll
-                        for (int i = 0; i < 128; ++i)
-                            if (i >= vis) r[i] = 0xff800000u;  // -inf: exp2 gives exactly 0
-                    }
-                    float mx = -INFINITY, mx1 = -INFINITY;  // two chains for instruction-level parallelism
-                    if constexpr (ALIBI) {
-#pragma unroll
-                        for (int c = 0; c < 4; ++c) {
-                            float a = -INFINITY, b = -INFINITY;
-#pragma unroll
-                            for (int i = 32 * c; i < 32 * c + 32; i += 4) {
-                                asm("max.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(__uint_as_float(r[i])), "f"(__uint_as_float(r[i + 1])));
-                                asm("max.f32 %0, %0, %1, %2;" : "+f"(b) : "f"(__uint_as_float(r[i + 2])), "f"(__uint_as_float(r[i + 3])));
-                            }
-                            // the chunk's largest bias sits at its last column for a positive slope, at its first otherwise
-                            const float edge = slope_rel >= 0.f ? (float)(32 * c + 31) : (float)(32 * c);
-                            mx = fmaxf(mx, fmaf(slope_rel, edge, fmaxf(a, b)));
-                        }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 128; i += 4) {
-                            asm("max.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(__uint_as_float(r[i])), "f"(__uint_as_float(r[i + 1])));
-                            asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(__uint_as_float(r[i + 2])), "f"(__uint_as_float(r[i + 3])));
-                        }
-                    }
-                    const float m_cand = fmaxf(m, (fmaxf(mx, mx1) + bias_base) * c_log2);
-                    const bool grow = (m_cand - m) > kRescaleThreshold;
-                    float alpha = 1.0f;
-                    if (grow) {
-                        alpha = ex2(m - m_cand);
-                        m = m_cand;
-                    }
-                    if (j > 0 && __any_sync(0xffffffffu, grow)) {
-                        uint32_t o[32];
-#pragma unroll
-                        for (int c = 0; c < D / 32; ++c) {
-                            tmem_ld32(t_o + c * 32, o);
-                            tc_wait_ld();
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-                            tmem_st32(t_o + c * 32, o);
-                        }
-                    }
-                    l *= alpha;
-                    if ((warp & 3) == 0 && lane == 0) TRACE_STAMP(2);
-                    // P = exp2(S*c - m) as bf16, written over S; two scores per packed f32x2 FMA
-                    uint64_t c2, nm2, sum2 = 0, sum3 = 0;
-                    // m is still -inf only while every key this row has met was masked (the first tile of a split
-                    // part may lie wholly behind the row's diagonal): all its scores are -inf and P must come out 0
-                    const float neg_m0 = m == -INFINITY ? 0.f : fmaf(bias_base, c_log2, -m);
-                    asm("mov.b64 %0, {%1, %1};" : "=l"(nm2) : "f"(neg_m0));
-                    asm("mov.b64 %0, {%1, %1};" : "=l"(c2) : "f"(c_log2));
-                    [[maybe_unused]] uint64_t step2 = 0;  // ALiBi: the addend's advance per pair of columns
-                    [[maybe_unused]] float cs = 0.f;
-                    if constexpr (ALIBI) {
-                        cs = slope_rel * c_log2;
-                        asm("mov.b64 %0, {%1, %1};" : "=l"(step2) : "f"(2.f * cs));
-                    }
+                for (int c = 0; c < 4; ++c) tmem_ld32(t_s + c * 32, r + c * 32);
+                tc_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_free(buf));  // the next scores may overwrite the tile
+                if (lane == 0) TRACE_STAMP(1);
+                // ALiBi: the bias of column i is (slope / c) * i on top of a part that is the same for the whole tile
+                // row (bias_base).  It is never added to the scores in a pass of its own: the exponent pass below
+                // folds it into the addend of its FMA (a running pair that advances by two columns per step), and
+                // the maximum is taken per 32-column chunk of raw scores plus the chunk's largest bias, which bounds
+                // the true maximum from above by at most 31 columns' worth of slope (any reference point at or above
+                // the maximum serves the online softmax: P only gets smaller, O and the row sum with it).
+                float bias_base = 0.f;
+                if constexpr (ALIBI) bias_base = slope_rel * (bias_pos0 + (float)key0);
+                if (tile_masked) {
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
-                        uint32_t pk[16];
-                        if constexpr (ALIBI) {
-                            // the addend of the chunk's first pair, exact; the running sum then covers 16 steps only
-                            const float a0 = fmaf(cs, (float)(32 * c), neg_m0), a1 = fmaf(cs, (float)(32 * c + 1), neg_m0);
-                            asm("mov.b64 %0, {%1, %2};" : "=l"(nm2) : "f"(a0), "f"(a1));
-                        }
+                        const int v = vis - 32 * c;
+                        const uint32_t seen = v >= 32 ? 0xffffffffu : v <= 0 ? 0u : (1u << v) - 1u;
 #pragma unroll
-                        for (int i = 0; i < 32; i += 2) {
-                            uint64_t s2, t2, p2;
-                            asm("mov.b64 %0, {%1, %2};" : "=l"(s2) : "r"(r[c * 32 + i]), "r"(r[c * 32 + i + 1]));
-                            asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t2) : "l"(s2), "l"(c2), "l"(nm2));
-                            if constexpr (ALIBI) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(nm2) : "l"(step2));
-                            float t0, t1;
-                            asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t2));
-                            float p0 = t0, p1 = t1;
-                            if (POLY && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
-                                ex2_poly(p0, p1);
-                            } else {
-                                p0 = ex2(t0);
-                                p1 = ex2(t1);
-                            }
-                            asm("mov.b64 %0, {%1, %2};" : "=l"(p2) : "f"(p0), "f"(p1));
-                            if (i & 2) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum3) : "l"(p2));
-                            else asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum2) : "l"(p2));
-                            if constexpr (F16IO) {
-                                __half2 h2 = __floats2half2_rn(p0, p1);
-                                pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                            } else {
-                                __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
-                                pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                            }
-                        }
-                        tmem_st16(t_s + c * 16, pk);
-                        if (kEarlyKeys > 0 && (c + 1) * 32 == kEarlyKeys) {
-                            tc_wait_st();
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) mbar_arrive(p_part(w));
-                        }
+                        for (int i = 0; i < 32; ++i)
+                            if (!((seen >> i) & 1)) r[32 * c + i] = 0xff800000u;  // -inf: exp2 gives exactly 0
                     }
-                    {
-                        float s0, s1, s2f, s3;
-                        asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(sum2));
-                        asm("mov.b64 {%0, %1}, %2;" : "=f"(s2f), "=f"(s3) : "l"(sum3));
-                        l += (s0 + s1) + (s2f + s3);
-                    }
-                    if ((warp & 3) == 0 && lane == 0) TRACE_STAMP(3);
-                    tc_wait_st();
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(p_full(w));
-                    if ((warp & 3) == 0 && lane == 0) TRACE_STAMP(4);
                 }
-                if ((warp & 3) == 0 && lane == 0) TRACE_FLUSH(w, n - 1);
-            }
-
-            if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 0);
-            const int next_lin = item_index(p, k + 1);
-            if (p.rope_q_table && next_lin >= 0 && ok) {
-                const WorkItem nx = make_item<SPLIT, VARLEN>(p, next_lin, split_rec);
-                if (nx.n_tiles[w] > 0) {
-                    // Rotate the Q tile in place (bf16 in, fp16 out).  A warp rotates its 32 rows; lane l
-                    // takes the 16-byte chunk (l mod CH) of row (step * RPS + l / CH), so that the (cos, sin) table is
-                    // read in contiguous row segments.
-                    constexpr int CH = D / 8;     // 16-byte chunks (8 elements, 4 pairs) per row
-                    constexpr int RPS = 32 / CH;  // rows per step of one warp
-                    const int ch = lane % CH;
-                    const int first_row = nx.r0 + w * kTileRows;
-                    // (cos, sin) of the lane's first row come from the table; each further step advances the angle by
-                    // RPS positions with the rotation (cos, sin)(RPS * inv_freq), which keeps the table traffic at two
-                    // 16-byte loads per thread.  The recurrence error (a few 1e-7 over CH steps) is far below the
-                    // rounding of the fp16 result.
-                    float cc[4], ss[4], cstep[4], sstep[4];
-                    {
-                        const int rr = nx.table_row0 + min(first_row + lane_base + lane / CH, nx.q_len - 1);
-                        const float4 *tp = reinterpret_cast<const float4 *>(p.rope_q_table + (long long)rr * (D / 2)) + 2 * ch;
-                        const float4 cs0 = __ldg(tp), cs1 = __ldg(tp + 1);  // (c, s, c, s) x 2
-                        cc[0] = cs0.x; ss[0] = cs0.y; cc[1] = cs0.z; ss[1] = cs0.w;
-                        cc[2] = cs1.x; ss[2] = cs1.y; cc[3] = cs1.z; ss[3] = cs1.w;
+                float mx = -INFINITY, mx1 = -INFINITY;  // two chains for instruction-level parallelism
+                if constexpr (ALIBI) {
 #pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float2 stp = p.rope_step[ch * 4 + e];
-                            cstep[e] = stp.x;
-                            sstep[e] = stp.y;
+                    for (int c = 0; c < 4; ++c) {
+                        float a = -INFINITY, b = -INFINITY;
+#pragma unroll
+                        for (int i = 32 * c; i < 32 * c + 32; i += 4) {
+                            asm("max.f32 %0, %0, %1, %2;" : "+f"(a) : "f"(__uint_as_float(r[i])), "f"(__uint_as_float(r[i + 1])));
+                            asm("max.f32 %0, %0, %1, %2;" : "+f"(b) : "f"(__uint_as_float(r[i + 2])), "f"(__uint_as_float(r[i + 3])));
                         }
+                        // the chunk's largest bias sits at its last column for a positive slope, at its first otherwise
+                        const float edge = slope_rel >= 0.f ? (float)(32 * c + 31) : (float)(32 * c);
+                        mx = fmaxf(mx, fmaf(slope_rel, edge, fmaxf(a, b)));
                     }
-                    // rotations before this one: the finished items plus the current one
-                    if (!mbar_wait(q_full(w), (done + (run ? 1u : 0u)) & 1, abort_flag)) {
-                        record_timeout(p, 290 + w);
-                        ok = false;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 128; i += 4) {
+                        asm("max.f32 %0, %0, %1, %2;" : "+f"(mx) : "f"(__uint_as_float(r[i])), "f"(__uint_as_float(r[i + 1])));
+                        asm("max.f32 %0, %0, %1, %2;" : "+f"(mx1) : "f"(__uint_as_float(r[i + 2])), "f"(__uint_as_float(r[i + 3])));
                     }
-                    if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 1);
-                    if (ok) {
-                        uint8_t *tile = q_s + w * C::kTileBytes;
-                        // all of the thread's chunks are fetched before any is written back: the loads are then in
-                        // flight together instead of each waiting behind the previous step's store
-                        uint4 raw[CH];
-#pragma unroll
-                        for (int st = 0; st < CH; ++st) {
-                            const int rt = lane_base + st * RPS + lane / CH;  // row in tile
-                            raw[st] = *reinterpret_cast<const uint4 *>(tile + (ch >> 3) * C::kBoxBytes + rt * 128 + (((ch & 7) ^ (rt & 7)) << 4));
-                        }
-#pragma unroll
-                        for (int st = 0; st < CH; ++st) {
-                            const int rt = lane_base + st * RPS + lane / CH;  // row in tile
-                            const int off = (ch >> 3) * C::kBoxBytes + rt * 128 + (((ch & 7) ^ (rt & 7)) << 4);
-                            if (st > 0) {
-#pragma unroll
-                                for (int e = 0; e < 4; ++e) {
-                                    const float c1 = cc[e] * cstep[e] - ss[e] * sstep[e];
-                                    ss[e] = ss[e] * cstep[e] + cc[e] * sstep[e];
-                                    cc[e] = c1;
-                                }
-                            }
-                            if (first_row + rt >= nx.q_len) continue;  // rows past q_len are not used
-                            const uint32_t in[4] = {raw[st].x, raw[st].y, raw[st].z, raw[st].w};
-                            uint32_t hi[4];
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                float x, y;
-                                if constexpr (F16IO) {
-                                    const float2 xy = __half22float2(*reinterpret_cast<const __half2 *>(&in[e]));
-                                    x = xy.x;
-                                    y = xy.y;
-                                } else {
-                                    x = __uint_as_float(in[e] << 16);
-                                    y = __uint_as_float(in[e] & 0xffff0000u);
-                                }
-                                const float rx = x * cc[e] - y * ss[e], ry = x * ss[e] + y * cc[e];
-                                const __half2 h2 = __floats2half2_rn(rx, ry);
-                                hi[e] = *reinterpret_cast<const uint32_t *>(&h2);
-                            }
-                            *reinterpret_cast<uint4 *>(tile + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        }
-                    }
-                    fence_proxy_async();  // generic-proxy writes -> visible to the tensor core's async proxy
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(q_ready(w));
-                    if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 2);
                 }
-            }
-
-            if (run && ok) {
-                if (!mbar_wait(o_final(w), done & 1, abort_flag)) {
-                    record_timeout(p, 310 + w);
+                const float m_cand = fmaxf(m, (fmaxf(mx, mx1) + bias_base) * c_log2);
+                const bool grow = (m_cand - m) > kRescaleThreshold;
+                float alpha = 1.0f;
+                if (grow) {
+                    alpha = ex2(m - m_cand);
+                    m = m_cand;
+                }
+                // P and O belong to the slot's previous value product until it is done
+                if (tiles > 0 && !mbar_wait(pv_done(w), (tiles - 1) & 1, abort_flag)) {
+                    record_timeout(p, 320 + w);
                     ok = false;
                 }
-                ++done;
-            }
-            if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 3);
-            if (run && ok) {
+                ++tiles;
                 tc_fence_after();
-                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
-                const int row = it.r0 + w * kTileRows + row_in_tile, b = it.b, h = it.h;
-                if (SPLIT && it.part_slot >= 0) {
-                    // a part of a split item: unnormalised O, running max and sum go to the partial record
-                    const long long prow = (long long)it.part_slot * (2 * kTileRows) + w * kTileRows + row_in_tile;
-                    float4 *po = reinterpret_cast<float4 *>(p.part_o + prow * D);
-                    uint32_t r[32];
-#pragma unroll
-                    for (int c = 0; c < D / 32; ++c) {
-                        tmem_ld32(t_o + c * 32, r);
+                if (j > 0 && __any_sync(0xffffffffu, grow)) {
+#pragma unroll 1
+                    for (int c = 0; c < D; c += 16) {  // (few columns at a time: the scores occupy the registers)
+                        uint32_t o[16];
+                        tmem_ld16(t_o + c, o);
                         tc_wait_ld();
 #pragma unroll
-                        for (int q4 = 0; q4 < 8; ++q4)
-                            po[c * 8 + q4] = make_float4(__uint_as_float(r[q4 * 4]), __uint_as_float(r[q4 * 4 + 1]),
-                                                         __uint_as_float(r[q4 * 4 + 2]), __uint_as_float(r[q4 * 4 + 3]));
+                        for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+                        tmem_st16(t_o + c, o);
                     }
-                    p.part_ml[prow] = make_float2(m, l);
-                    tc_fence_before();
-                } else {
-                    // O leaves through shared memory: every thread writes its row's 128 bytes of a 64-column box in the
-                    // swizzled box layout and each warp sends its 32 rows with one bulk store (whole lines), instead of
-                    // 32-byte stores 256 bytes apart per thread
-                    const float inv = 1.0f / l;
-                    uint8_t *stg = o_stage + w * C::kOutStageBytes;
-                    uint32_t ro[D];  // the whole row of O: all loads in flight, one wait
+                }
+                l *= alpha;
+                if (lane == 0) TRACE_STAMP(2);
+                // P = exp2(S*c - m) in 16 bits; two scores per packed f32x2 FMA
+                uint64_t c2, nm2, sum2 = 0, sum3 = 0;
+                // m is still -inf only while every key this row has met was masked (the first tile of a split
+                // part may lie wholly behind the row's diagonal): all its scores are -inf and P must come out 0
+                const float neg_m0 = m == -INFINITY ? 0.f : fmaf(bias_base, c_log2, -m);
+                asm("mov.b64 %0, {%1, %1};" : "=l"(nm2) : "f"(neg_m0));
+                asm("mov.b64 %0, {%1, %1};" : "=l"(c2) : "f"(c_log2));
+                [[maybe_unused]] uint64_t step2 = 0;  // ALiBi: the addend's advance per pair of columns
+                [[maybe_unused]] float cs = 0.f;
+                if constexpr (ALIBI) {
+                    cs = slope_rel * c_log2;
+                    asm("mov.b64 %0, {%1, %1};" : "=l"(step2) : "f"(2.f * cs));
+                }
 #pragma unroll
-                    for (int c = 0; c < D / 32; ++c) tmem_ld32(t_o + c * 32, ro + c * 32);
-                    tc_wait_ld();
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t pk[16];
+                    if constexpr (ALIBI) {
+                        // the addend of the chunk's first pair, exact; the running sum then covers 16 steps only
+                        const float a0 = fmaf(cs, (float)(32 * c), neg_m0), a1 = fmaf(cs, (float)(32 * c + 1), neg_m0);
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(nm2) : "f"(a0), "f"(a1));
+                    }
 #pragma unroll
-                    for (int hf = 0; hf < D / 64; ++hf) {
-                        const uint32_t *r = ro + hf * 64;
-                        uint32_t pk[32];
-#pragma unroll
-                        for (int i = 0; i < 64; i += 2) {
-                            if constexpr (F16IO) {
-                                __half2 h2 = __floats2half2_rn(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
-                                pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                            } else {
-                                __nv_bfloat162 h2 =
-                                    __floats2bfloat162_rn(__uint_as_float(r[i]) * inv, __uint_as_float(r[i + 1]) * inv);
-                                pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
-                            }
+                    for (int i = 0; i < 32; i += 2) {
+                        uint64_t s2, t2, p2;
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(s2) : "r"(r[c * 32 + i]), "r"(r[c * 32 + i + 1]));
+                        asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(t2) : "l"(s2), "l"(c2), "l"(nm2));
+                        if constexpr (ALIBI) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(nm2) : "l"(step2));
+                        float t0, t1;
+                        asm("mov.b64 {%0, %1}, %2;" : "=f"(t0), "=f"(t1) : "l"(t2));
+                        float p0 = t0, p1 = t1;
+                        if (POLY && (i >> 1) % kPolyEvery == kPolyEvery - 1) {
+                            ex2_poly(p0, p1);
+                        } else {
+                            p0 = ex2(t0);
+                            p1 = ex2(t1);
                         }
-                        if (VARLEN && row >= it.q_len) {  // a padded row of a variable-length batch: O = 0
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) pk[i] = 0;
-                        }
-                        // A warp stages and sends its own 32 rows, so the four warps of the slot never wait for one
-                        // another here.  The staging rows are reused by the next box: the lane that sent the previous one
-                        // waits for that bulk store's read only now, after the next box has been fetched and converted
-                        // (or an item later), when it is long done.
-                        if (lane == 0 && store_pending) {
-                            bulk_wait_group_read0();
-                            store_pending = false;
-                        }
-                        __syncwarp();
-#pragma unroll
-                        for (int ch = 0; ch < 8; ++ch)
-                            *reinterpret_cast<uint4 *>(stg + row_in_tile * 128 + ((ch ^ (row_in_tile & 7)) << 4)) =
-                                make_uint4(pk[ch * 4], pk[ch * 4 + 1], pk[ch * 4 + 2], pk[ch * 4 + 3]);
-                        fence_proxy_async();  // generic-proxy writes -> visible to the bulk copy's async proxy
-                        __syncwarp();
-                        // (rows past q_len are clipped by the tensor map; a box that starts past it is not sent at all)
-                        if (lane == 0 && it.r0 + w * kTileRows + lane_base < p.q_len) {
-                            tma_store_4d(&p.map_o, hf * 64, it.r0 + w * kTileRows + lane_base, h, b, smem_u32(stg + lane_base * 128));
-                            bulk_commit_group();
-                            store_pending = true;
+                        asm("mov.b64 %0, {%1, %2};" : "=l"(p2) : "f"(p0), "f"(p1));
+                        if (i & 2) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum3) : "l"(p2));
+                        else asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum2) : "l"(p2));
+                        if constexpr (F16IO) {
+                            __half2 h2 = __floats2half2_rn(p0, p1);
+                            pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
+                        } else {
+                            __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
+                            pk[i >> 1] = *reinterpret_cast<uint32_t *>(&h2);
                         }
                     }
-                    if (row < p.q_len)
-                        p.lse[((long long)b * p.q_heads + h) * p.lse_hs + row] = VARLEN && row >= it.q_len ? -INFINITY : (m + log2f(l)) * kLn2;
-                    // the O columns are overwritten by the next item's first PV MMA, which is issued only after this
-                    // thread's next hand-over of P: program order keeps the reads above ahead of it
-                    tc_fence_before();
+                    tmem_st16(t_p + c * 16, pk);
                 }
-            } else if (SPLIT && k >= 0 && ok) {
-                // a part in which this Q tile has no KV tile at all still owns a partial record: an empty one
-                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
-                if (it.part_slot >= 0)
-                    p.part_ml[(long long)it.part_slot * (2 * kTileRows) + w * kTileRows + row_in_tile] = make_float2(-INFINITY, 0.f);
-            }
-            if (VARLEN && k >= 0 && !run && ok) {
-                // a tile past its sequence's live rows: O = 0, LSE = -inf (src/asymmetric_grouped.rs:103-104)
-                const WorkItem it = make_item<SPLIT, VARLEN>(p, item_index(p, k), split_rec);
-                const int row = it.r0 + w * kTileRows + row_in_tile;
-                uint8_t *stg = o_stage + w * C::kOutStageBytes;
-                if (lane == 0 && store_pending) {
-                    bulk_wait_group_read0();
-                    store_pending = false;
+                {
+                    float s0, s1, s2f, s3;
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(sum2));
+                    asm("mov.b64 {%0, %1}, %2;" : "=f"(s2f), "=f"(s3) : "l"(sum3));
+                    l += (s0 + s1) + (s2f + s3);
                 }
+                if (lane == 0) TRACE_STAMP(3);
+                tc_wait_st();
+                tc_fence_before();
                 __syncwarp();
-#pragma unroll
-                for (int ch = 0; ch < 8; ++ch) *reinterpret_cast<uint4 *>(stg + row_in_tile * 128 + (ch << 4)) = make_uint4(0, 0, 0, 0);
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0 && it.r0 + w * kTileRows + lane_base < p.q_len) {
-                    for (int hf = 0; hf < D / 64; ++hf)
-                        tma_store_4d(&p.map_o, hf * 64, it.r0 + w * kTileRows + lane_base, it.h, it.b, smem_u32(stg + lane_base * 128));
-                    bulk_commit_group();
-                    store_pending = true;
-                }
-                if (row < p.q_len) p.lse[((long long)it.b * p.q_heads + it.h) * p.lse_hs + row] = -INFINITY;
+                if (lane == 0) mbar_arrive(p_full(w));
+                if (lane == 0) TRACE_STAMP(4);
             }
-            if ((warp & 3) == 0 && lane == 0) TRACEB(k, w, 4);
-            if (next_lin < 0) break;
+            if (lane == 0) TRACE_FLUSH(warp, n - 1);
+            if (!ok) break;
+            // (max, sum) of the item's rows for the warps that store it, which have read those of the item before
+            if (done > 0 && !mbar_wait(o_free(w), (done - 1) & 1, abort_flag)) {
+                record_timeout(p, 330 + w);
+                ok = false;
+                break;
+            }
+            ++done;
+            ml_s[w * kTileRows + row_in_tile] = make_float2(m, l);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ml_full(w));
         }
-        if (store_pending) bulk_wait_group_read0();  // the staging space must outlive the last store's read
     }
 
     if (*abort_flag) {
@@ -1370,7 +1481,8 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     kp.div_heads = make_fastdiv(p.q_heads);
     kp.div_group = make_fastdiv(p.group);
     kp.causal = p.causal;
-    kp.causal_off = p.causal_off;
+    // 2^30 rows do not fit the device: an offset beyond hides nothing, and row + offset stays an int
+    kp.causal_off = (int)std::max<int64_t>(-(1 << 30), std::min<int64_t>(p.causal_off, 1 << 30));
     kp.scale_log2 = p.scale * kLog2e;
     kp.idesc_qk = make_idesc(q_f16 ? kFmtF16 : kFmtBF16, (k_f16 || convk || io16 || k_shadow) ? kFmtF16 : kFmtBF16, 0, 0, 128, 128);
     kp.idesc_pv = io16 ? make_idesc(kFmtF16, kFmtF16, 0, 1, 128, (uint32_t)D) : make_idesc(kFmtBF16, kFmtBF16, 0, 1, 128, (uint32_t)D);
@@ -1463,3 +1575,4 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
 }
 
 }  // namespace flat
+

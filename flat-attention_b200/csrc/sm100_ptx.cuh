@@ -85,14 +85,11 @@ constexpr uint32_t kSuspendNs = 20000;         // one suspended poll lasts at mo
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     if (mbar_try_wait(bar, parity)) return true;
     const uint32_t start = (uint32_t)clock();
-    for (;;) {
+    do {
         if (mbar_try_wait_suspend(bar, parity, kSuspendNs)) return true;
-        if (*abort_flag != 0) return false;
-        if ((uint32_t)clock() - start > kWaitCycles) {
-            *abort_flag = 1;
-            return false;
-        }
-    }
+    } while (*abort_flag == 0 && (uint32_t)clock() - start <= kWaitCycles);
+    *abort_flag = 1;
+    return false;
 }
 
 // ---- TMA -------------------------------------------------------------------------------------
@@ -193,6 +190,40 @@ __device__ __forceinline__ void mma_ts_off(uint32_t d_tmem, uint32_t a_tmem, uin
         : "memory");
 }
 
+// The same with the descriptors given by their low words (start address and leading byte offset; `kDescHi1024` is the high word
+// of a 128-byte-swizzled operand whose stride byte offset is 1024): half the registers and additions per instruction.
+constexpr uint32_t kDescHi1024 = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void mma_ss_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t off16, uint32_t idesc,
+                                          uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b32 la, lb;\n"
+        ".reg .b64 da, db;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "add.u32 la, %1, %5;\n"
+        "add.u32 lb, %2, %5;\n"
+        "mov.b64 da, {la, %6};\n"
+        "mov.b64 db, {lb, %6};\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n"
+        "}\n" ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(off16), "n"(kDescHi1024)
+        : "memory");
+}
+__device__ __forceinline__ void mma_ts_lo(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t off16, uint32_t idesc,
+                                          uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b32 lb;\n"
+        ".reg .b64 db;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "add.u32 lb, %2, %5;\n"
+        "mov.b64 db, {lb, %6};\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %3, p;\n"
+        "}\n" ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(off16), "n"(kDescHi1024)
+        : "memory");
+}
+
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp reads lane (lane_base + t).
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
     asm volatile(
@@ -203,6 +234,15 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t *r) {
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
           "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t *r) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
 }
