@@ -2,14 +2,14 @@
 //
 // Bound by the f32 FMA pipe (128 lanes per clock and SM; the tensor cores have no f32 mode of this precision), so both
 // products are laid out to feed it: a CTA owns 64 query rows of one (batch, q_head) and streams K/V tiles of 64 keys
-// through shared memory; 128 threads hold 4 rows x 8 keys of the scores and 4 rows x D/8 columns of O in registers, so
-// a 16-byte shared-memory read serves 10 to 13 multiply-adds (the row-per-four-threads kernel in fwd_simt.cu reads one
-// K and one V vector for four).  Products run as packed f32x2 FMAs: a score is two running sums (even and odd
-// dimensions) over each half of the head dimension, an O pair is two adjacent columns.
+// through shared memory; at D = 128 256 threads hold 4 rows x 4 keys of the scores and 4 rows x D/16 columns of O in
+// registers, at D = 64 128 threads twice that, so a 16-byte shared-memory read serves 8 to 13 multiply-adds (the
+// row-per-four-threads kernel in fwd_simt.cu reads one K and one V vector for four).  Products run as packed f32x2 FMAs: a
+// score is two running sums (even and odd dimensions) over each half of the head dimension, an O pair is two adjacent columns.
 // Few query blocks leave most SMs idle and the causal diagonal makes them uneven, so the KV tiles of a query block are
 // dealt to a cluster of up to 8 CTAs, which combine their (max, sum, O) through distributed shared memory in rank
 // order: one launch, no scratch, bitwise repeatable.  8 / 2 heads, 512 rows, D = 128, causal, RoPE: 219 us with the kernel of
-// fwd_simt.cu, 45 us here; 2 x 2048 rows, 16 / 4 heads 3470 us and 1180 us (29 TFLOP/s).
+// fwd_simt.cu, 44 us here; 2 x 2048 rows, 16 / 4 heads 3470 us and 1180 us (29 TFLOP/s).
 // RoPE: K and Q are rotated on the way into shared memory with the (cos, sin) table of the call's positions (find_tables());
 // without one the same sincosf runs here.
 #include <cooperative_groups.h>
@@ -26,9 +26,13 @@ namespace cg = cooperative_groups;
 
 constexpr int kRows = 64;    // query rows per CTA
 constexpr int kKeys = 64;    // keys per tile
-constexpr int kThreads = 128;
+// tx: lanes that share a row.  Twice the threads with half the tile each hide more of the shared-memory latency at D = 128 (8 / 2
+// heads: 356 rows 41.3 -> 37.0 us, 512 rows 45.1 -> 43.6, 2 x 2048 rows, 16 / 4 heads 1207 both); at D = 64 a read then serves too
+// few multiply-adds (1784 rows 164 -> 166 us, 2 x 2048 rows without a mask 1049 -> 1068).
+template <int D> constexpr int kLanes = D == 128 ? 16 : 8;
+template <int D> constexpr int kThreads = kRows / 4 * kLanes<D>;
 constexpr int kRowsPerThread = 4;   // ty + 16 r
-constexpr int kKeysPerThread = 8;   // tx + 8 i
+template <int D> constexpr int kKeysPerThread = kKeys / kLanes<D>;  // tx + kLanes i
 constexpr int kMaxCluster = 8;
 
 struct F32Params {
@@ -72,8 +76,8 @@ template <int D>
 __device__ __forceinline__ void load_rows(float *dst, int stride, const float *src, int64_t rs, int64_t first, int live) {
     constexpr int kVec = D / 4;
 #pragma unroll
-    for (int u = 0; u < 64 * kVec / kThreads; ++u) {
-        const int i = u * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+    for (int u = 0; u < 64 * kVec / kThreads<D>; ++u) {
+        const int i = u * kThreads<D> + threadIdx.x, r = i / kVec, v = i % kVec;
         cp_async16(dst + r * stride + 4 * v, src + (first + (r < live ? r : 0)) * rs + 4 * v, r < live);
     }
 }
@@ -83,8 +87,8 @@ __device__ __forceinline__ bool copied_non_finite(const float *src) {
     constexpr int kVec = D / 4;
     uint64_t zero[4] = {};
 #pragma unroll 2
-    for (int u = 0; u < 64 * kVec / kThreads; ++u) {
-        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(src + 4 * (u * kThreads + threadIdx.x));
+    for (int u = 0; u < 64 * kVec / kThreads<D>; ++u) {
+        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(src + 4 * (u * kThreads<D> + threadIdx.x));
         fma2(zero[2 * u & 3], x.x, 0);
         fma2(zero[2 * u + 1 & 3], x.y, 0);
     }
@@ -98,25 +102,25 @@ __device__ __forceinline__ bool copied_non_finite(const float *src) {
 template <int D>
 __device__ __forceinline__ void load_rotated_rows(float *dst, int stride, const float *src, int64_t rs, int64_t first, int live,
                                                   const float2 *table, int64_t pos0, const float *inv_freq) {
-    constexpr int kVec = D / 4, kBatch = 8;
+    constexpr int kVec = D / 4, kBatch = 64 * kVec / kThreads<D> < 8 ? 64 * kVec / kThreads<D> : 8;
 #pragma unroll
-    for (int u0 = 0; u0 < 64 * kVec / kThreads; u0 += kBatch) {
+    for (int u0 = 0; u0 < 64 * kVec / kThreads<D>; u0 += kBatch) {
         float4 x[kBatch], cs[kBatch];
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
-            const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+            const int i = (u0 + u) * kThreads<D> + threadIdx.x, r = i / kVec, v = i % kVec;
             x[u] = *reinterpret_cast<const float4 *>(src + (first + (r < live ? r : 0)) * rs + 4 * v);
         }
         if (table) {
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+                const int i = (u0 + u) * kThreads<D> + threadIdx.x, r = i / kVec, v = i % kVec;
                 cs[u] = *reinterpret_cast<const float4 *>(table + (first + (r < live ? r : 0)) * (D / 2) + 2 * v);
             }
         } else {
 #pragma unroll
             for (int u = 0; u < kBatch; ++u) {
-                const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+                const int i = (u0 + u) * kThreads<D> + threadIdx.x, r = i / kVec, v = i % kVec;
                 const float pos = (float)(pos0 + first + r);
                 sincosf(__fmul_rn(pos, inv_freq[2 * v]), &cs[u].y, &cs[u].x);
                 sincosf(__fmul_rn(pos, inv_freq[2 * v + 1]), &cs[u].w, &cs[u].z);
@@ -124,7 +128,7 @@ __device__ __forceinline__ void load_rotated_rows(float *dst, int stride, const 
         }
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
-            const int i = (u0 + u) * kThreads + threadIdx.x, r = i / kVec, v = i % kVec;
+            const int i = (u0 + u) * kThreads<D> + threadIdx.x, r = i / kVec, v = i % kVec;
             const float4 y = x[u], c = cs[u];
             *reinterpret_cast<float4 *>(dst + r * stride + 4 * v) =
                 r < live ? make_float4(y.x * c.x - y.y * c.y, y.x * c.y + y.y * c.x, y.z * c.z - y.w * c.w, y.z * c.w + y.w * c.z)
@@ -137,28 +141,29 @@ __device__ __forceinline__ void load_rotated_rows(float *dst, int stride, const 
 // its code beside the plain loop costs that one registers.
 template <int D>
 __device__ __noinline__ void accumulate_seen(uint64_t *o, const float *ps, const float *vs, int seen) {
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int tx = threadIdx.x % kLanes<D>, ty = threadIdx.x / kLanes<D>;
     for (int r = 0; r < kRowsPerThread; ++r)
         for (int k = 0; k < min(kKeys, seen + 16 * r); ++k) {
+            constexpr int kCols = D / (4 * kLanes<D>);
             const float x = ps[(ty + 16 * r) * Tile<D>::kPStride + k];
-            for (int c = 0; c < D / 32; ++c) {
-                const ulonglong2 vv = *reinterpret_cast<const ulonglong2 *>(vs + k * D + 4 * tx + 32 * c);
-                fma2(o[(r * (D / 32) + c) * 2], pack2(x, x), vv.x);
-                fma2(o[(r * (D / 32) + c) * 2 + 1], pack2(x, x), vv.y);
+            for (int c = 0; c < kCols; ++c) {
+                const ulonglong2 vv = *reinterpret_cast<const ulonglong2 *>(vs + k * D + 4 * tx + 4 * kLanes<D> * c);
+                fma2(o[(r * kCols + c) * 2], pack2(x, x), vv.x);
+                fma2(o[(r * kCols + c) * 2 + 1], pack2(x, x), vv.y);
             }
         }
 }
 
 template <int D, bool ALIBI>
-__global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_constant__ F32Params fp) {
+__global__ void __launch_bounds__(kThreads<D>, 2) fwd_f32_kernel(const __grid_constant__ F32Params fp) {
     using T = Tile<D>;
-    constexpr int kCols = D / 32;  // float4 columns of O per thread and row
+    constexpr int kCols = D / (4 * kLanes<D>);  // float4 columns of O per thread and row
     const FwdParams &p = fp.f;
     extern __shared__ __align__(16) float smem[];
     float *qs = smem + T::kQ, *ks = smem + T::kK, *vs = smem + T::kV, *stat = smem + T::kStat;
     float *ps = ks;
 
-    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int tx = threadIdx.x % kLanes<D>, ty = threadIdx.x / kLanes<D>;
     cg::cluster_group cluster = cg::this_cluster();
     const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
     const int q_blocks = (int)gridDim.x / parts;
@@ -203,14 +208,14 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
         __syncthreads();
 
         // S = Q K^T: two half products of D/2 dimensions, each as sums over even and over odd dimensions
-        float s[kRowsPerThread][kKeysPerThread];
+        float s[kRowsPerThread][kKeysPerThread<D>];
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
-            uint64_t acc[kRowsPerThread][kKeysPerThread];
+            uint64_t acc[kRowsPerThread][kKeysPerThread<D>];
 #pragma unroll
             for (int r = 0; r < kRowsPerThread; ++r)
 #pragma unroll
-                for (int i = 0; i < kKeysPerThread; ++i) acc[r][i] = 0;
+                for (int i = 0; i < kKeysPerThread<D>; ++i) acc[r][i] = 0;
             const float *qp = qs + ty * T::kStride + half * (D / 2), *kp = ks + tx * T::kStride + half * (D / 2);
 #pragma unroll 2
             for (int d = 0; d < D / 2; d += 4) {
@@ -218,8 +223,8 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
 #pragma unroll
                 for (int r = 0; r < kRowsPerThread; ++r) qv[r] = *reinterpret_cast<const ulonglong2 *>(qp + 16 * r * T::kStride + d);
 #pragma unroll
-                for (int i = 0; i < kKeysPerThread; ++i) {
-                    const ulonglong2 kv = *reinterpret_cast<const ulonglong2 *>(kp + 8 * i * T::kStride + d);
+                for (int i = 0; i < kKeysPerThread<D>; ++i) {
+                    const ulonglong2 kv = *reinterpret_cast<const ulonglong2 *>(kp + kLanes<D> * i * T::kStride + d);
 #pragma unroll
                     for (int r = 0; r < kRowsPerThread; ++r) {
                         fma2(acc[r][i], qv[r].x, kv.x);
@@ -230,7 +235,7 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
 #pragma unroll
             for (int r = 0; r < kRowsPerThread; ++r)
 #pragma unroll
-                for (int i = 0; i < kKeysPerThread; ++i) {
+                for (int i = 0; i < kKeysPerThread<D>; ++i) {
                     const float2 e = unpack2(acc[r][i]);
                     s[r][i] = half ? s[r][i] + (e.x + e.y) : e.x + e.y;
                 }
@@ -248,24 +253,24 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
             // src/attention_bias.rs:93-94
             const int64_t bias0 = ALIBI ? p.alibi_kv_off - p.alibi_q_off - (r0 + row) + k0 + tx : 0;
 #pragma unroll
-            for (int i = 0; i < kKeysPerThread; ++i) {
+            for (int i = 0; i < kKeysPerThread<D>; ++i) {
                 float sc = s[r][i] * p.scale;
-                if constexpr (ALIBI) sc = __fadd_rn(sc, __fmul_rn(slope, (float)(bias0 + 8 * i)));
-                s[r][i] = tx + 8 * i < lim ? sc : -INFINITY;
+                if constexpr (ALIBI) sc = __fadd_rn(sc, __fmul_rn(slope, (float)(bias0 + kLanes<D> * i)));
+                s[r][i] = tx + kLanes<D> * i < lim ? sc : -INFINITY;
                 mx = fmaxf(mx, s[r][i]);
             }
 #pragma unroll
-            for (int w = 1; w < 8; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
+            for (int w = 1; w < kLanes<D>; w <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, w));
             const bool any = mx != -INFINITY;  // a row none of whose keys counts in this tile keeps its state
             const float m_new = fmaxf(m[r], mx);
             const float alpha = !any ? 1.f : m[r] == -INFINITY ? 0.f : expf(m[r] - m_new);
             m[r] = m_new;
             float sum = 0.f;
 #pragma unroll
-            for (int i = 0; i < kKeysPerThread; ++i) {
+            for (int i = 0; i < kKeysPerThread<D>; ++i) {
                 const float e = !any || s[r][i] == -INFINITY ? 0.f : expf(s[r][i] - m_new);
                 sum += e;
-                ps[row * T::kPStride + tx + 8 * i] = e;
+                ps[row * T::kPStride + tx + kLanes<D> * i] = e;
             }
             l[r] = l[r] * alpha + sum;
             const uint64_t a2 = pack2(alpha, alpha);
@@ -282,7 +287,7 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
         bool by_row = false;
         if (diagonal) by_row = __syncthreads_or(copied_non_finite<D>(vs));
         else __syncthreads();
-        // V is there; a row of P is written and read by the same eight lanes
+        // V is there; a row of P is written and read by the same lanes of one warp
         if (!by_row) {
             // O += P V
 #pragma unroll 2
@@ -296,7 +301,7 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
                     ulonglong2 vv[kCols];
 #pragma unroll
                     for (int c = 0; c < kCols; ++c)
-                        vv[c] = *reinterpret_cast<const ulonglong2 *>(vs + (k + e) * D + 4 * tx + 32 * c);
+                        vv[c] = *reinterpret_cast<const ulonglong2 *>(vs + (k + e) * D + 4 * tx + 4 * kLanes<D> * c);
 #pragma unroll
                     for (int r = 0; r < kRowsPerThread; ++r) {
                         const float x = e == 0 ? pv[r].x : e == 1 ? pv[r].y : e == 2 ? pv[r].z : pv[r].w;
@@ -323,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
 #pragma unroll
     for (int r = 0; r < kRowsPerThread; ++r)
 #pragma unroll
-        for (int w = 1; w < 8; w <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], w);
+        for (int w = 1; w < kLanes<D>; w <<= 1) l[r] += __shfl_xor_sync(0xffffffffu, l[r], w);
 
     float *obase = (float *)p.o + (int64_t)b * p.o_bs + (int64_t)h * p.o_hs;
     float *lse = p.lse + ((int64_t)b * p.q_heads + h) * p.lse_hs;
@@ -336,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
 #pragma unroll
             for (int c = 0; c < kCols; ++c) {
                 const float2 a = unpack2(o[r][2 * c]), e = unpack2(o[r][2 * c + 1]);
-                *reinterpret_cast<float4 *>(obase + (int64_t)(r0 + row) * p.o_rs + 4 * tx + 32 * c) =
+                *reinterpret_cast<float4 *>(obase + (int64_t)(r0 + row) * p.o_rs + 4 * tx + 4 * kLanes<D> * c) =
                     make_float4(a.x * inv, a.y * inv, e.x * inv, e.y * inv);
             }
             if (tx == 0) lse[r0 + row] = m[r] + logf(l[r]);
@@ -357,10 +362,10 @@ __global__ void __launch_bounds__(kThreads, 2) fwd_f32_kernel(const __grid_const
     for (int r = 0; r < kRowsPerThread; ++r)
 #pragma unroll
         for (int c = 0; c < kCols; ++c)
-            *reinterpret_cast<ulonglong2 *>(os + (ty + 16 * r) * D + 4 * tx + 32 * c) = make_ulonglong2(o[r][2 * c], o[r][2 * c + 1]);
+            *reinterpret_cast<ulonglong2 *>(os + (ty + 16 * r) * D + 4 * tx + 4 * kLanes<D> * c) = make_ulonglong2(o[r][2 * c], o[r][2 * c + 1]);
     cluster.sync();
     constexpr int kVecs = kRows * (D / 4);
-    for (int i = part * kVecs / parts + threadIdx.x; i < (part + 1) * kVecs / parts; i += kThreads) {
+    for (int i = part * kVecs / parts + threadIdx.x; i < (part + 1) * kVecs / parts; i += kThreads<D>) {
         const int row = i / (D / 4), v = i % (D / 4);
         if (row >= rows) continue;
         float mx = -INFINITY;
@@ -390,7 +395,7 @@ int launch(flat_ctx *ctx, const F32Params &fp, int parts) {
     FLAT_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)((p.q_len + kRows - 1) / kRows * parts), (unsigned)p.q_heads, (unsigned)p.batch);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kThreads<D>);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
