@@ -430,7 +430,14 @@ uint64_t plan_decode(flat_ctx *ctx, int dtype, DecodeParams &p, const int32_t *h
     p.chunk_tokens = 0;
     p.balanced = 0;
     p.short_partials = 0;
+    p.cluster = 0;
     if (!decode_fast_path_ok(dtype, p.head_dim, p.group)) return 0;
+    if (kv_splits == 0 && offsets && decode_mma_supported(dtype, p)) {
+        int max_len = host_lens ? 0 : p.uniform_len;
+        for (int s = 0; host_lens && s < p.num_seqs; ++s) max_len = std::max(max_len, host_lens[s]);
+        p.cluster = decode_cluster_size(ctx, p, max_len);
+        if (p.cluster) return 0;
+    }
     if (kv_splits == 0 && offsets && decode_mma_supported(dtype, p) &&
         (uint64_t)(p.num_seqs + 1) * sizeof(int32_t) <= kWorkspaceMeta - kSeqOffsetsAt) {
         offsets->resize(p.num_seqs + 1);

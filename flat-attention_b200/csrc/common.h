@@ -208,6 +208,7 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p);
 // ---- decode ----------------------------------------------------------------------------------
 // Tables up to this size are kernel arguments of the tensor-core decode: a copy of its own costs a short context 4 us of 18.
 constexpr int kInlinePages = 256;
+constexpr int kMaxDecodeCluster = 8;  // CTAs, the portable limit
 struct DecodeParams {
     const void *q;       // [num_seqs, q_heads*head_dim]
     const void *k, *v;   // paged: [pages, page_size, kv_heads*head_dim]; resident: [batch, capacity, ...]
@@ -237,6 +238,7 @@ struct DecodeParams {
     // sequences they belong to.  seq_offsets[s] is where sequence s starts (device, num_seqs+1
     // entries).  Partial slot of (sequence, CTA) = CTA index - first CTA touching the sequence;
     // kv_splits then holds the maximum number of slots per sequence.
+    int cluster;                         // > 0: short contexts, a cluster of this many CTAs per KV head, no partials
     int out_f32;                         // write the final O as f32 whatever the storage type (cross-GPU partials)
     int balanced;
     int span_tokens;
@@ -252,6 +254,7 @@ bool decode_fast_path_ok(int dtype, int head_dim, int group);
 int launch_decode(flat_ctx *ctx, int dtype, const DecodeParams &p);
 // bf16 tensor-core decode (mma.sync), head_dim 64/128, group <= 8, pages of a multiple of 16 tokens
 bool decode_mma_supported(int dtype, const DecodeParams &p);
+int decode_cluster_size(const flat_ctx *ctx, const DecodeParams &p, int max_len);
 int launch_decode_mma(flat_ctx *ctx, const DecodeParams &p);
 // part i of the partial O / LSE starts part_stride_o / part_stride_lse floats after part i-1
 int launch_splitkv_merge(flat_ctx *ctx, int dtype, int parts, int64_t rows, int head_dim,

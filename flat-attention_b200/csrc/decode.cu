@@ -494,7 +494,7 @@ bool decode_fast_path_ok(int dtype, int head_dim, int group) {
 int launch_decode(flat_ctx *ctx, int dtype, const DecodeParams &p) {
     if (p.num_seqs > 65535) return fail(ctx, FLAT_ERR_DISPATCH_LIMIT, "decode batch %d exceeds 65535", p.num_seqs);
     if (decode_mma_supported(dtype, p)) {
-        launch_decode_mma(ctx, p);
+        if (int st = launch_decode_mma(ctx, p)) return st;
         ctx->launches += 1;
         FLAT_CUDA_OK(ctx, cudaGetLastError());
         return p.out_f32 ? merge_chunks<float>(ctx, p) : merge_chunks<__nv_bfloat16>(ctx, p);

@@ -58,6 +58,31 @@ def test_decode_asks_for_no_more_workspace_than_spans_of_64(lens):
     assert c.device_status() == 0
 
 
+# lengths around the cluster sizes of short contexts (128 tokens per CTA with one tile per warp, eight CTAs, four tiles per
+# warp), mixed batches whose shortest sequence leaves warps and CTAs without a token, and one sequence more than SMs allow
+@pytest.mark.parametrize("lens", [[128], [129], [513], [1024], [1025], [4096], [4097], [1, 17, 900], [2000, 3, 129, 64], [300] * 18,
+                                  [300] * 19])
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 8, 64), (32, 8, 128), (64, 8, 128)])
+def test_decode_clusters(lens, Hq, Hkv, D):
+    """Against the same call with one part per sequence (P is rounded to bf16, 2^-9, relative to another running maximum)."""
+    page, c = 16, ctx()
+    pages = [-(-n // page) for n in lens]
+    g = torch.Generator().manual_seed(7)
+    Q = torch.randn(len(lens), Hq * D, generator=g).bfloat16()
+    K, V = (torch.randn(sum(pages) * page, Hkv * D, generator=g).bfloat16() for _ in range(2))
+    tables = np.zeros((len(lens), max(pages)), np.int32)
+    order = np.random.default_rng(1).permutation(sum(pages))
+    for i, n in enumerate(pages):
+        tables[i, :n] = order[sum(pages[:i]):sum(pages[:i]) + n]
+    args = (fa.BF16, np.array(lens, np.int32), tables, sum(pages), max(pages), Q, K, V, Hq, Hkv, D, page, 5e5)
+    o, l = run_batched(c, *args)
+    eo, el = run_batched(c, *args, splits=1)
+    assert np.abs(o - eo).max() <= 2e-2 and np.abs(l - el).max() <= 2e-3
+    again, al = run_batched(c, *args)
+    assert np.array_equal(o, again) and np.array_equal(l, al)
+    assert c.device_status() == 0
+
+
 # (B, Hq, Hkv, N, D): clusters of 1, 4, 3, 8 and 8 CTAs per key tile on 148 SMs, with and without a mask
 @pytest.mark.parametrize("B,Hq,Hkv,N,D", [(1, 4, 4, 100, 64), (1, 8, 1, 130, 128), (1, 12, 1, 128, 64), (1, 32, 2, 600, 64),
                                           (1, 16, 1, 700, 128)])
