@@ -630,6 +630,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_launch();  // the next call's first kernel, behind this CTA's TMEM allocation
     grid_dependency_wait();
     constexpr uint32_t kColQ = 0, kColX = 64, kColY = 192, kColDS = 320, kColAcc = 384;
 
@@ -924,6 +925,7 @@ __global__ void __launch_bounds__(DqSpillCfg<D, HEADS>::kThreadsDq, 1) bwd_dq_sp
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    grid_dependency_launch();  // the next call's first kernel, behind this CTA's TMEM allocation
     grid_dependency_wait();
 
     if (warp == 4 && !*abort_flag && elect_one()) {
@@ -1009,10 +1011,11 @@ __global__ void __launch_bounds__(DqSpillCfg<D, HEADS>::kThreadsDq, 1) bwd_dq_sp
 constexpr int kPrepFlight = 4;
 template <int D> constexpr int kPrepRows = kPrepFlight * 256 / (D / 8);
 template <int D>
-__global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *__restrict__ d_out,
-                                                       const __nv_bfloat16 *__restrict__ out, const float *__restrict__ lse,
-                                                       float *__restrict__ delta, float *__restrict__ neg_lse2, int seq_len,
-                                                       int seq_pad) {
+__global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *d_out, const __nv_bfloat16 *out, const float *lse, float *delta,
+                                                       float *neg_lse2, int seq_len, int seq_pad) {
+    // what the dK/dV kernel reads before its own wait is complete once this wait is over; the inputs may come from the kernel
+    // before, so nothing here is read through the read-only path
+    grid_dependency_wait();
     grid_dependency_launch();
     constexpr int kLanes = D / 8, kStep = 256 / kLanes;
     static_assert(kTile % kPrepRows<D> == 0, "a block's rows lie in one (batch, head)");
@@ -1023,8 +1026,8 @@ __global__ void __launch_bounds__(256) bwd_prep_kernel(const __nv_bfloat16 *__re
 #pragma unroll
     for (int u = 0; u < kPrepFlight; ++u) {
         const int64_t row = bh * seq_len + min(n0 + u * kStep, seq_len - 1);
-        a[u] = __ldg(reinterpret_cast<const uint4 *>(d_out + row * D) + sub);
-        o[u] = __ldg(reinterpret_cast<const uint4 *>(out + row * D) + sub);
+        a[u] = reinterpret_cast<const uint4 *>(d_out + row * D)[sub];
+        o[u] = reinterpret_cast<const uint4 *>(out + row * D)[sub];
     }
 #pragma unroll
     for (int u = 0; u < kPrepFlight; ++u) {
@@ -1097,8 +1100,9 @@ int launch_backward_sm100(flat_ctx *ctx, const BwdParams &p) {
     float *delta = reinterpret_cast<float *>(scratch_ptr(ctx));
     float *neg_lse2 = delta + rows_pad;
     auto *prep = D == 128 ? bwd_prep_kernel<128> : bwd_prep_kernel<64>;
-    prep<<<(unsigned)(rows_pad / (D == 128 ? kPrepRows<128> : kPrepRows<64>)), 256, 0, ctx->stream>>>(
-        static_cast<const __nv_bfloat16 *>(p.d_out), static_cast<const __nv_bfloat16 *>(p.out), p.lse, delta, neg_lse2, N, seq_pad);
+    FLAT_CUDA_OK(ctx, launch_dependent(may_overlap_previous(ctx), prep, dim3((unsigned)(rows_pad / (D == 128 ? kPrepRows<128> : kPrepRows<64>))),
+                                       256, 0, ctx->stream, static_cast<const __nv_bfloat16 *>(p.d_out),
+                                       static_cast<const __nv_bfloat16 *>(p.out), p.lse, delta, neg_lse2, N, seq_pad));
     ctx->launches += 1;
 
     BwdKernelParams kp{};

@@ -338,6 +338,7 @@ __global__ void __launch_bounds__(32 * WARPS) merge_row_kernel(int parts, int he
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t row = blockIdx.x;
     int live = parts;
+    grid_dependency_launch();
     grid_dependency_wait();
     if (seq_offsets) {
         const int seq = (int)(row / rows_per_seq);

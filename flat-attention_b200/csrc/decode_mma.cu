@@ -329,6 +329,8 @@ __global__ void __launch_bounds__(32 * kClusterWarps, 1)
     __shared__ float2 part_ml[kClusterWarps][8];
     __shared__ __align__(16) float cta_o[8 * D];
     __shared__ float2 cta_ml[8];
+    grid_dependency_launch();
+    grid_dependency_wait();
     cg::cluster_group cluster = cg::this_cluster();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;
@@ -428,6 +430,7 @@ __global__ void __launch_bounds__(32 * kClusterWarps, 1)
 
 template <int D, typename Table>
 __global__ void __launch_bounds__(256, 2) decode_mma_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__ Table table) {
+    grid_dependency_wait();
     const int warp = threadIdx.x >> 5;
     const int kv_head = blockIdx.y * (blockDim.x >> 5) + warp;
     if (kv_head >= p.kv_heads) return;
@@ -497,11 +500,13 @@ static cudaError_t launch_cluster(flat_ctx *ctx, const DecodeParams &p, const Ta
     cfg.gridDim = dim3((unsigned)p.cluster, (unsigned)p.kv_heads, (unsigned)p.num_seqs);
     cfg.blockDim = dim3(32 * kClusterWarps);
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim = {(unsigned)p.cluster, 1, 1};
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_dependent()
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = may_overlap_previous(ctx) ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, decode_cluster_kernel<D, Table>, p, table);
 }
 
@@ -520,16 +525,16 @@ int launch_decode_mma(flat_ctx *ctx, const DecodeParams &p) {
     const int warps = p.kv_heads < 8 ? p.kv_heads : 8;
     dim3 grid(p.kv_splits, (p.kv_heads + warps - 1) / warps, p.num_seqs);
     if (p.balanced) grid = dim3(p.num_ctas, (p.kv_heads + warps - 1) / warps, 1);
+    const bool overlap = may_overlap_previous(ctx);
     KernelTimer timer(ctx);
     if (p.host_pages) {
         InlineTable table;
         std::copy(p.host_pages, p.host_pages + p.max_pages, table.pages);
-        if (p.head_dim == 128) decode_mma_kernel<128, InlineTable><<<grid, warps * 32, 0, ctx->stream>>>(p, table);
-        else decode_mma_kernel<64, InlineTable><<<grid, warps * 32, 0, ctx->stream>>>(p, table);
-    } else if (p.head_dim == 128) {
-        decode_mma_kernel<128, DeviceTable><<<grid, warps * 32, 0, ctx->stream>>>(p, DeviceTable{});
+        FLAT_CUDA_OK(ctx, launch_dependent(overlap, p.head_dim == 128 ? decode_mma_kernel<128, InlineTable> : decode_mma_kernel<64, InlineTable>,
+                                           grid, warps * 32, 0, ctx->stream, p, table));
     } else {
-        decode_mma_kernel<64, DeviceTable><<<grid, warps * 32, 0, ctx->stream>>>(p, DeviceTable{});
+        FLAT_CUDA_OK(ctx, launch_dependent(overlap, p.head_dim == 128 ? decode_mma_kernel<128, DeviceTable> : decode_mma_kernel<64, DeviceTable>,
+                                           grid, warps * 32, 0, ctx->stream, p, DeviceTable{}));
     }
     return FLAT_OK;
 }

@@ -159,6 +159,8 @@ __global__ void __launch_bounds__(kThreads<D>, 2) fwd_f32_kernel(const __grid_co
     using T = Tile<D>;
     constexpr int kCols = D / (4 * kLanes<D>);  // float4 columns of O per thread and row
     const FwdParams &p = fp.f;
+    grid_dependency_launch();
+    grid_dependency_wait();
     extern __shared__ __align__(16) float smem[];
     float *qs = smem + T::kQ, *ks = smem + T::kK, *vs = smem + T::kV, *stat = smem + T::kStat;
     float *ps = ks;
@@ -398,12 +400,14 @@ int launch(flat_ctx *ctx, const F32Params &fp, int parts) {
     cfg.blockDim = dim3(kThreads<D>);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // see launch_dependent()
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)parts;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = may_overlap_previous(ctx) ? 2 : 1;
     FLAT_CUDA_OK(ctx, cudaLaunchKernelEx(&cfg, kernel, fp));
     ctx->launches += 1;
     return FLAT_OK;

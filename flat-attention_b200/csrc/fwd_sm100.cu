@@ -194,6 +194,7 @@ struct KernelParams {
     float alibi_inline[kInlineSlopes];
     int alibi_delta;            // ALIBI kernels: bias position of key 0 minus bias position of query row 0
     float alibi_inv_scale;      // ALIBI kernels: 1 / softmax scale
+    int first_in_call;  // no kernel of this call before this one: wait before any access to memory
     long long *trace;
 };
 
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
 
     const int warp = warp_index_uniform();
     const int lane = threadIdx.x & 31;
-    if constexpr (SPLIT) grid_dependency_launch();  // the merge kernel
+    grid_dependency_launch();  // the merge kernel, or the next call's first
 
     if (warp == kProducerWarp && lane == 0) {
         *abort_flag = 0;
@@ -479,6 +480,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
+    if (p.first_in_call) grid_dependency_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1164,6 +1166,7 @@ template <int D, bool F16IO>
 __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const __grid_constant__ KernelParams p, int first_lin) {
     constexpr int kCols = D / 32;
     constexpr int kRowsPerCta = 2 * kTileRows / kMergeCtasPerItem;
+    grid_dependency_launch();
     grid_dependency_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int item = blockIdx.x / kMergeCtasPerItem;
@@ -1220,10 +1223,10 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const __grid_const
 // rotation blocks still wait for and come up in another order (604 -> 647 us for B = 4, N = 4096, 32 / 8 heads, D = 128).
 constexpr int kRotateHeads = 4;
 template <int D, bool F16IN>
-__global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *__restrict__ x, __half *__restrict__ y,
-                                                            const float2 *__restrict__ table, int heads, int rows, int batch_heads,
-                                                            int64_t bs, int64_t hs, int64_t rs) {
+__global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *x, __half *y, const float2 *__restrict__ table,
+                                                            int heads, int rows, int batch_heads, int64_t bs, int64_t hs, int64_t rs) {
     constexpr int kVecs = D / 8;
+    grid_dependency_wait();
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
     const int v = (int)(i % kVecs);
     const int n = (int)(i / kVecs);
@@ -1447,8 +1450,9 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
                               (unsigned)std::min((batch_heads + kRotateHeads - 1) / kRotateHeads, 65535));
             auto *rotate = D == 128 ? (p.f16_io ? rotate_to_f16_kernel<128, true> : rotate_to_f16_kernel<128, false>)
                                     : (p.f16_io ? rotate_to_f16_kernel<64, true> : rotate_to_f16_kernel<64, false>);
-            rotate<<<blocks, 256, 0, ctx->stream>>>(reinterpret_cast<const uint16_t *>(p.k), rk, kt, p.kv_heads, p.kv_len, batch_heads,
-                                                    p.kv_bs, p.kv_hs, p.kv_rs);
+            FLAT_CUDA_OK(ctx, launch_dependent(may_overlap_previous(ctx), rotate, blocks, 256, 0, ctx->stream,
+                                               reinterpret_cast<const uint16_t *>(p.k), rk, kt, p.kv_heads, p.kv_len, batch_heads, p.kv_bs,
+                                               p.kv_hs, p.kv_rs));
             ctx->launches += 1;
             k_ptr = rk;
             k_rs = D; k_hs = (int64_t)p.kv_len * D; k_bs = k_hs * p.kv_heads;
@@ -1528,8 +1532,9 @@ int launch_forward_sm100(flat_ctx *ctx, const FwdParams &p) {
     auto run = [&](auto kernel, int smem_bytes) -> int {
         FLAT_CUDA_OK(ctx, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes));
         KernelTimer timer(ctx);
-        // the kernel before this one in the stream is the K rotation: all it has to wait for
-        FLAT_CUDA_OK(ctx, launch_dependent(p.rope_k, kernel, dim3(grid), kThreads, smem_bytes, ctx->stream, kp));
+        // the kernel before this one in the stream is the K rotation, all it has to wait for, or one of another call
+        kp.first_in_call = !p.rope_k;
+        FLAT_CUDA_OK(ctx, launch_dependent(p.rope_k || may_overlap_previous(ctx), kernel, dim3(grid), kThreads, smem_bytes, ctx->stream, kp));
         if (plan.split > 1) {
             const int first_lin = plan.full_rounds * (int)grid;
             auto *merge = D == 128 ? (io16 ? fwd_split_merge_kernel<128, true> : fwd_split_merge_kernel<128, false>)

@@ -285,3 +285,91 @@ def test_captured_calls_replay_to_the_same_bits():
     torch.cuda.synchronize()
     assert all(torch.equal(x, y) for x, y in zip((out, grads, dec), want))
     assert c.device_status() == 0
+
+
+# one forward kernel, rotation and forward, rotation, forward and merge of split parts; the tiled f32 kernel
+@pytest.mark.parametrize("dtype,rope,H,N,D", [("BF16", False, 2, 100, 64), ("BF16", True, 4, 333, 128), ("F16", True, 2, 4096, 64),
+                                              ("F32", True, 2, 200, 128)])
+def test_calls_that_read_what_the_call_before_wrote(dtype, rope, H, N, D):
+    """Calls overlap their launches with the end of the call before; what they read is complete all the same.  Each forward
+    takes the output of the one before as Q, K and V."""
+    c, code = ctx(), getattr(fa, dtype)
+    td, shp = fa.torch_dtype(code), fa.shape(1, H, H, N, N, D)
+    first = torch.randn(H * N * D, generator=torch.Generator().manual_seed(1)).to(td).cuda()
+    outs = [c.create_output_buffer(code, shp) for _ in range(12)]
+
+    def chain(between):
+        x = first
+        for out in outs:
+            if rope:
+                c.forward_grouped_rope(code, shp, fa.config(True), fa.rotary(5e5, 0, 0), x, x, x, out)
+            else:
+                c.forward_grouped(code, shp, fa.config(True), x, x, x, out)
+            between()
+            x = c.split_output(out, code, shp)[0].reshape(-1)
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    expected = chain(torch.cuda.synchronize)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(chain(lambda: None), expected))
+    assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [40, 700, 9000])
+def test_decode_steps_that_read_the_step_before(n):
+    """The same for decode steps, in clusters and in spans with a merge: each takes the output of the one before as Q."""
+    H, D, c = 8, 128, ctx()
+    cache = fa.CudaResidentKvCache(c, fa.BF16, 1, H, n, D)
+    g = torch.Generator().manual_seed(2)
+    cache.record_append(*(torch.randn(n * H * D, generator=g).bfloat16().cuda() for _ in range(2)), n)
+    first = torch.randn(H * D, generator=g).bfloat16().cuda()
+    outs = [c.create_decode_output_buffer(fa.BF16, 1, H, D) for _ in range(30)]
+
+    def chain(between):
+        x = first
+        for out in outs:
+            c.decode_resident(fa.BF16, 1, H, H, D, n, n, fa.config(True), 5e5, n - 1, x, cache.k_buffer(), cache.v_buffer(), out)
+            between()
+            x = c.split_decode_output(out, fa.BF16, 1, H, D)[0].reshape(-1)
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    expected = chain(torch.cuda.synchronize)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(chain(lambda: None), expected))
+    assert c.device_status() == 0
+
+
+def test_backward_that_reads_the_forward_before():
+    """Training steps back to back: the gradients of each are those of its own forward."""
+    B, Hq, Hkv, N, D, c = 2, 8, 2, 300, 64, ctx()
+    shp, cfg = fa.shape(B, Hq, Hkv, N, N, D), fa.config(True)
+    L = fa.backward_layout(fa.BF16, shp)
+    packed, g = c.empty_bytes(L.input_bytes), torch.Generator().manual_seed(3)
+
+    def view(at, count):
+        return packed[at:at + 2 * count].view(torch.bfloat16)
+
+    q, k, v, do = view(L.q_offset, L.q_elements), view(L.k_offset, L.kv_elements), view(L.v_offset, L.kv_elements), view(L.d_out_offset, L.q_elements)
+    for x in (q, k, v, do):
+        x.copy_(torch.randn(x.numel(), generator=g).bfloat16())
+    start, grads = packed.clone(), [c.empty_bytes(L.output_bytes) for _ in range(10)]
+
+    def steps(between):
+        packed.copy_(start)
+        for grad in grads:
+            c.forward_grouped(fa.BF16, shp, cfg, q, k, v, packed[L.out_offset:])
+            between()
+            c.backward_grouped(fa.BF16, shp, cfg, packed, grad)
+            between()
+            c.forward_grouped(fa.BF16, shp, cfg, q, k, v, packed[L.out_offset:])  # O becomes the next step's Q
+            between()
+            q.copy_(view(L.out_offset, L.q_elements))
+        torch.cuda.synchronize()
+        return [x.clone() for x in grads]
+
+    expected = steps(torch.cuda.synchronize)
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(steps(lambda: None), expected))
+    assert c.device_status() == 0
