@@ -9,7 +9,7 @@
 // Few query blocks leave most SMs idle and the causal diagonal makes them uneven, so the KV tiles of a query block are
 // dealt to a cluster of up to 8 CTAs, which combine their (max, sum, O) through distributed shared memory in rank
 // order: one launch, no scratch, bitwise repeatable.  8 / 2 heads, 512 rows, D = 128, causal, RoPE: 219 us with the kernel of
-// fwd_simt.cu, 44 us here; 2 x 2048 rows, 16 / 4 heads 3470 us and 1180 us (29 TFLOP/s).
+// fwd_simt.cu, 42 us here; 2 x 2048 rows, 16 / 4 heads 3470 us and 1180 us (29 TFLOP/s).
 // RoPE: K and Q are rotated on the way into shared memory with the (cos, sin) table of the call's positions (find_tables());
 // without one the same sincosf runs here.
 #include <cooperative_groups.h>
