@@ -147,8 +147,9 @@ inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 g
 // Whether the first kernel of a call may be launched the same way, behind whatever kernel is before it in the stream: the end
 // of one call and the launch and set-up of the next then overlap.  Such a kernel waits (grid_dependency_wait()) before its
 // first access to memory, and a kernel that lets its dependents start before its own wait has only dependents that do the
-// same: what a call reads is complete when it reads it.  Not while the stream is captured, where the kernel before may be a
-// node of any kind.
+// same: what a call reads is complete when it reads it.  It may have been written while the kernel was already resident, so
+// no dependent kernel reads through the read-only path (.nc, __ldg, const __restrict__).  Not while the stream is captured,
+// where the kernel before may be a node of any kind.
 inline bool may_overlap_previous(flat_ctx *ctx) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) {

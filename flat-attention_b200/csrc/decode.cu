@@ -329,11 +329,10 @@ __global__ void __launch_bounds__(kMergeDims * GROUPS) merge_kernel(int parts, i
 // rows of 150 parts (2 sequences of 60001 tokens) take 6.4 us where a block reduction, staged weights and one column per
 // thread took 8.5; a decode step of 700 tokens went from 12.3 to 10.3 us.
 template <typename T, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) merge_row_kernel(int parts, int head_dim, const float *__restrict__ partial_o,
-                                                               const float *__restrict__ partial_lse, T *__restrict__ o,
-                                                               float *__restrict__ lse, const int32_t *context_lens,
-                                                               int uniform_len, int chunk_tokens, int rows_per_seq,
-                                                               const int32_t *seq_offsets, int span_tokens, int64_t rows) {
+__global__ void __launch_bounds__(32 * WARPS) merge_row_kernel(int parts, int head_dim, const float *partial_o, const float *partial_lse,
+                                                               T *o, float *lse, const int32_t *context_lens, int uniform_len,
+                                                               int chunk_tokens, int rows_per_seq, const int32_t *seq_offsets,
+                                                               int span_tokens, int64_t rows) {
     __shared__ float4 acc_s[WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t row = blockIdx.x;

@@ -31,9 +31,11 @@ namespace cg = cooperative_groups;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 
-__device__ __forceinline__ uint4 ldg_stream(const void *p) {
+// K and V are read once.  Not through the read-only path (.nc): the kernel may be resident while the one before it in the
+// stream still writes them (launch_dependent()), and .nc is for memory that nobody writes while the kernel runs.
+__device__ __forceinline__ uint4 ld_stream(const void *p) {
     uint4 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
     return r;
 }
@@ -154,8 +156,8 @@ __device__ __forceinline__ void load_tile(const DecodeParams &p, int kv_head, in
     const bool ok_a = g < left, ok_b = g + 8 < left;
 #pragma unroll
     for (int j = 0; j < kChunks; ++j) {
-        x.ka[j] = ok_a ? ldg_stream(ktile + (int64_t)g * row_bytes + (32 * j + 8 * c) * 2) : make_uint4(0, 0, 0, 0);
-        x.kb[j] = ok_b ? ldg_stream(ktile + (int64_t)(g + 8) * row_bytes + (32 * j + 8 * c) * 2) : make_uint4(0, 0, 0, 0);
+        x.ka[j] = ok_a ? ld_stream(ktile + (int64_t)g * row_bytes + (32 * j + 8 * c) * 2) : make_uint4(0, 0, 0, 0);
+        x.kb[j] = ok_b ? ld_stream(ktile + (int64_t)(g + 8) * row_bytes + (32 * j + 8 * c) * 2) : make_uint4(0, 0, 0, 0);
     }
     const int vt[4] = {2 * c, 2 * c + 1, 2 * c + 8, 2 * c + 9};
 #pragma unroll
@@ -163,7 +165,7 @@ __device__ __forceinline__ void load_tile(const DecodeParams &p, int kv_head, in
         const bool ok = vt[i] < left;
 #pragma unroll
         for (int u = 0; u < kVecs; ++u)
-            x.vv[i][u] = ok ? ldg_stream(vtile + (int64_t)vt[i] * row_bytes + ((D / 8) * g + 8 * u) * 2) : make_uint4(0, 0, 0, 0);
+            x.vv[i][u] = ok ? ld_stream(vtile + (int64_t)vt[i] * row_bytes + ((D / 8) * g + 8 * u) * 2) : make_uint4(0, 0, 0, 0);
     }
 }
 

@@ -336,7 +336,7 @@ __device__ __forceinline__ void rotate_q_tile(const KernelParams &p, const WorkI
     {
         const int rr = nx.table_row0 + min(first_row + lane_base + lane / CH, nx.q_len - 1);
         const float4 *tp = reinterpret_cast<const float4 *>(p.rope_q_table + (long long)rr * (D / 2)) + 2 * ch;
-        const float4 cs0 = __ldg(tp), cs1 = __ldg(tp + 1);  // (c, s, c, s) x 2
+        const float4 cs0 = tp[0], cs1 = tp[1];  // (c, s, c, s) x 2
         cc[0] = cs0.x; ss[0] = cs0.y; cc[1] = cs0.z; ss[1] = cs0.w;
         cc[2] = cs1.x; ss[2] = cs1.y; cc[3] = cs1.z; ss[3] = cs1.w;
 #pragma unroll
@@ -954,7 +954,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             // position arithmetic is exact.
             float slope_rel = 0.f, bias_pos0 = 0.f;
             if constexpr (ALIBI) {
-                slope_rel = (p.alibi_slopes ? __ldg(p.alibi_slopes + it.h) : p.alibi_inline[it.h]) * p.alibi_inv_scale;
+                slope_rel = (p.alibi_slopes ? p.alibi_slopes[it.h] : p.alibi_inline[it.h]) * p.alibi_inv_scale;
                 bias_pos0 = (float)(p.alibi_delta + it.j0 * kTileRows - (it.r0 + w * kTileRows + row_in_tile));
             }
 
@@ -1223,7 +1223,7 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const __grid_const
 // rotation blocks still wait for and come up in another order (604 -> 647 us for B = 4, N = 4096, 32 / 8 heads, D = 128).
 constexpr int kRotateHeads = 4;
 template <int D, bool F16IN>
-__global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *x, __half *y, const float2 *__restrict__ table,
+__global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *x, __half *y, const float2 *table,
                                                             int heads, int rows, int batch_heads, int64_t bs, int64_t hs, int64_t rs) {
     constexpr int kVecs = D / 8;
     grid_dependency_wait();
@@ -1232,7 +1232,7 @@ __global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *x, _
     const int n = (int)(i / kVecs);
     if (n >= rows) return;
     const float4 *tab = reinterpret_cast<const float4 *>(table + (int64_t)n * (D / 2) + v * 4);
-    const float4 cs0 = __ldg(tab), cs1 = __ldg(tab + 1);
+    const float4 cs0 = tab[0], cs1 = tab[1];
     const float cc[4] = {cs0.x, cs0.z, cs1.x, cs1.z}, ss[4] = {cs0.y, cs0.w, cs1.y, cs1.w};
     for (int bh0 = blockIdx.y * kRotateHeads; bh0 < batch_heads; bh0 += gridDim.y * kRotateHeads) {
         uint4 raw[kRotateHeads];

@@ -373,3 +373,130 @@ def test_backward_that_reads_the_forward_before():
     for _ in range(5):
         assert all(torch.equal(a, b) for a, b in zip(steps(lambda: None), expected))
     assert c.device_status() == 0
+
+
+# clusters of one tile per warp and of several, spans with a merge
+@pytest.mark.parametrize("n", [40, 700, 9000])
+@pytest.mark.parametrize("paged", [True, False])
+def test_decode_of_tokens_that_the_call_before_appended(n, paged):
+    """A serving loop appends and decodes: each step reads K and V that the call directly before it wrote, over and over at the
+    same addresses and with other values each time."""
+    Hq, Hkv, D, c, steps = 8, 8, 128, ctx(), 8
+    cache = (fa.CudaPagedKvCache(c, fa.BF16, 16, (n + 15) // 16, Hkv, D) if paged else fa.CudaResidentKvCache(c, fa.BF16, 1, Hkv, n, D))
+    g = torch.Generator(device="cuda").manual_seed(n)
+    kv = [torch.randn(2, n * Hkv * D, generator=g, device="cuda").bfloat16() for _ in range(steps)]
+    q = torch.randn(Hq * D, generator=g, device="cuda").bfloat16()
+    outs = [c.create_decode_output_buffer(fa.BF16, 1, Hq, D) for _ in range(steps)]
+
+    def loop(between):
+        for (k, v), out in zip(kv, outs):
+            cache.reset()
+            cache.record_append(k, v, n)
+            between()
+            if paged:
+                c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, n - 1, q, cache.k_buffer(), cache.v_buffer(), out)
+            else:
+                c.decode_resident(fa.BF16, 1, Hq, Hkv, D, n, n, fa.config(True), 5e5, n - 1, q, cache.k_buffer(), cache.v_buffer(), out)
+            between()
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    expected = loop(torch.cuda.synchronize)
+    assert not torch.equal(expected[0], expected[1])
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(loop(lambda: None), expected))
+    assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [128, 700, 9000])
+def test_decode_of_the_output_of_the_forward_before(n):
+    """K and V of a decode are the output of the forward launched directly before it, whose last kernel lets its dependents
+    start early."""
+    H, D, c, steps = 8, 128, ctx(), 6
+    shp = fa.shape(1, H, H, n, n, D)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    x, q = (torch.randn(rows * H * D, generator=g, device="cuda").bfloat16() for rows in (n, 1))
+    out = c.create_output_buffer(fa.BF16, shp)  # one buffer: the forward of a step overwrites what the decode before it read
+    o = c.split_output(out, fa.BF16, shp, fa.PROJECTION)[0].reshape(-1)
+    outs = [c.create_decode_output_buffer(fa.BF16, 1, H, D) for _ in range(steps)]
+
+    def loop(between):
+        for i, dec in enumerate(outs):
+            c.forward_projection_rope_asymmetric(fa.BF16, shp, fa.config(i % 2 == 0), fa.rotary(5e5, 0, 0), x, x, x, out)
+            between()
+            c.decode_resident(fa.BF16, 1, H, H, D, n, n, fa.config(True), 5e5, n - 1, q, o, o, dec)
+            between()
+        torch.cuda.synchronize()
+        return [dec.clone() for dec in outs]
+
+    expected = loop(torch.cuda.synchronize)
+    assert not torch.equal(expected[0], expected[1])
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(loop(lambda: None), expected))
+    assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("dtype,rotate_k", [("BF16", True), ("BF16", False), ("F16", True), ("F32", True)])
+def test_calls_that_fill_a_new_rotation_table(dtype, rotate_k):
+    """Each call has other positions, so the (cos, sin) table that its first kernel reads was written directly before it."""
+    H, N, D, c, code = 4, 200, 128, ctx(), getattr(fa, dtype)
+    td, shp = fa.torch_dtype(code), fa.shape(1, H, H, N, N, D)
+    g = torch.Generator().manual_seed(1)
+    q, k, v = (torch.randn(N * H * D, generator=g).to(td).cuda() for _ in range(3))
+    outs = [c.create_output_buffer(code, shp) for _ in range(10)]
+
+    def loop(between):
+        for i, out in enumerate(outs):
+            c.forward_projection_rope_asymmetric(code, shp, fa.config(True), fa.rotary(5e5, 1000 * i + 7, 500 * i, rotate_k), q, k, v, out)
+            between()
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    expected = loop(torch.cuda.synchronize)
+    assert not torch.equal(expected[0], expected[1])
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(loop(lambda: None), expected))
+    assert c.device_status() == 0
+
+
+@pytest.mark.parametrize("kind", ["forward", "f32", "decode"])
+def test_overlapped_calls_behind_another_stream(kind):
+    """The context changes its stream, and a call's input comes from work of another stream that its own was made to wait for."""
+    H, N, D, page = 4, 700, 128, 16
+    code = fa.F32 if kind == "f32" else fa.BF16
+    td, streams = fa.torch_dtype(code), [torch.cuda.Stream() for _ in range(2)]
+    c, shp = fa.Context(0, stream=streams[0]), fa.shape(1, H, H, N, N, D)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    a = torch.randn(2048, 2048, generator=g, device="cuda")
+    x = torch.empty(N * H * D, dtype=td, device="cuda")
+    outs = [c.create_decode_output_buffer(code, 1, H, D) if kind == "decode" else c.create_output_buffer(code, shp) for _ in range(10)]
+
+    def call(out):
+        if kind == "decode":
+            c.decode_resident(code, 1, H, H, D, N, N, fa.config(True), 5e5, N - 1, x[:H * D], x, x, out)
+        else:
+            c.forward_grouped_rope(code, shp, fa.config(True), fa.rotary(5e5, 0), x, x, x, out)
+
+    def loop(between):
+        for i, out in enumerate(outs):
+            mine, other = streams[i % 2], streams[1 - i % 2]
+            mine.wait_stream(other)  # the scratch of the context is the call before's until then
+            with torch.cuda.stream(other):
+                other.wait_stream(mine)
+                y = a
+                for _ in range(4):
+                    y = y @ a * 0.02
+                x.copy_((y.reshape(-1)[:x.numel()] + i).to(td))
+            mine.wait_stream(other)
+            c.set_stream(mine)
+            call(out)
+            call(out)
+            between()
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    expected = loop(torch.cuda.synchronize)
+    assert not torch.equal(expected[0], expected[1])
+    for _ in range(3):
+        assert all(torch.equal(p, q) for p, q in zip(loop(lambda: None), expected))
+    assert c.device_status() == 0
