@@ -207,16 +207,18 @@ __device__ __forceinline__ void take_tile(const uint32_t (&qhi)[D / 32][4], cons
     if (g + 8 >= left) s[2] = s[3] = -INFINITY;
 
     // ---- online softmax per head (columns 2c, 2c+1); tokens live on g: reduce over lanes 4, 8, 16
+    const float m0 = st.m0, m1 = st.m1;
     float mx0 = fmaxf(s[0], s[2]), mx1 = fmaxf(s[1], s[3]);
 #pragma unroll
     for (int w = 4; w < 32; w <<= 1) {
         mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, w));
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, w));
     }
-    const float n0 = fmaxf(st.m0, mx0), n1 = fmaxf(st.m1, mx1);  // finite: every tile has a live token g = 0
-    const float a0 = ex2f(st.m0 - n0), a1 = ex2f(st.m1 - n1);    // m = -inf gives 0
-    st.m0 = n0;
-    st.m1 = n1;
+    st.m0 = fmaxf(st.m0, mx0);
+    st.m1 = fmaxf(st.m1, mx1);
+    // every score so far -inf: their exponentials are 0 (a NaN stays one)
+    const float n0 = st.m0 == -INFINITY ? 0.f : st.m0, n1 = st.m1 == -INFINITY ? 0.f : st.m1;
+    const float a0 = ex2f(m0 - n0), a1 = ex2f(m1 - n1);  // m = -inf gives 0
     s[0] = ex2f(s[0] - n0);
     s[2] = ex2f(s[2] - n0);
     s[1] = ex2f(s[1] - n1);
@@ -370,7 +372,9 @@ __global__ void __launch_bounds__(32 * kClusterWarps, 1)
         const int h = 2 * c + hh;
         if (h >= G) continue;
         const float m = hh ? st.m1 : st.m0, l = hh ? st.l1 : st.l0;
-        const bool live = l > 0.f;  // not a warp without a token, nor one whose scores are not finite: both count for nothing
+        // A warp without a live token, or whose scores are all -inf, counts for nothing.  A NaN score makes l NaN: such a part
+        // counts, here and below, so that O and LSE of the head come out NaN and not as those of the other warps' tokens.
+        const bool live = l != 0.f;
         float *to = &part_o[warp][h][(D / 8) * g];
 #pragma unroll
         for (int i = 0; i < D / 16; i += 2)
@@ -388,7 +392,7 @@ __global__ void __launch_bounds__(32 * kClusterWarps, 1)
 #pragma unroll
         for (int w = 0; w < kClusterWarps; ++w) {
             const float2 ml = part_ml[w][h];
-            const float f = ml.x == -INFINITY ? 0.f : ex2f(ml.x - mx);
+            const float f = ml.y == 0.f ? 0.f : ex2f(ml.x - mx);
             sum = fmaf(f, ml.y, sum);
             o = fmaf(f, part_o[w][h][d], o);
         }
@@ -414,13 +418,13 @@ __global__ void __launch_bounds__(32 * kClusterWarps, 1)
         }
 #pragma unroll
         for (int r = 0; r < kMaxDecodeCluster; ++r) {
-            const float f = ml[r].x == -INFINITY ? 0.f : ex2f(ml[r].x - mx);
+            const float f = ml[r].y == 0.f ? 0.f : ex2f(ml[r].x - mx);
             sum = fmaf(f, ml[r].y, sum);
             o0 = fmaf(f, x[r].x, o0);
             o1 = fmaf(f, x[r].y, o1);
         }
-        // no maximum only when every tile was skipped (flagged page-table entries): O = 0, LSE = -inf
-        const bool empty = mx == -INFINITY;
+        // nothing counts only when every tile was skipped (flagged page-table entries): O = 0, LSE = -inf
+        const bool empty = sum == 0.f;
         const float inv = empty ? 0.f : 1.0f / sum;
         const int64_t row = (int64_t)seq * p.q_heads + kv_head * G + h;
         if (p.out_f32) *reinterpret_cast<float2 *>((float *)p.o + row * D + d) = make_float2(o0 * inv, o1 * inv);

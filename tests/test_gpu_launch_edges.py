@@ -83,6 +83,55 @@ def test_decode_clusters(lens, Hq, Hkv, D):
     assert c.device_status() == 0
 
 
+# tokens: clusters of one CTA and of eight (one tile per warp, several), and spans with a merge
+@pytest.mark.parametrize("n", [10, 40, 700, 4096, 6000])
+def test_decode_of_scores_that_are_not_finite(n):
+    """A NaN in a query, or in a key, reaches O of the heads that meet it, whichever warp or CTA has the key; the other heads keep
+    every bit.  Keys whose score overflows to -inf count for nothing."""
+    Hq, Hkv, D, page, c = 8, 2, 128, 16, ctx()
+    G = Hq // Hkv
+    rng = torch.Generator().manual_seed(n)
+    k, v = (torch.randn(n, Hkv, D, generator=rng).bfloat16() for _ in range(2))
+    q = torch.randn(Hq, D, generator=rng).bfloat16()
+
+    def decode(q, k):
+        cache = fa.CudaPagedKvCache(c, fa.BF16, page, -(-n // page), Hkv, D)
+        cache.record_append(k.reshape(-1).cuda(), v.reshape(-1).cuda(), n)
+        out = c.create_decode_output_buffer(fa.BF16, 1, Hq, D)
+        before = c.launch_count()
+        c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, n - 1, q.reshape(-1).cuda(), cache.k_buffer(),
+                       cache.v_buffer(), out)
+        assert c.launch_count() - before == (1 if n <= 4096 else 2)
+        return unpack(out, fa.BF16, Hq, D)
+
+    o, l = (x.reshape(Hq, -1) for x in decode(q, k))
+    bad = q.clone()
+    bad[1, 5] = float("nan")
+    bo, bl = (x.reshape(Hq, -1) for x in decode(bad, k))
+    others = np.arange(Hq) != 1
+    assert np.isnan(bo[1]).all() and not np.isfinite(bl[1]).any()
+    assert np.array_equal(bo[others], o[others]) and np.array_equal(bl[others], l[others])
+    for token in (0, n // 2, n - 1):
+        bad = k.clone()
+        bad[token, 1, 5] = float("nan")
+        bo, bl = (x.reshape(Hq, -1) for x in decode(q, bad))
+        assert np.isnan(bo[G:]).all(), token
+        assert np.isnan(bl[G:]).all() or n > 4096, token
+        assert np.array_equal(bo[:G], o[:G]) and np.array_equal(bl[:G], l[:G]), token
+    # The last pair of dimensions turns by at most 6000 * 5e5^(-126/128) = 0.015, and Q is scaled by 2^-3: 2^64 against -2^70
+    # overflows, but not the low half of Q (2^-8 of it at most) against it.  The other tokens' k there is 0.
+    big, low = q.clone(), k.clone()
+    big[0] = 0
+    big[0, 126] = 2.0 ** 64
+    low[:, 0, 126:] = 0
+    low[:min(n - 1, 100), 0, 126] = -2.0 ** 70
+    bo, bl = (x.reshape(Hq, -1) for x in decode(big, low))
+    live = n - min(n - 1, 100)
+    assert np.abs(bo[0] - v[-live:, 0].float().mean(0).numpy()).max() <= 2e-2
+    assert abs(bl[0, 0] - np.log(live)) <= 2e-3
+    assert c.device_status() == 0
+
+
 # (B, Hq, Hkv, N, D): clusters of 1, 4, 3, 8 and 8 CTAs per key tile on 148 SMs, with and without a mask
 @pytest.mark.parametrize("B,Hq,Hkv,N,D", [(1, 4, 4, 100, 64), (1, 8, 1, 130, 128), (1, 12, 1, 128, 64), (1, 32, 2, 600, 64),
                                           (1, 16, 1, 700, 128)])
