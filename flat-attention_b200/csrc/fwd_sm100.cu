@@ -513,12 +513,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
         auto load_q = [&](int w) {
             if ((w ? it.n_tiles[1] : it.n_tiles[0]) == 0 || !ok) return;
             // the slot is free once every S MMA of its previous tile has completed
-            if (q_loads[w] > 0 && !mbar_wait(q_empty(w), (q_loads[w] - 1) & 1, abort_flag)) {
+            if (q_loads[w] > 0 && !mbar_wait_warp(q_empty(w), (q_loads[w] - 1) & 1, abort_flag)) {
                 if (lane == 0) record_timeout(p, 110 + w);
                 ok = false;
+                return;
             }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) return;
             ++q_loads[w];
             if (lane == 0) {
                 mbar_expect_tx(q_full(w), C::kTileBytes);
@@ -532,12 +531,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             uint32_t &cnt = is_k ? k_cnt : v_cnt;
             const int s = cnt % C::kStages;
             const uint32_t phase = (cnt / C::kStages) & 1;
-            if (!mbar_wait(is_k ? k_empty(s) : v_empty(s), phase ^ 1, abort_flag)) {
+            if (!mbar_wait_warp(is_k ? k_empty(s) : v_empty(s), phase ^ 1, abort_flag)) {
                 if (lane == 0) record_timeout(p, 100 + s);
                 ok = false;
+                return;
             }
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) return;
             ++cnt;
             const CUtensorMap *map = is_k ? &p.map_k : &p.map_v;
             const uint32_t dst = smem_u32((is_k ? k_s : v_s) + s * C::kTileBytes);
@@ -729,7 +727,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             const int n_max = max(it.n_tiles[0], it.n_tiles[1]);
             for (int j = 0; ok && j < n_max; ++j, ++ring) {
                 const int s = ring % C::kStages;
-                if (!mbar_wait(k_full(s), (ring / C::kStages) & 1, abort_flag)) {
+                if (!mbar_wait_warp(k_full(s), (ring / C::kStages) & 1, abort_flag)) {
                     record_timeout(p, 400 + s);
                     ok = false;
                     break;
@@ -794,7 +792,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                             // The tile before has been rotated: only then does the parity of q_full tell this tile's arrival
                             // (the first one is the softmax warps', and may be gone by the time these look).
                             const uint32_t parity = (phases >> w) & 1;
-                            if (!mbar_wait(q_ready(w), parity ^ 1, abort_flag) || !mbar_wait(q_full(w), parity, abort_flag)) {
+                            if (!mbar_wait_warp(q_ready(w), parity ^ 1, abort_flag) || !mbar_wait_warp(q_full(w), parity, abort_flag)) {
                                 record_timeout(p, 290 + w);
                                 ok = false;
                             }
@@ -813,13 +811,11 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                 const bool run = (w ? it.n_tiles[1] : it.n_tiles[0]) > 0;
                 if (run) {
                     const uint32_t parity = (phases >> (2 + w)) & 1;
-                    const bool got = mbar_wait(ml_full(w), parity, abort_flag) && mbar_wait(o_final(w), parity, abort_flag);
-                    if (!got) {
+                    if (!mbar_wait_warp(ml_full(w), parity, abort_flag) || !mbar_wait_warp(o_final(w), parity, abort_flag)) {
                         record_timeout(p, 310 + w);
                         ok = false;
+                        break;
                     }
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
                     phases ^= 4u << w;
                     tc_fence_after();
                     const float2 ml = ml_s[w * kTileRows + row_in_tile];
@@ -928,7 +924,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             const int n = w ? it.n_tiles[1] : it.n_tiles[0];
             if (n <= 0) continue;
             if (done == 0 && p.rope_q_table) {  // the slot's first Q tile
-                if (!mbar_wait(q_full(w), 0, abort_flag)) {
+                if (!mbar_wait_warp(q_full(w), 0, abort_flag)) {
                     record_timeout(p, 280 + w);
                     ok = false;
                 } else {
@@ -962,7 +958,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             // registers.  O in TMEM is rescaled only when the running max grew by more than 2^8.
             TRACE_LOCAL;
             for (int j = 0; ok && j < n; ++j) {
-                if (!mbar_wait(s_full(w), tiles & 1, abort_flag)) {
+                if (!mbar_wait_warp(s_full(w), tiles & 1, abort_flag)) {
                     record_timeout(p, 300 + w);
                     ok = false;
                     break;
@@ -1031,7 +1027,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
                     m = m_cand;
                 }
                 // P and O belong to the slot's previous value product until it is done
-                if (tiles > 0 && !mbar_wait(pv_done(w), (tiles - 1) & 1, abort_flag)) {
+                if (tiles > 0 && !mbar_wait_warp(pv_done(w), (tiles - 1) & 1, abort_flag)) {
                     record_timeout(p, 320 + w);
                     ok = false;
                 }
@@ -1115,7 +1111,7 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
             if (lane == 0) TRACE_FLUSH(warp, n - 1);
             if (!ok) break;
             // (max, sum) of the item's rows for the warps that store it, which have read those of the item before
-            if (done > 0 && !mbar_wait(o_free(w), (done - 1) & 1, abort_flag)) {
+            if (done > 0 && !mbar_wait_warp(o_free(w), (done - 1) & 1, abort_flag)) {
                 record_timeout(p, 330 + w);
                 ok = false;
                 break;

@@ -82,14 +82,22 @@ __device__ __forceinline__ bool mbar_try_wait_suspend(uint32_t bar, uint32_t par
 // leaves its loop, so the kernel always terminates and the context stays usable.
 constexpr uint32_t kWaitCycles = 2000000000u;  // about one second (32-bit cycle counter, wrap-safe difference)
 constexpr uint32_t kSuspendNs = 20000;         // one suspended poll lasts at most 20 us
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
-    if (mbar_try_wait(bar, parity)) return true;
+__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     const uint32_t start = (uint32_t)clock();
     do {
         if (mbar_try_wait_suspend(bar, parity, kSuspendNs)) return true;
     } while (*abort_flag == 0 && (uint32_t)clock() - start <= kWaitCycles);
     *abort_flag = 1;
     return false;
+}
+// For a thread on its own.
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, abort_flag);
+}
+// For a whole warp, all of whose lanes get the same answer: one lane may see the phase, or the abort flag, when another does
+// not, and a warp of which a part leaves its loop hangs at the next instruction that takes all of it (tcgen05.ld, __syncwarp).
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, abort_flag));
 }
 
 // ---- TMA -------------------------------------------------------------------------------------

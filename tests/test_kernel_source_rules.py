@@ -65,3 +65,32 @@ def test_dependent_kernels_do_not_read_through_the_read_only_path(file, kernel):
         header, body = found[name]
         assert not re.search(r"\.nc\b|__ldg\s*\(", body), name
         assert not re.search(r"const\s+[\w:]+\s*\*\s*__restrict__", header), name
+
+
+def enclosing_conditions(body, at):
+    """The text in front of each block that is open at position `at`, outermost first."""
+    stack, last = [], 0
+    for i, ch in enumerate(body[:at]):
+        if ch == "{":
+            stack.append(body[last:i])
+        elif ch == "}":
+            stack.pop()
+        if ch in "{};":
+            last = i + 1
+    return stack
+
+
+@pytest.mark.parametrize("file,kernel", [("fwd_sm100.cu", "fwd_sm100_kernel")])
+def test_warps_leave_a_wait_that_gave_up_as_a_whole(file, kernel):
+    """mbar_wait answers each lane for itself; warps whose lanes all wait take mbar_wait_warp, which answers them alike."""
+    body = sources()[file][kernel][1]
+    calls = list(re.finditer(r"\bmbar_(?:wait|wait_warp)\(", body))
+    assert calls
+    for call in calls:
+        one_thread = any("elect_one()" in condition for condition in enclosing_conditions(body, call.start()))
+        assert one_thread == (call.group() == "mbar_wait("), body[call.start() - 80:call.end() + 60]
+
+
+def test_the_warp_wide_wait_answers_every_lane_alike():
+    body = sources()["fwd_sm100.cu"]["mbar_wait_warp"][1]
+    assert all(part.strip().startswith("__all_sync(0xffffffffu,") for part in body[body.index("return") + 6:].split("||"))
