@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
         for (int it = 0; ok && it < n_iter; ++it) {
             const int s = it % C::kStages;
             const uint8_t *stage = ring + s * C::kStageBytes;
-            if (!mbar_wait(rg_full(s), (it / C::kStages) & 1, abort_flag)) {  // LSE / delta of this stage
+            if (!mbar_wait_warp(rg_full(s), (it / C::kStages) & 1, abort_flag)) {  // LSE / delta of this stage
                 timeout(p, 300);
                 ok = false;
                 break;
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
             const int t = first + (it0 + it) % per_head;
             const bool diag = p.causal && t == t_own;
             // ---- phase 1: P^T ----
-            if (!mbar_wait(x_full, it & 1, abort_flag)) {
+            if (!mbar_wait_warp(x_full, it & 1, abort_flag)) {
                 timeout(p, 310);
                 ok = false;
                 break;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
             if (lane == 0) mbar_arrive(p_ready);
             if (warp == 0 && lane == 0 && it < 16) TRS(it, 6);
             // ---- phase 2: dS^T ----
-            if (!mbar_wait(y_full, it & 1, abort_flag)) {
+            if (!mbar_wait_warp(y_full, it & 1, abort_flag)) {
                 timeout(p, 315);
                 ok = false;
                 break;
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
                 if constexpr (SPILL) {
                     // ... and into the staging tile of the spill: row = key, this warp group's 64 queries = 128 bytes of box
                     // `half`, 16-byte chunks swizzled by the row (the layout the dQ kernel's MMAs read it back in)
-                    if (!mbar_wait(ds_free, (it & 1) ^ 1, abort_flag)) {  // the previous tile's store has read the space
+                    if (!mbar_wait_warp(ds_free, (it & 1) ^ 1, abort_flag)) {  // the previous tile's store has read the space
                         timeout(p, 317);
                         ok = false;
                         break;
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_sm100_kernel(const __grid_con
             if (SPILL && lane == 0) mbar_arrive(ds_staged);
             if (warp == 0 && lane == 0 && it < 16) TRS(it, 7);
         }
-        if (ok && n_iter > 0 && !mbar_wait(acc_final, 0, abort_flag)) {
+        if (ok && n_iter > 0 && !mbar_wait_warp(acc_final, 0, abort_flag)) {
             timeout(p, 320);
             ok = false;
         }
@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
 
         // Q rows from the swizzled TMA tile into TMEM: lane = row, 32-bit column c holds elements 2c, 2c + 1 (the
         // layout of an A operand); warp group `half` copies the 64-element box `half`
-        if (!mbar_wait(st_full, 0, abort_flag)) {
+        if (!mbar_wait_warp(st_full, 0, abort_flag)) {
             timeout(p, 290);
             ok = false;
         }
@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
         }
         const uint32_t t_x = t_lane + kColX + half * 64, t_y = t_lane + kColY + half * 64;
         for (int it = 0; ok && it < n_iter; ++it) {
-            if (!mbar_wait(xy_full, it & 1, abort_flag)) {
+            if (!mbar_wait_warp(xy_full, it & 1, abort_flag)) {
                 timeout(p, 310);
                 ok = false;
                 break;
@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
                 ds[i >> 1] = *reinterpret_cast<const uint32_t *>(&dsb);
             }
             if (warp == 0 && lane == 0) TRACE(0, it, 2);
-            if (it > 0 && !mbar_wait(ds_free, (it - 1) & 1, abort_flag)) {  // the dQ MMAs of the previous tile read dS
+            if (it > 0 && !mbar_wait_warp(ds_free, (it - 1) & 1, abort_flag)) {  // the dQ MMAs of the previous tile read dS
                 timeout(p, 315);
                 ok = false;
                 break;
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
             if (lane == 0) mbar_arrive(ds_full);
             if (warp == 0 && lane == 0) TRACE(0, it, 3);
         }
-        if (ok && !mbar_wait(acc_final, 0, abort_flag)) {
+        if (ok && !mbar_wait_warp(acc_final, 0, abort_flag)) {
             timeout(p, 320);
             ok = false;
         }
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(DqSpillCfg<D, HEADS>::kThreadsDq, 1) bwd_dq_sp
     } else if (warp < 4) {
         // ================= epilogue =================
         const int row_local = warp * 32 + lane;  // TMEM lane = query row
-        if (mbar_wait(acc_final, 0, abort_flag)) {
+        if (mbar_wait_warp(acc_final, 0, abort_flag)) {
             tc_fence_after();
             const bool store = t_own * kTile + row_local < p.seq_len;
             const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);

@@ -80,7 +80,8 @@ def enclosing_conditions(body, at):
     return stack
 
 
-@pytest.mark.parametrize("file,kernel", [("fwd_sm100.cu", "fwd_sm100_kernel")])
+@pytest.mark.parametrize("file,kernel", [("fwd_sm100.cu", "fwd_sm100_kernel"), ("bwd_sm100.cu", "bwd_sm100_kernel"),
+                                         ("bwd_sm100.cu", "bwd_dq_sm100_kernel"), ("bwd_sm100.cu", "bwd_dq_spill_kernel")])
 def test_warps_leave_a_wait_that_gave_up_as_a_whole(file, kernel):
     """mbar_wait answers each lane for itself; warps whose lanes all wait take mbar_wait_warp, which answers them alike."""
     body = sources()[file][kernel][1]
