@@ -630,8 +630,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_dq_sm100_kernel(const __grid_
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dependency_launch();  // the next call's first kernel, behind this CTA's TMEM allocation
     grid_dependency_wait();
+    grid_dependency_launch();  // the next call's first kernel, behind this CTA's TMEM allocation
     constexpr uint32_t kColQ = 0, kColX = 64, kColY = 192, kColDS = 320, kColAcc = 384;
 
     if (warp >= 8) {
@@ -925,8 +925,8 @@ __global__ void __launch_bounds__(DqSpillCfg<D, HEADS>::kThreadsDq, 1) bwd_dq_sp
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    grid_dependency_launch();  // the next call's first kernel, behind this CTA's TMEM allocation
     grid_dependency_wait();
+    grid_dependency_launch();  // the next call's first kernel, behind this CTA's TMEM allocation
 
     if (warp == 4 && !*abort_flag && elect_one()) {
         // ================= producer =================

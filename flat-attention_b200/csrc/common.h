@@ -125,10 +125,10 @@ inline char *scratch_ptr(flat_ctx *ctx) { return static_cast<char *>(ctx->worksp
             return ::flat::fail((ctx), FLAT_ERR_EXECUTION, "%s: %s", #expr, cudaGetErrorString(e__)); \
     } while (0)
 
-// A kernel launched so that it may start while the kernel before it in the stream (one of this library's, launched by the
-// same call) is still running: it must execute grid_dependency_wait() before it reads what that kernel writes, and the
-// other one tells when its dependent may start with grid_dependency_launch().  Between two short kernels this hides
-// the launch and the second one's set-up.
+// A kernel launched so that it may start while the kernel before it in the stream is still running: it must execute
+// grid_dependency_wait() before it reads what that kernel writes.  That one tells when its dependent may start with
+// grid_dependency_launch(); without it the dependent comes in as its blocks end.  Between two short kernels this hides the
+// launch and the second one's set-up.
 template <typename... P, typename... A>
 inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
                                     A &&...args) {
@@ -144,12 +144,14 @@ inline cudaError_t launch_dependent(bool dependent, void (*kernel)(P...), dim3 g
     cfg.numAttrs = dependent ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
-// Whether the first kernel of a call may be launched the same way, behind whatever kernel is before it in the stream: the end
-// of one call and the launch and set-up of the next then overlap.  Such a kernel waits (grid_dependency_wait()) before its
-// first access to memory, and a kernel that lets its dependents start before its own wait has only dependents that do the
-// same: what a call reads is complete when it reads it.  It may have been written while the kernel was already resident, so
-// no dependent kernel reads through the read-only path (.nc, __ldg, const __restrict__).  Not while the stream is captured,
-// where the kernel before may be a node of any kind.
+// Whether the first kernel of a call may be launched the same way, behind whatever kernel is before it in the stream, another
+// call's or the application's: the end of one call and the launch and set-up of the next then overlap.  Such a kernel waits
+// before its first access to memory.  The last kernel of a call lets its dependent start behind its own wait only: the
+// dependent may be the application's, and what that does before it waits has always been able to count on whatever came
+// before the kernel in front of it.  (A kernel inside a call whose dependent is this library's may let it start earlier, see
+// bwd_sm100_kernel.)  What a dependent kernel reads is complete when it reads it, but it may have been written while the kernel
+// was already resident, so none reads through the read-only path (.nc, __ldg, const __restrict__).  Not while the stream is
+// captured, where the kernel before may be a node of any kind.
 inline bool may_overlap_previous(flat_ctx *ctx) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess) {

@@ -337,8 +337,8 @@ __global__ void __launch_bounds__(32 * WARPS) merge_row_kernel(int parts, int he
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t row = blockIdx.x;
     int live = parts;
-    grid_dependency_launch();
     grid_dependency_wait();
+    grid_dependency_launch();
     if (seq_offsets) {
         const int seq = (int)(row / rows_per_seq);
         live = (seq_offsets[seq + 1] - 1) / span_tokens - seq_offsets[seq] / span_tokens + 1;

@@ -333,8 +333,8 @@ __global__ void __launch_bounds__(32 * kClusterWarps, 1)
     __shared__ float2 part_ml[kClusterWarps][8];
     __shared__ __align__(16) float cta_o[8 * D];
     __shared__ float2 cta_ml[8];
-    grid_dependency_launch();
     grid_dependency_wait();
+    grid_dependency_launch();
     cg::cluster_group cluster = cg::this_cluster();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, c = lane & 3;

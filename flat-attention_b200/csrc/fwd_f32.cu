@@ -28,7 +28,8 @@ constexpr int kRows = 64;    // query rows per CTA
 constexpr int kKeys = 64;    // keys per tile
 // tx: lanes that share a row.  Twice the threads with half the tile each hide more of the shared-memory latency at D = 128 (8 / 2
 // heads: 356 rows 41.3 -> 37.0 us, 512 rows 45.1 -> 43.6, 2 x 2048 rows, 16 / 4 heads 1207 both); at D = 64 a read then serves too
-// few multiply-adds (1784 rows 164 -> 166 us, 2 x 2048 rows without a mask 1049 -> 1068).
+// few multiply-adds (1784 rows 164 -> 166 us, 2 x 2048 rows without a mask 1049 -> 1068).  The 128 registers of the 256 threads
+// do not hold all of it: 80 bytes of a thread spill, 64 with ALiBi.
 template <int D> constexpr int kLanes = D == 128 ? 16 : 8;
 template <int D> constexpr int kThreads = kRows / 4 * kLanes<D>;
 constexpr int kRowsPerThread = 4;   // ty + 16 r
@@ -159,8 +160,8 @@ __global__ void __launch_bounds__(kThreads<D>, 2) fwd_f32_kernel(const __grid_co
     using T = Tile<D>;
     constexpr int kCols = D / (4 * kLanes<D>);  // float4 columns of O per thread and row
     const FwdParams &p = fp.f;
-    grid_dependency_launch();
     grid_dependency_wait();
+    grid_dependency_launch();
     extern __shared__ __align__(16) float smem[];
     float *qs = smem + T::kQ, *ks = smem + T::kK, *vs = smem + T::kV, *stat = smem + T::kStat;
     float *ps = ks;
@@ -446,7 +447,7 @@ bool holds(const flat_ctx::RopeTable &t, const FwdParams &p, int64_t first, int6
 
 // The (cos, sin) tables of a call.  Those of the tensor-core kernels are read where they hold the positions, and never
 // written; else the context's table of this mode is made to hold one range with the positions of Q and of K, unless it does.
-// Without a table the kernel evaluates the same angles itself, for every tile again (512 rows 61 us instead of 45): under
+// Without a table the kernel evaluates the same angles itself, for every tile again (512 rows 47 us instead of 42): under
 // stream capture, where a replay would read what later calls have put there, beyond kF32TableBytes, and where the context
 // got no memory.
 void find_tables(flat_ctx *ctx, F32Params *fp) {

@@ -21,12 +21,12 @@
 // and 195 us.
 // The softmax warps hold a whole score row (128 registers) and must not spill: a spilled register is a store that the next
 // mbarrier arrival has to wait for (the period of a tile pair went from 4.7k to 3.4k clk when the spills went).  The code is
-// kept small for the same reason: ten warps run five different loops, and 86 KB of instructions missed the instruction
+// kept small for the same reason: 15 or 16 warps run five different loops, and 86 KB of instructions missed the instruction
 // cache 78 times per tile pair.
 //
 // RoPE: Q is rotated inside this kernel.  The raw bf16 Q tile lands in shared memory by TMA, the
-// softmax thread that owns a row rotates it in place with a (cos, sin) table of the call's
-// positions and hands the tile to the MMA warp; rotated operands are stored as fp16, which keeps
+// storing warps (a slot's first tile: its softmax warps) rotate it in place, 16-byte chunks of whole rows at a time, with a
+// (cos, sin) table of the call's positions and hand it to the issuing thread; rotated operands are stored as fp16, which keeps
 // their rounding eight times smaller than bf16 would (the 2e-3 LSE tolerance needs that).  K is
 // rotated once per call by a small prologue kernel into fp16 scratch (every K tile is read by
 // many CTAs, so rotating it in-kernel would repeat the work 32 times).  When the cache already
@@ -433,8 +433,13 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
 
     const int warp = warp_index_uniform();
     const int lane = threadIdx.x & 31;
-    grid_dependency_launch();  // the merge kernel, or the next call's first
 
+    // The merge kernel, or the first of the next call, may come in once whatever was before this call is complete: behind this
+    // kernel's wait, or, behind a K rotation, which lets nothing start early, at once.  Both stand here and not behind the set-up
+    // below: with the trigger there, or in one warp, some instantiations come out 2 to 3% slower (D = 64, 2 x 1000 rows, 3000
+    // keys, 32 / 8 heads: 72.9 us, 74.3 behind the set-up, 75.5 in the producer warp; K converted 78.7, 80.1, 81.2).
+    if (p.first_in_call) grid_dependency_wait();
+    grid_dependency_launch();
     if (warp == kProducerWarp && lane == 0) {
         *abort_flag = 0;
         for (int w = 0; w < 2; ++w) {
@@ -480,7 +485,6 @@ __global__ void __launch_bounds__(kThreads, 1) fwd_sm100_kernel(const __grid_con
         tmem_alloc(smem_u32(tmem_slot), 512);
         tmem_relinquish();
     }
-    if (p.first_in_call) grid_dependency_wait();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -1162,8 +1166,8 @@ template <int D, bool F16IO>
 __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const __grid_constant__ KernelParams p, int first_lin) {
     constexpr int kCols = D / 32;
     constexpr int kRowsPerCta = 2 * kTileRows / kMergeCtasPerItem;
-    grid_dependency_launch();
     grid_dependency_wait();
+    grid_dependency_launch();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int item = blockIdx.x / kMergeCtasPerItem;
     const int lin = first_lin + item;

@@ -67,6 +67,18 @@ def test_dependent_kernels_do_not_read_through_the_read_only_path(file, kernel):
         assert not re.search(r"const\s+[\w:]+\s*\*\s*__restrict__", header), name
 
 
+# bwd_sm100_kernel is never the last of its call: its dependent is the dQ kernel, which waits before it touches memory
+@pytest.mark.parametrize("file,kernel", [x for x in KERNELS if x[1] != "bwd_sm100_kernel"])
+def test_the_last_kernel_of_a_call_lets_its_dependent_start_behind_its_own_wait(file, kernel):
+    """The dependent may be the application's: what it does before it waits may count on everything before this kernel.  (The
+    forward behind its K rotation does not wait first: the rotation lets nothing start before its blocks, which wait, have ended.)"""
+    body = sources()[file][kernel][1]
+    for launch in re.finditer(r"grid_dependency_launch\(\)", body):
+        assert re.search(r"grid_dependency_wait\(\);\s*$", body[:launch.start()]), body[:launch.start()][-200:]
+    if kernel == "rotate_to_f16_kernel":
+        assert "grid_dependency_launch" not in body
+
+
 def enclosing_conditions(body, at):
     """The text in front of each block that is open at position `at`, outermost first."""
     stack, last = [], 0
