@@ -13,18 +13,23 @@ from tests.test_gpu_decode_cache import oracle_decode, run_batched, unpack
 pytestmark = pytest.mark.gpu
 
 
-# tokens: one span of one tile, its edges, the largest table that travels with the launch (256 pages) and one page more
-@pytest.mark.parametrize("n", [1, 15, 16, 17, 33, 256 * 16, 256 * 16 + 1])
-@pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 64), (32, 8, 128)])
-def test_paged_decode_spans_and_tables(n, Hq, Hkv, D):
-    c, page = ctx(), 16
+# tokens and page size: clusters around one tile and at their longest (4096 tokens, 256 pages, the largest table that travels
+# with the launch); spans with a table in memory, and with one that travels: longer contexts in larger pages, more KV heads than
+# clusters take
+@pytest.mark.parametrize("n,page", [(1, 16), (15, 16), (16, 16), (17, 16), (33, 16), (256 * 16, 16), (256 * 16 + 1, 16), (4097, 32),
+                                    (8192, 32), (8193, 32), (6145, 64)])
+@pytest.mark.parametrize("Hq,Hkv,D", [(8, 2, 64), (32, 8, 128), (16, 16, 128)])
+def test_paged_decode_spans_and_tables(n, page, Hq, Hkv, D):
+    c = ctx()
     cache = fa.CudaPagedKvCache(c, fa.BF16, page, (n + page - 1) // page + 1, Hkv, D)
     g = torch.Generator().manual_seed(n)
     k, v, q = (torch.randn(r * D, generator=g).bfloat16() for r in (n * Hkv, n * Hkv, Hq))
     cache.record_append(k.cuda(), v.cuda(), n)
     out = c.create_decode_output_buffer(fa.BF16, 1, Hq, D)
     out.fill_(0x7f)
+    before = c.launch_count()
     c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, n - 1, q.cuda(), cache.k_buffer(), cache.v_buffer(), out)
+    assert c.launch_count() - before == (1 if n <= (2048 if Hkv == 16 else 4096) else 2)  # a cluster, or spans and a merge
     o, l = unpack(out, fa.BF16, Hq, D)
     eo, el = oracle_decode(q.float().numpy(), k.float().numpy().reshape(n, -1), v.float().numpy().reshape(n, -1), Hq, Hkv, D, 5e5,
                            n - 1, 0, True)
@@ -35,8 +40,8 @@ def test_paged_decode_spans_and_tables(n, Hq, Hkv, D):
 
 # lengths of the batch: single sequences on either side of the span rule, a full batch of short ones, and one long among many
 # short ones, whose parts (dense over all sequences) would take four times the memory with spans of 16 tokens
-@pytest.mark.parametrize("lens", [[700], [2048], [2064], [6000], [8000], [700] * 16, [100] * 128, [2048] + [16] * 11,
-                                  [2048] + [16] * 127])
+@pytest.mark.parametrize("lens", [[4097], [6144], [6145], [6000], [8000], [700] * 16, [700] * 20, [100] * 128, [2048] + [16] * 18,
+                                  [2048] + [16] * 127, [2064] + [16] * 18])
 def test_decode_asks_for_no_more_workspace_than_spans_of_64(lens):
     """Shorter spans keep their parts in memory of the context: the workspace is bounded by the parts of 64-token spans."""
     Hq, Hkv, D, page, c = 32, 8, 128, 16, fa.Context(0)
@@ -49,6 +54,7 @@ def test_decode_asks_for_no_more_workspace_than_spans_of_64(lens):
         tables[i, :n] = sum(pages[:i]) + np.arange(n)
     args = (fa.BF16, np.array(lens, np.int32), tables, sum(pages), max(pages), Q, K, V, Hq, Hkv, D, page, 5e5)
     o, l = run_batched(c, *args)
+    assert c.launch_count() == 2  # spans and a merge, not a cluster
     padded = [-(-n // 16) * 16 for n in lens]
     span = max(64, (-(-sum(padded) // (2 * 148)) + 15) // 16 * 16)
     parts = -(-max(padded) // span) + 1
@@ -83,6 +89,40 @@ def test_decode_clusters(lens, Hq, Hkv, D):
     assert c.device_status() == 0
 
 
+@pytest.mark.parametrize("lens,at", [([40], [(0, 1)]), ([40, 16], [(1, 0)]), ([900, 700], [(0, 0), (0, 40), (1, 43)])])
+def test_decode_clusters_skip_pages_outside_the_pool(lens, at):
+    """Entries of the device's page table that are outside the pool are not read: their tokens count for nothing, a sequence
+    without any other gets O = 0 and LSE = -inf, and the call is flagged."""
+    Hq, Hkv, D, page, c = 8, 2, 64, 16, ctx()
+    pages = [-(-n // page) for n in lens]
+    g = torch.Generator().manual_seed(11)
+    Q = torch.randn(len(lens), Hq * D, generator=g).bfloat16()
+    K, V = (torch.randn(sum(pages) * page, Hkv * D, generator=g).bfloat16() for _ in range(2))
+    tables = np.zeros((len(lens), max(pages)), np.int32)
+    for i, n in enumerate(pages):
+        tables[i, :n] = sum(pages[:i]) + np.arange(n)
+    broken, qpos = tables.copy(), np.array(lens, np.int32) - 1
+    for k, (s, i) in enumerate(at):
+        broken[s, i] = -1 if k % 2 else sum(pages) + 1000
+    out = c.create_decode_output_buffer(fa.BF16, len(lens), Hq, D)
+    before = c.launch_count()
+    c.decode_paged_batched(fa.BF16, len(lens), Hq, Hkv, D, page, sum(pages), max(pages), *(torch.from_numpy(x).cuda() for x in
+                           (broken, np.array(lens, np.int32), qpos)), tables, np.array(lens, np.int32), qpos, fa.config(True), 5e5,
+                           Q.cuda(), K.cuda(), V.cuda(), out)
+    assert c.launch_count() - before == 1
+    assert c.device_status() == 35  # FLAT_ERR_PAGE_OUT_OF_RANGE, cleared by the read
+    o, l = unpack(out, fa.BF16, len(lens) * Hq, D)
+    o, l = o.reshape(len(lens), Hq, D), l.reshape(len(lens), Hq)
+    for s, n in enumerate(lens):
+        rows = [tables[s, t // page] * page + t % page for t in range(n) if (s, t // page) not in at]
+        if not rows:
+            assert not o[s].any() and np.isneginf(l[s]).all()
+            continue
+        eo, el = oracle_decode(Q[s].float().numpy(), K.float().numpy()[rows], V.float().numpy()[rows], Hq, Hkv, D, 5e5, n - 1, 0, True)
+        assert np.abs(o[s].reshape(-1) - eo.reshape(-1)).max() <= 2e-2
+        assert np.abs(l[s].reshape(-1) - el.reshape(-1)).max() <= 2e-3
+
+
 # tokens: clusters of one CTA and of eight (one tile per warp, several), and spans with a merge
 @pytest.mark.parametrize("n", [10, 40, 700, 4096, 6000])
 def test_decode_of_scores_that_are_not_finite(n):
@@ -101,7 +141,7 @@ def test_decode_of_scores_that_are_not_finite(n):
         before = c.launch_count()
         c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, n - 1, q.reshape(-1).cuda(), cache.k_buffer(),
                        cache.v_buffer(), out)
-        assert c.launch_count() - before == (1 if n <= 4096 else 2)
+        assert c.launch_count() - before == (1 if n <= 4096 else 2)  # a cluster, or spans and a merge
         return unpack(out, fa.BF16, Hq, D)
 
     o, l = (x.reshape(Hq, -1) for x in decode(q, k))
@@ -215,14 +255,16 @@ def test_padded_batches_around_the_lengths_that_travel_with_the_launch(S, dtype)
     lens = rng.integers(1, N + 1, S)
     lens[0], lens[-1] = N, 33
     seqs = [fa.VarlenSequence(int(n), int(n), 0, int(rng.integers(0, 3000))) for n in lens]
-    cache = fa.CudaPagedKvCache(c, fa.BF16, 16, 40, Hkv, D)
-    kv = torch.randn(2, 600 * Hkv * D, generator=torch.Generator().manual_seed(S)).bfloat16().cuda()
-    cache.record_append(kv[0], kv[1], 600)
+    cache = fa.CudaPagedKvCache(c, fa.BF16, 32, 160, Hkv, D)
+    kv = torch.randn(2, 5000 * Hkv * D, generator=torch.Generator().manual_seed(S)).bfloat16().cuda()
+    cache.record_append(kv[0], kv[1], 5000)
     dq, decoded = dev(randn(Hq * D, 70), torch.bfloat16), []
 
     def decode():
         out = c.create_decode_output_buffer(fa.BF16, 1, Hq, D)
-        c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, 599, dq, cache.k_buffer(), cache.v_buffer(), out)
+        before = c.launch_count()
+        c.decode_paged(fa.BF16, cache.table(), Hq, Hkv, D, fa.config(True), 5e5, 4999, dq, cache.k_buffer(), cache.v_buffer(), out)
+        assert c.launch_count() - before == 2  # spans, whose plan lies in the workspace, and a merge
         decoded.append(out)
 
     shp, rot = fa.shape(S, Hq, Hkv, N, N, D), fa.rotary(5e5, 0)
