@@ -145,31 +145,9 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// D[tmem] (+)= A[smem] * B[smem]
-__device__ __forceinline__ void mma_ss(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n"
-        ".reg .pred p;\n"
-        "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n"
-        "}\n" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// The same with descriptor = base + offset formed inside the asm block (offset in 16-byte units, added to the
-// start-address field): an unrolled issue sequence then keeps only the base descriptors in registers.
+// D[tmem] (+)= A[smem] * B[smem] and A[tmem] * B[smem].  A descriptor is base + offset, formed inside the asm block (offset in
+// 16-byte units, added to the start-address field): an unrolled issue sequence then keeps only the base descriptors in
+// registers.
 __device__ __forceinline__ void mma_ss_off(uint32_t d_tmem, uint64_t a_base, uint64_t b_base, uint32_t off16, uint32_t idesc,
                                            uint32_t accumulate) {
     asm volatile(
