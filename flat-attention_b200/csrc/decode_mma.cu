@@ -486,9 +486,10 @@ bool decode_mma_supported(int dtype, const DecodeParams &p) {
 // CTAs per KV head for a batch whose longest context has `max_len` tokens, or 0: the spans of decode_mma_kernel.  One tile per
 // warp where the CTAs suffice, up to kClusterTiles; all clusters have to be resident at once, which with one CTA per SM more
 // than eight of the largest are not (16 KV heads, 1000 tokens: 12.3 us with 16 clusters of eight, 10.3 with spans and a merge).
-// Spans and merge / cluster, D = 128, 32 / 8 heads: 700 tokens 10.3 / 8.2 us, 2000 12.3 / 10.3, 4096 14.4 / 13.3; 64 / 8 heads,
-// 300 10.3 / 9.0, 3500 14.4 / 14.3; 16 / 16 heads, 400 10.3 / 8.2; four sequences of up to 1500 tokens 17.5 / 14.8, 16 of up
-// to 500 20.4 / 15.0; D = 64, 16 / 4 heads, 300 9.0 / 7.0, 4096 10.2 / 10.3.
+// Spans and merge / cluster, launches not yet overlapped (common.h), D = 128, 32 / 8 heads: 700 tokens 10.3 / 8.2 us, 2000
+// 12.3 / 10.3, 4096 14.4 / 13.3 (overlapped 6.7, 8.0 and 10.4); 64 / 8 heads, 300 10.3 / 9.0, 3500 14.4 / 14.3; 16 / 16 heads,
+// 400 10.3 / 8.2; four sequences of up to 1500 tokens 17.5 / 14.8, 16 of up to 500 20.4 / 15.0; D = 64, 16 / 4 heads, 300 9.0 /
+// 7.0, 4096 10.2 / 10.3.
 int decode_cluster_size(const flat_ctx *ctx, const DecodeParams &p, int max_len) {
     if (p.kv_heads > 65535 || p.num_seqs > 65535 || max_len < 1) return 0;
     const int tiles = (max_len + 15) / 16;

@@ -416,8 +416,9 @@ int launch(flat_ctx *ctx, const F32Params &fp, int parts) {
 
 // CTAs per query block.  A CTA costs its tiles and about kOverheadTiles more (its Q rows, its share of the combination); the
 // call lasts as long as its longest CTA, and as long as everything takes over the CTAs that run at once (two per SM).
-// The cluster size with the smaller of the two maxima is taken.  8 heads, D = 128, causal: 512 rows 45 us with 4 CTAs (49
-// with 8, 57 us before loads were batched), 1024 rows 118 us with 4 (131 with 2), 2048 rows 400 us with 2 (472 with 1).
+// The cluster size with the smaller of the two maxima is taken.  An overhead of 1 / 2 / 3 tiles, 8 / 2 heads, causal: D = 128,
+// 512 rows 48.0 / 42.0 / 42.0 us, 768 77.9 / 77.8 / 78.1, 1024 119.6 / 119.7 / 119.2, 2048 356 / 377 / 379; D = 64, 512 rows
+// 28.8 / 24.5 / 24.5, 1024 68.4 / 68.6 / 68.4, 1784 164 / 164 / 172.
 constexpr int kOverheadTiles = 2;
 int cluster_parts(const flat_ctx *ctx, const FwdParams &p) {
     const int64_t blocks = (p.q_len + kRows - 1) / kRows;

@@ -66,13 +66,13 @@ constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // log2 domain
 // At D = 64 the two products of a score cost the tensor pipe half of what they do at D = 128, and the exponent pass (16
 // exponentials per clock and SM of the special-function unit) is the longest part of the chain of a tile: every kPolyEvery-th
-// pair of scores takes 2^t from the FMA and integer pipes instead.  binary16, 8 x 1500 rows, 16 heads, no mask: 135.4 us
-// without, 130.9 us with every 4th pair (133 us with every 8th, 138 us with 3 of 8); masked calls are within 1.5% of each
-// other (4 x 2000 rows 77.0 and 78.1 us, 8000 rows 387 us both, the training step of 2 x 1000 rows 66.1 and 65.7 us).  At D =
-// 128 it costs time (a 32768-token chunked prefill 18.5 -> 19.5 ms), so the flag follows D; nor is it used where K is
-// converted in shared memory (CONVK): the converting warps need the same pipes (9774 tokens in chunks of 1024, 32 / 8 heads,
-// D = 64 979 -> 995 us), nor for K and V behind a page table (the same call with the binary16 shadow 964 -> 984 us) and for
-// padded batches, whose items are short (16 x 1024 rows, 32 / 8 heads 162 -> 165 us).
+// pair of scores takes 2^t from the FMA and integer pipes instead.  binary16, 16 heads, no mask, without and with every 4th
+// pair: 8 x 1000 rows 58.4 and 55.8 us, 4 x 1500 62.4 and 59.6, 2 x 1500 44.4 and 42.6, 8 x 1500 115.0 and 114.7; causal 16 / 4
+// heads: 8000 rows 172.7 and 170.7, 4 x 2000 56.5 and 57.1, the training step of 2 x 1000 rows 62.7 and 61.8.  Where it is left
+// out it cost time in the kernel that kept P over the scores: at D = 128 (a 32768-token chunked prefill 18.5 -> 19.5 ms), where
+// K is converted in shared memory (9774 tokens in chunks of 1024, 32 / 8 heads, D = 64 979 -> 995 us: the converting warps need
+// the same pipes), for K and V behind a page table (the same call with the binary16 shadow 964 -> 984 us) and for padded
+// batches, whose items are short (16 x 1024 rows, 32 / 8 heads 162 -> 165 us).
 constexpr int kPolyEvery = 4;
 
 __device__ __forceinline__ uint64_t pack2(float a, float b) {
@@ -1220,7 +1220,8 @@ __global__ void __launch_bounds__(256) fwd_split_merge_kernel(const __grid_const
 // kRotateHeads heads, whose loads are in flight together and share one read of the table (32 bytes per 16 of K), and the
 // grid's dimensions are the row and the head, so that no index is divided by a runtime number but the head.
 // The attention kernel behind it is brought in as its blocks end, not before: told to start earlier, its CTAs take SMs that
-// rotation blocks still wait for and come up in another order (604 -> 647 us for B = 4, N = 4096, 32 / 8 heads, D = 128).
+// rotation blocks still wait for and come up in another order (32 / 8 heads, D = 128: 16 padded prompts of 1024 rows 187 -> 210
+// us, B = 4, N = 4096 473 -> 487; it would gain where few CTAs run, 512 rows of 1500 keys 28.8 -> 27.1).
 constexpr int kRotateHeads = 4;
 template <int D, bool F16IN>
 __global__ void __launch_bounds__(256) rotate_to_f16_kernel(const uint16_t *x, __half *y, const float2 *table,
@@ -1380,9 +1381,11 @@ SplitPlan plan_split(int sm_count, const FwdParams &p) {
     }
     if (pl.rem_items == 0) return pl;
     int split = std::min(sm_count / pl.rem_items, 8);
-    // a part costs a Q load, a rotation, an epilogue of its own and a share of the merge launch (about 10 us together):
-    // it should keep at least kMinPartTiles KV tiles.  The last round holds the shortest items, the shortest of all is
-    // the first query block
+    // a part costs a Q load, a rotation, an epilogue of its own and a share of the merge launch: it should keep at least
+    // kMinPartTiles KV tiles.  With 16 / 8 / 4: binary16 encoder, 16 heads, D = 64, 8 x 1500 rows 114.7 / 115.0 / 120.7 us, 8 x
+    // 1000 55.8 / 55.8 / 65.7, 2 x 1500 42.6 / 42.5 / 46.3; 32 / 8 heads, D = 128, causal, 512 rows of 1500 keys 28.8 / 28.8 /
+    // 35.8, 1500 of 6000 132 / 129 / 129, 256 of 4096 48.7 / 42.2 / 42.2 (8 loses nowhere and gains there: not taken yet).
+    // The last round holds the shortest items, the shortest of all is the first query block
     long long visible = p.kv_len;
     if (p.causal) visible = std::min<long long>(p.kv_len, p.causal_off + std::min(p.q_len, 2 * kTileRows));
     const int n_min = (int)((visible + kTileRows - 1) / kTileRows);
