@@ -33,10 +33,10 @@ import time
 ROOT = os.path.dirname(os.path.abspath(__file__))
 
 # DRAM bytes (read + written) per launch of each leg's dominant kernel(s) on exactly the workloads timed below, taken from
-# one `ncu --set full` capture each; the summaries and their commands are under profiles/.  The profiler cannot run inside
+# one `ncu` capture each; the summaries and their commands are under profiles/.  The profiler cannot run inside
 # this script, so the figures are carried as constants and change only when a kernel changes.
 NCU_TRAFFIC = {
-    "forward": 311_873_792 + 111_970_304,  # fwd_sm100_kernel<128>, C2
+    "forward": 299_456_768 + 98_107_136,  # fwd_sm100_kernel<128>, C2
     "decode": 1_110_817_000 + 3_957_504,  # decode_mma_kernel<128>, C3
     # the 16 launches of fwd_sm100_kernel<128,paged,shadow> of one C4 sequence, summed (one ncu pass over a whole sequence)
     "chunked": 4196745216 + 500366592,

@@ -16,9 +16,9 @@
 // The N x N matrix never leaves TMEM.  Since P does not lie over S, the next scores are formed while the softmax warps work:
 // at D = 64 each slot has a score tile of its own, at D = 128 (512 columns: O 2 x 128, P 2 x 64, S 128) both slots take one
 // in turn, which also keeps them half a period apart.  While P lay over S a slot's chain was softmax, value product, next
-// scores, one after another: B=4, 32/8 heads, N=4096, D=128, causal, RoPE 597 us a pass, 514 now; a 32768-token chunked
-// prefill 18.6 ms, 15.1 now; binary16 encoder 8 x 1500, 16 heads, D=64 131 us, 119 now; 16 padded prompts of 1024 rows 223
-// and 195 us.
+// scores, one after another.  Before and now, in turn on one box, at its power limit: B=4, 32/8 heads, N=4096, D=128, causal,
+// RoPE 593 and 545 us a pass; a 32768-token chunked prefill 18.2 and 16.0 ms; binary16 encoder 8 x 1500, 16 heads, D=64 133 and
+// 124 us; 16 padded prompts of 1024 rows 220 and 201 us.  (The first passes, at full clocks: 475 us, 14.1 ms, 116 us, 186 us.)
 // The softmax warps hold a whole score row (128 registers) and must not spill: a spilled register is a store that the next
 // mbarrier arrival has to wait for (the period of a tile pair went from 4.7k to 3.4k clk when the spills went).  The code is
 // kept small for the same reason: 15 or 16 warps run five different loops, and 86 KB of instructions missed the instruction
