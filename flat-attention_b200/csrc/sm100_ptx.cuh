@@ -99,6 +99,11 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag) {
     return __all_sync(0xffffffffu, mbar_try_wait(bar, parity)) || __all_sync(0xffffffffu, mbar_wait_slow(bar, parity, abort_flag));
 }
+// For two phases at once, with one reduction.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, mbar_try_wait(bar0, parity0) && mbar_try_wait(bar1, parity1)) ||
+           __all_sync(0xffffffffu, mbar_wait_slow(bar0, parity0, abort_flag) && mbar_wait_slow(bar1, parity1, abort_flag));
+}
 
 // ---- TMA -------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

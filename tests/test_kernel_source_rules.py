@@ -105,5 +105,9 @@ def test_warps_leave_a_wait_that_gave_up_as_a_whole(file, kernel):
 
 
 def test_the_warp_wide_wait_answers_every_lane_alike():
-    body = sources()["fwd_sm100.cu"]["mbar_wait_warp"][1]
-    assert all(part.strip().startswith("__all_sync(0xffffffffu,") for part in body[body.index("return") + 6:].split("||"))
+    body = sources()["fwd_sm100.cu"]["mbar_wait_warp"][1]  # for one phase and for two
+    answers = re.findall(r"return([^;]*);", body)
+    assert answers
+    for answer in answers:
+        votes = answer.split("||")
+        assert all(vote.strip().startswith("__all_sync(0xffffffffu,") for vote in votes)
